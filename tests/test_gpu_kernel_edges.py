@@ -1,0 +1,42 @@
+"""Kernels and dispatch rules at the sizes where they can go wrong: edges of
+tiles, remainders, split and unsplit launches, against the FP64 oracle."""
+import numpy as np
+import pytest
+
+from baemm_b200 import _capi, meshes
+from baemm_b200.helmholtz import APPLY_TC, Helmholtz_CUDA
+from oracle import oracle as O
+
+from tests.helpers import crandn, relerr
+
+pytestmark = pytest.mark.gpu
+
+# The single-precision forms hold every operator to 1e-5 of the FP64 oracle
+# (FP32 geometry of well-shaped triangles, two-level FP32 sums); the FP64 form
+# to 1e-11.
+TOL32, TOL64 = 1e-5, 1e-11
+COEFF = {"bie": lambda k: [0.5, -1j * k, 1, 0], "dtn": lambda k: [0.5, -1j * k, 0, 1],
+         "sl": lambda k: [0, 1j, 0, 0], "all": lambda k: [0.3 + 0.1j, 0.7 - 1j * k, 1 + 0.3j, 0.4 - 0.2j]}
+
+
+def _apply(mode, grid, wc, wcs, cname, setup=lambda H: None):
+    """(library, FP64 oracle) boundary applies on a torus of 2 * grid[0] * grid[1] triangles."""
+    coords, tris = meshes.torus(n_minor=grid[0], n_major=grid[1])
+    meas = meshes.fibonacci_sphere(4)
+    kap = np.linspace(1.0, 6.0, wc // wcs)
+    coeff = np.array([COEFF[cname](k) for k in kap], np.complex128)
+    B = crandn(np.random.default_rng(7), coords.shape[0], wc)
+    got, ref = np.zeros_like(B), np.zeros_like(B)
+    with Helmholtz_CUDA(coords, tris, meas) as H:
+        H.SetApplyMode(mode)
+        setup(H)
+        H.ApplyBoundaryOperators_PL(1.0, B, 0.0, got, kap, coeff, wc, wcs)
+    O.Oracle(coords, tris, meas, precision=64).ApplyBoundaryOperators_PL(1.0, B, 0.0, ref, kap, coeff, wc, wcs)
+    return got, ref
+
+
+@pytest.mark.parametrize("ctas", [1, 5, 23, 148, 300])
+def test_tensor_core_split_blocks(ctas):
+    """Target blocks shared by one, a few and many CTAs (the sums of their workspace slots)."""
+    got, ref = _apply(APPLY_TC, (13, 23), 64, 32, "bie", lambda H: H.SetTuning(_capi.TUNE_TC_CTAS, ctas))
+    assert relerr(got, ref) < TOL32
