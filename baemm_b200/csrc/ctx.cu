@@ -333,8 +333,8 @@ template <class R>
 void Ctx::dense_apply(const cplx<R> *Btri, cplx<R> *Ctri, int64_t r0, int64_t r1)
 {
     if constexpr (std::is_same<R, double>::value)
-        launch_boundary_dense<double>(mesh, flags, prm_d.p, wave_count, wave_chunk_size, Btri, Ctri, stream, 2, r0,
-                                      r1);
+        launch_boundary_dense<double>(mesh, flags, prm_d.p, wave_count, wave_chunk_size, Btri, Ctri, stream,
+                                      {&split_d}, -1, r0, r1);
     else if (apply_mode == BAEMM_APPLY_TC && tc_supported(wave_count, wave_chunk_size))
     {
         if (!tc_geo_ready)
@@ -365,7 +365,7 @@ void Ctx::dense_apply(const cplx<R> *Btri, cplx<R> *Ctri, int64_t r0, int64_t r1
     }
     else
         launch_boundary_dense<float>(mesh, flags, prm_f.p, wave_count, wave_chunk_size, Btri, Ctri, stream,
-                                     dense_variant, r0, r1);
+                                     {&split_f}, dense_variant, r0, r1);
 }
 
 // ApplyBoundaryOperators.hpp:289-391 on device blocks.
@@ -461,7 +461,8 @@ void Ctx::apply_nearfield(Text alpha, const Text *B, int64_t ldB, Text beta, Tex
         launch_avop<Text, double>(mesh, B, ldB, wave_count, Bt, stream);
         launch_pack_points<double>(npts, pts3, p4, stream);
         mark(1);
-        launch_nearfield_dense<double>(mesh, nf, prm_d.p, wave_count, wave_chunk_size, p4, npts, Bt, Cp, stream);
+        launch_nearfield_dense<double>(mesh, nf, prm_d.p, wave_count, wave_chunk_size, p4, npts, Bt, Cp, stream,
+                                       {&split_d});
         mark(2);
         launch_combine<Text, double>(npts, wave_count, al, Cp, be, C, ldC, stream);
     }
@@ -486,7 +487,7 @@ void Ctx::apply_nearfield(Text alpha, const Text *B, int64_t ldB, Text beta, Tex
         }
         else
             launch_nearfield_dense<float>(mesh, nf, prm_f.p, wave_count, wave_chunk_size, p4, npts, Bt, Cp, stream,
-                                          dense_variant);
+                                          {&split_f}, dense_variant);
         mark(2);
         launch_combine<Text, float>(npts, wave_count, al, Cp, be, C, ldC, stream);
     }

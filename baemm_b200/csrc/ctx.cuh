@@ -56,7 +56,7 @@ public:
     int block_size = 64;
     int gmres_max_iter = 30, gmres_max_restarts = 3;
     int apply_mode = BAEMM_APPLY_FP32;
-    int dense_variant = 0;            // plain FP32 dense kernel variant (launch_boundary_dense)
+    int dense_variant = -1;           // plain FP32 dense kernel variant (launch_boundary_dense); -1: not set
     TcTuning tc_tune;                 // tensor-core form settings (TcTuning in ops.cuh)
     DevBuf<float2> tc_ws;             // tensor-core form: partial sums of target blocks split between CTAs
     bool tc_geo_ready = false;        // mesh.tgeo_f built
@@ -76,6 +76,8 @@ public:
     // work buffers
     DevBuf<float2> Btri_f, Ctri_f, ff_partial_f;
     DevBuf<double2> Btri_d, Ctri_d, ff_partial_d;
+    DevBuf<float2> split_f;             // partial blocks of dense launches split over the sources
+    DevBuf<double2> split_d;
     DevBuf<float> dirs_f;
     DevBuf<double> dirs_d;
     DevBuf<float> pts_f;                // near field: evaluation points, npts x 4

@@ -18,6 +18,8 @@
 // Herglotz kernels whose mask is always 1, FarFieldOperatorKernel.cl:89).
 #include "ops.cuh"
 
+#include <algorithm>
+
 namespace baemm
 {
 
@@ -89,9 +91,11 @@ template <class R, int COLS, bool SL, bool DL, bool ADL>
 __global__ void __launch_bounds__(kTargets, std::is_same<R, double>::value ? 4 : 1)
 boundary_dense_kernel(DenseTargets<R> tg, const R *__restrict__ mid4, const R *__restrict__ nrm4,
                       const cplx<R> *__restrict__ B, cplx<R> *__restrict__ C,
-                      const typename Prm<R>::type *__restrict__ prm, int n, int wc, int wcs)
+                      const typename Prm<R>::type *__restrict__ prm, int n, int wc, int wcs, int per_split)
 {
     __shared__ Tile<R, COLS> tile;
+    const int jb = blockIdx.z * per_split, je = min(n, jb + per_split);   // this split's sources
+    C += (int64_t)blockIdx.z * tg.m * wc;
     const int i = blockIdx.x * kTargets + threadIdx.x;
     const int iself = tg.self ? tg.off + i : -1;   // the source index excluded for this target (none: -1)
     const int col0 = blockIdx.y * COLS;
@@ -117,12 +121,12 @@ boundary_dense_kernel(DenseTargets<R> tg, const R *__restrict__ mid4, const R *_
     #pragma unroll
     for (int k = 0; k < COLS; ++k) { acc[k].x = R(0); acc[k].y = R(0); }
 
-    for (int j0 = 0; j0 < n; j0 += kTile)
+    for (int j0 = jb; j0 < je; j0 += kTile)
     {
         __syncthreads();
-        stage_tile<R, COLS, DL, false>(tile, mid4, nrm4, B, wc, col0, j0, n);
+        stage_tile<R, COLS, DL, false>(tile, mid4, nrm4, B, wc, col0, j0, je);
         __syncthreads();
-        const int smax = min(kTile, n - j0);
+        const int smax = min(kTile, je - j0);
         #pragma unroll
         for (int k = 0; k < COLS; ++k)
         {
@@ -191,14 +195,14 @@ boundary_dense_kernel(DenseTargets<R> tg, const R *__restrict__ mid4, const R *_
     }
 }
 
-// Plain FP32 form with packed FP32x2 arithmetic (sm_100 FFMA2).  Each thread
-// owns TT targets (i, i + 128, ...) and the 16 columns of one wave chunk.  A
-// complex MAC  c += a b  is two packed FMAs:
+// Packed FP32x2 arithmetic (sm_100 FFMA2), one target per thread and the 16
+// columns of one wave chunk (variant 1).  A complex MAC  c += a b  is two
+// packed FMAs:
 //     c += (a.re, a.re) * (b.re, b.im)
 //     c += (a.im, a.im) * (-b.im, b.re)
 // so the tile stages every RHS row twice, as b and as the swapped, negated
 // (-b.im, b.re).  Half the issue slots of the scalar form for the same FMA-pipe
-// work; TT > 1 shares every staged RHS row between TT targets.
+// work.
 constexpr int kPackedCols = 16;
 
 struct PackedTile
@@ -209,145 +213,304 @@ struct PackedTile
     float2 Bw[kTile][kPackedCols];
 };
 
-template <int TT, bool SL, bool DL, bool ADL>
-__global__ void __launch_bounds__(kTargets, TT == 1 ? 4 : 3)
+template <bool SL, bool DL, bool ADL>
+__global__ void __launch_bounds__(kTargets, 4)
 boundary_packed_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, const float *__restrict__ nrm4,
                        const float2 *__restrict__ B, float2 *__restrict__ C, const ChunkParamsF *__restrict__ prm,
-                       int n, int wc, int wcs)
+                       int n, int wc, int wcs, int per_split)
 {
     __shared__ PackedTile tile;
+    const int jb = blockIdx.z * per_split, je = min(n, jb + per_split);   // this split's sources
     const int col0 = blockIdx.y * kPackedCols;
     const int ch = col0 / wcs;
     const float kap = prm[ch].kappa;
     const float2 c1 = prm[ch].c[1], c2 = prm[ch].c[2], c3 = prm[ch].c[3];
-    int ti[TT], tself[TT];
-    float3 x[TT], nu[TT];
-    #pragma unroll
-    for (int t = 0; t < TT; ++t)
+    const int tid = threadIdx.x;
+    const int ti = blockIdx.x * kTargets + tid;
+    const int tself = tg.self ? tg.off + ti : -1;
+    float3 x = make_float3(0.f, 0.f, 0.f), nu = x;
+    if (ti < tg.m)
     {
-        ti[t] = blockIdx.x * (kTargets * TT) + t * kTargets + threadIdx.x;
-        tself[t] = tg.self ? tg.off + ti[t] : -1;
-        x[t] = make_float3(0.f, 0.f, 0.f);
-        nu[t] = make_float3(0.f, 0.f, 0.f);
-        if (ti[t] < tg.m)
+        const float4 m = reinterpret_cast<const float4 *>(tg.pts4)[ti];
+        x = make_float3(m.x, m.y, m.z);
+        if (ADL)
         {
-            const float4 m = reinterpret_cast<const float4 *>(tg.pts4)[ti[t]];
-            x[t] = make_float3(m.x, m.y, m.z);
-            if (ADL)
-            {
-                const float4 q = reinterpret_cast<const float4 *>(nrm4)[tg.off + ti[t]];
-                nu[t] = make_float3(q.x, q.y, q.z);
-            }
+            const float4 q = reinterpret_cast<const float4 *>(nrm4)[tg.off + ti];
+            nu = make_float3(q.x, q.y, q.z);
         }
     }
-    float2 acc[TT][kPackedCols], tacc[TT][kPackedCols];   // running total, this tile's sum (two-level sum)
+    float2 acc[kPackedCols], tacc[kPackedCols];   // running total, this tile's sum (two-level sum)
     #pragma unroll
-    for (int t = 0; t < TT; ++t)
-        #pragma unroll
-        for (int k = 0; k < kPackedCols; ++k) acc[t][k] = make_float2(0.f, 0.f);
+    for (int k = 0; k < kPackedCols; ++k) acc[k] = make_float2(0.f, 0.f);
 
-    for (int j0 = 0; j0 < n; j0 += kTile)
+    for (int j0 = jb; j0 < je; j0 += kTile)
     {
         __syncthreads();
+        if (tid < kTile)
         {
-            const int tid = threadIdx.x;
-            if (tid < kTile)
-            {
-                const int j = j0 + tid;
-                tile.y[tid] = (j < n) ? reinterpret_cast<const float4 *>(mid4)[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-            else if (DL && tid < 2 * kTile)
-            {
-                const int sidx = tid - kTile, j = j0 + sidx;
-                tile.mu[sidx] = (j < n) ? reinterpret_cast<const float4 *>(nrm4)[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-            for (int idx = tid; idx < kTile * kPackedCols; idx += kTargets)
-            {
-                const int sidx = idx / kPackedCols, k = idx % kPackedCols, j = j0 + sidx;
-                const float2 b = (j < n) ? B[(int64_t)j * wc + col0 + k] : make_float2(0.f, 0.f);
-                tile.B[sidx][k] = b;
-                tile.Bw[sidx][k] = make_float2(-b.y, b.x);
-            }
+            const int j = j0 + tid;
+            tile.y[tid] = (j < je) ? reinterpret_cast<const float4 *>(mid4)[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        else if (DL && tid < 2 * kTile)
+        {
+            const int sidx = tid - kTile, j = j0 + sidx;
+            tile.mu[sidx] = (j < je) ? reinterpret_cast<const float4 *>(nrm4)[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        for (int idx = tid; idx < kTile * kPackedCols; idx += kTargets)
+        {
+            const int sidx = idx / kPackedCols, k = idx % kPackedCols, j = j0 + sidx;
+            const float2 b = (j < je) ? B[(int64_t)j * wc + col0 + k] : make_float2(0.f, 0.f);
+            tile.B[sidx][k] = b;
+            tile.Bw[sidx][k] = make_float2(-b.y, b.x);
         }
         __syncthreads();
-        const int smax = min(kTile, n - j0);
+        const int smax = min(kTile, je - j0);
         #pragma unroll
-        for (int t = 0; t < TT; ++t)
-            #pragma unroll
-            for (int k = 0; k < kPackedCols; ++k) tacc[t][k] = make_float2(0.f, 0.f);
+        for (int k = 0; k < kPackedCols; ++k) tacc[k] = make_float2(0.f, 0.f);
         for (int s = 0; s < smax; ++s)
         {
             const float4 yv = tile.y[s];
             float4 mv = make_float4(0.f, 0.f, 0.f, 0.f);
             if (DL) mv = tile.mu[s];
-            float2 Ar[TT], Ai[TT];
-            #pragma unroll
-            for (int t = 0; t < TT; ++t)
+            const float zx = yv.x - x.x, zy = yv.y - x.y, zz = yv.z - x.z;
+            const float r2 = zx * zx + zy * zy + zz * zz;
+            const float rinv = (j0 + s == tself) ? 0.f : rsqrtf(r2);
+            const float r = r2 * rinv;
+            const float kr = kap * r;
+            float sn, cs;
+            __sincosf(kr, &sn, &cs);
+            float ax = 0.f, ay = 0.f;
+            if (SL)
             {
-                const float zx = yv.x - x[t].x, zy = yv.y - x[t].y, zz = yv.z - x[t].z;
-                const float r2 = zx * zx + zy * zy + zz * zz;
-                const float rinv = (j0 + s == tself[t]) ? 0.f : rsqrtf(r2);
-                const float r = r2 * rinv;
-                const float kr = kap * r;
-                float sn, cs;
-                __sincosf(kr, &sn, &cs);
-                float ax = 0.f, ay = 0.f;
-                if (SL)
-                {
-                    const float er = cs * rinv, ei = sn * rinv;
-                    ax = c1.x * er - c1.y * ei;
-                    ay = c1.x * ei + c1.y * er;
-                }
-                if (DL || ADL)
-                {
-                    const float r3 = rinv * rinv * rinv;
-                    const float g0 = -(kr * sn + cs) * r3;
-                    const float g1 = (kr * cs - sn) * r3;
-                    float fx = 0.f, fy = 0.f;
-                    if (DL)
-                    {
-                        const float dm = zx * mv.x + zy * mv.y + zz * mv.z;
-                        fx += c2.x * dm;
-                        fy += c2.y * dm;
-                    }
-                    if (ADL)
-                    {
-                        const float dn = zx * nu[t].x + zy * nu[t].y + zz * nu[t].z;
-                        fx -= c3.x * dn;
-                        fy -= c3.y * dn;
-                    }
-                    ax += fx * g0 - fy * g1;
-                    ay += fx * g1 + fy * g0;
-                }
-                Ar[t] = make_float2(ax, ax);
-                Ai[t] = make_float2(ay, ay);
+                const float er = cs * rinv, ei = sn * rinv;
+                ax = c1.x * er - c1.y * ei;
+                ay = c1.x * ei + c1.y * er;
             }
+            if (DL || ADL)
+            {
+                const float r3 = rinv * rinv * rinv;
+                const float g0 = -(kr * sn + cs) * r3;
+                const float g1 = (kr * cs - sn) * r3;
+                float fx = 0.f, fy = 0.f;
+                if (DL)
+                {
+                    const float dm = zx * mv.x + zy * mv.y + zz * mv.z;
+                    fx += c2.x * dm;
+                    fy += c2.y * dm;
+                }
+                if (ADL)
+                {
+                    const float dn = zx * nu.x + zy * nu.y + zz * nu.z;
+                    fx -= c3.x * dn;
+                    fy -= c3.y * dn;
+                }
+                ax += fx * g0 - fy * g1;
+                ay += fx * g1 + fy * g0;
+            }
+            const float2 Ar = make_float2(ax, ax), Ai = make_float2(ay, ay);
             #pragma unroll
             for (int k = 0; k < kPackedCols; ++k)
             {
-                const float2 b = tile.B[s][k], bw = tile.Bw[s][k];
-                #pragma unroll
-                for (int t = 0; t < TT; ++t)
-                {
-                    tacc[t][k] = __ffma2_rn(Ar[t], b, tacc[t][k]);
-                    tacc[t][k] = __ffma2_rn(Ai[t], bw, tacc[t][k]);
-                }
+                tacc[k] = __ffma2_rn(Ar, tile.B[s][k], tacc[k]);
+                tacc[k] = __ffma2_rn(Ai, tile.Bw[s][k], tacc[k]);
             }
         }
         #pragma unroll
-        for (int t = 0; t < TT; ++t)
-            #pragma unroll
-            for (int k = 0; k < kPackedCols; ++k) acc[t][k] = __fadd2_rn(acc[t][k], tacc[t][k]);
+        for (int k = 0; k < kPackedCols; ++k) acc[k] = __fadd2_rn(acc[k], tacc[k]);
+    }
+    if (ti < tg.m)
+    {
+        float2 *out = &C[((int64_t)blockIdx.z * tg.m + ti) * wc + col0];
+        #pragma unroll
+        for (int k = 0; k < kPackedCols; ++k) out[k] = acc[k];
+    }
+}
+
+// Plain FP32 form over pairs of targets (variant 2): the two halves of every
+// FP32x2 register are two targets (i, i + 128) of the thread, in the entry
+// evaluation as well as in the contraction
+//     (c.re, c.im) += (a.re b.re - a.im b.im, a.re b.im + a.im b.re),
+// four packed FMAs per column and pair of targets, with the right-hand side
+// staged as broadcast pairs (b.re, b.re, b.im, b.im): one 16-byte shared load
+// per column, no register shuffling, and the entry (about 22 packed
+// instructions with the real / imaginary coefficients of the solves, RI) is
+// shared by both targets.  Bound by the FP32 pipe: 64 packed FMAs per source
+// and pair of targets at 16 columns, a packed FMA taking two of its cycles.
+// Each 32-source tile is summed into fresh accumulators and added to running
+// totals in shared memory (a private float4 per thread and column; two-level
+// summation as in boundary_dense_kernel), which leaves the registers for four
+// CTAs of 128 threads per SM.
+// Measured: 2.91 ms on 20234 triangles x 32 columns (SL + DL', FP32 pipe 72 %
+// busy), the scalar kernel 4.95 ms; 157 us on 5120 x 16 in chunks of 8 columns,
+// the scalar kernel unsplit 480 us.
+constexpr int kPairTile = 32;
+
+template <int COLS>
+struct PairTile
+{
+    float4 g[kPairTile][3];        // (y.x, y.x, y.y, y.y), (y.z, y.z, mu.x, mu.x), (mu.y, mu.y, mu.z, mu.z)
+    float4 b[kPairTile][COLS];
+    float4 tot[COLS][kTargets];    // (re, re', im, im') of the thread's two targets
+};
+
+template <int COLS, bool SL, bool DL, bool ADL, bool RI>
+__global__ void __launch_bounds__(kTargets, 4)
+boundary_pair_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, const float *__restrict__ nrm4,
+                     const float2 *__restrict__ B, float2 *__restrict__ C, const ChunkParamsF *__restrict__ prm,
+                     int n, int wc, int wcs, int per_split)
+{
+    __shared__ PairTile<COLS> tile;
+    const int tid = threadIdx.x;
+    const int col0 = blockIdx.y * COLS;
+    const int jb = blockIdx.z * per_split, je = min(n, jb + per_split);   // this split's sources
+    const ChunkParamsF &q = prm[col0 / wcs];
+    const float2 nk = make_float2(-q.kappa, -q.kappa);
+    const float2 c1x = make_float2(q.c[1].x, q.c[1].x), c1y = make_float2(q.c[1].y, q.c[1].y);
+    const float2 nc2x = make_float2(-q.c[2].x, -q.c[2].x), nc2y = make_float2(-q.c[2].y, -q.c[2].y);
+    const float2 c3x = make_float2(q.c[3].x, q.c[3].x), c3y = make_float2(q.c[3].y, q.c[3].y);
+    const int t0 = blockIdx.x * (2 * kTargets) + tid, t1 = t0 + kTargets;
+    const int self0 = tg.self ? tg.off + t0 : -1, self1 = tg.self ? tg.off + t1 : -1;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 xa = t0 < tg.m ? reinterpret_cast<const float4 *>(tg.pts4)[t0] : zero;
+    const float4 xb = t1 < tg.m ? reinterpret_cast<const float4 *>(tg.pts4)[t1] : zero;
+    const float2 nx0 = make_float2(-xa.x, -xb.x), nx1 = make_float2(-xa.y, -xb.y), nx2 = make_float2(-xa.z, -xb.z);
+    float2 tn0 = make_float2(0.f, 0.f), tn1 = tn0, tn2 = tn0;
+    if (ADL)
+    {
+        const float4 na = t0 < tg.m ? reinterpret_cast<const float4 *>(nrm4)[tg.off + t0] : zero;
+        const float4 nb = t1 < tg.m ? reinterpret_cast<const float4 *>(nrm4)[tg.off + t1] : zero;
+        tn0 = make_float2(na.x, nb.x); tn1 = make_float2(na.y, nb.y); tn2 = make_float2(na.z, nb.z);
     }
     #pragma unroll
-    for (int t = 0; t < TT; ++t)
-        if (ti[t] < tg.m)
+    for (int k = 0; k < COLS; ++k) tile.tot[k][tid] = zero;   // private to the thread: no barrier needed
+
+    for (int j0 = jb; j0 < je; j0 += kPairTile)
+    {
+        __syncthreads();
+        if (tid < kPairTile)
         {
-            float4 *out = reinterpret_cast<float4 *>(&C[(int64_t)ti[t] * wc + col0]);
-            #pragma unroll
-            for (int k = 0; k < kPackedCols; k += 2)
-                out[k / 2] = make_float4(acc[t][k].x, acc[t][k].y, acc[t][k + 1].x, acc[t][k + 1].y);
+            const int j = j0 + tid;
+            const float4 y = j < je ? reinterpret_cast<const float4 *>(mid4)[j] : zero;
+            const float4 mu = DL && j < je ? reinterpret_cast<const float4 *>(nrm4)[j] : zero;
+            tile.g[tid][0] = make_float4(y.x, y.x, y.y, y.y);
+            tile.g[tid][1] = make_float4(y.z, y.z, mu.x, mu.x);
+            tile.g[tid][2] = make_float4(mu.y, mu.y, mu.z, mu.z);
         }
+        #pragma unroll
+        for (int idx = tid; idx < kPairTile * COLS; idx += kTargets)
+        {
+            const int s = idx / COLS, k = idx % COLS, j = j0 + s;
+            const float2 b = j < je ? B[(int64_t)j * wc + col0 + k] : make_float2(0.f, 0.f);
+            tile.b[s][k] = make_float4(b.x, b.x, b.y, b.y);
+        }
+        __syncthreads();
+        const int smax = min(kPairTile, je - j0);
+        float2 cr[COLS], ci[COLS];
+        #pragma unroll
+        for (int k = 0; k < COLS; ++k) cr[k] = ci[k] = make_float2(0.f, 0.f);
+        for (int s = 0; s < smax; ++s)
+        {
+            const float4 ga = tile.g[s][0], gb = tile.g[s][1], gc = tile.g[s][2];
+            const float2 zx = __fadd2_rn(make_float2(ga.x, ga.y), nx0);
+            const float2 zy = __fadd2_rn(make_float2(ga.z, ga.w), nx1);
+            const float2 zz = __fadd2_rn(make_float2(gb.x, gb.y), nx2);
+            const float2 r2 = __ffma2_rn(zz, zz, __ffma2_rn(zy, zy, __fmul2_rn(zx, zx)));
+            const float2 ri = make_float2(j0 + s == self0 ? 0.f : rsqrtf(r2.x), j0 + s == self1 ? 0.f : rsqrtf(r2.y));
+            const float2 nkr = __fmul2_rn(nk, __fmul2_rn(r2, ri));   // -k r
+            float sa, ca, sb, cb;
+            __sincosf(nkr.x, &sa, &ca);
+            __sincosf(nkr.y, &sb, &cb);
+            const float2 cs = make_float2(ca, cb), nsn = make_float2(sa, sb);   // cos(k r), -sin(k r)
+            // h = c1 / r + u + i k r (-u),  u = -(c2 (z.mu) - c3 (z.nu)) / r^3;  A = e^{i k r} h
+            float2 ux = make_float2(0.f, 0.f), uy = ux, hx = ux, hy = ux;
+            if (DL || ADL)
+            {
+                const float2 ri3 = __fmul2_rn(__fmul2_rn(ri, ri), ri);
+                if (DL)
+                {
+                    const float2 dm = __fmul2_rn(
+                        __ffma2_rn(zz, make_float2(gc.z, gc.w),
+                                   __ffma2_rn(zy, make_float2(gc.x, gc.y), __fmul2_rn(zx, make_float2(gb.z, gb.w)))),
+                        ri3);
+                    ux = __fmul2_rn(nc2x, dm);
+                    if (!RI) uy = __fmul2_rn(nc2y, dm);
+                }
+                if (ADL)
+                {
+                    const float2 dn = __fmul2_rn(__ffma2_rn(zz, tn2, __ffma2_rn(zy, tn1, __fmul2_rn(zx, tn0))), ri3);
+                    ux = DL ? __ffma2_rn(c3x, dn, ux) : __fmul2_rn(c3x, dn);
+                    if (!RI) uy = DL ? __ffma2_rn(c3y, dn, uy) : __fmul2_rn(c3y, dn);
+                }
+                hx = ux;
+                hy = __fmul2_rn(nkr, ux);
+                if (!RI)
+                {
+                    hx = __ffma2_rn(make_float2(-nkr.x, -nkr.y), uy, hx);
+                    hy = __fadd2_rn(hy, uy);
+                }
+            }
+            if (SL)
+            {
+                if (!RI) hx = __ffma2_rn(c1x, ri, hx);
+                hy = __ffma2_rn(c1y, ri, hy);
+            }
+            // (ar, ai) = (hx cos - hy sin, hx sin + hy cos)
+            const float2 ar = __ffma2_rn(hy, nsn, __fmul2_rn(hx, cs));
+            const float2 ai = __ffma2_rn(hy, cs, __fmul2_rn(make_float2(-hx.x, -hx.y), nsn));
+            const float2 nai = make_float2(-ai.x, -ai.y);
+            #pragma unroll
+            for (int k = 0; k < COLS; ++k)
+            {
+                const float4 b = tile.b[s][k];
+                const float2 br = make_float2(b.x, b.y), bi = make_float2(b.z, b.w);
+                cr[k] = __ffma2_rn(ar, br, cr[k]);
+                cr[k] = __ffma2_rn(nai, bi, cr[k]);
+                ci[k] = __ffma2_rn(ar, bi, ci[k]);
+                ci[k] = __ffma2_rn(ai, br, ci[k]);
+            }
+        }
+        #pragma unroll
+        for (int k = 0; k < COLS; ++k)
+        {
+            float4 t = tile.tot[k][tid];
+            t.x += cr[k].x; t.y += cr[k].y; t.z += ci[k].x; t.w += ci[k].y;
+            tile.tot[k][tid] = t;
+        }
+    }
+    float2 *out = C + (int64_t)blockIdx.z * tg.m * wc + col0;
+    #pragma unroll
+    for (int k = 0; k < COLS; ++k)
+    {
+        const float4 t = tile.tot[k][tid];
+        if (t0 < tg.m) out[(int64_t)t0 * wc + k] = make_float2(t.x, t.z);
+        if (t1 < tg.m) out[(int64_t)t1 * wc + k] = make_float2(t.y, t.w);
+    }
+}
+
+// C = the sum of the splits' partial blocks, in split order (four loads in flight).
+template <class R>
+__global__ void split_sum_kernel(const cplx<R> *__restrict__ partial, int splits, int64_t elems, cplx<R> *__restrict__ C)
+{
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= elems) return;
+    const cplx<R> *p = partial + e;
+    cplx<R> s = p[0];
+    int q = 1;
+    for (; q + 4 <= splits; q += 4)
+    {
+        cplx<R> v[4];
+        #pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = p[(q + u) * elems];
+        #pragma unroll
+        for (int u = 0; u < 4; ++u) { s.x += v[u].x; s.y += v[u].y; }
+    }
+    for (; q < splits; ++q)
+    {
+        const cplx<R> v = p[q * elems];
+        s.x += v.x;
+        s.y += v.y;
+    }
+    C[e] = s;
 }
 
 template <class R, int COLS, bool SL, bool DL>
@@ -553,11 +716,11 @@ __global__ void pack_points_kernel(int64_t m, const double *__restrict__ pts3, R
 
 // ---- dispatch helpers -----------------------------------------------------------
 template <class R, int COLS>
-void boundary_cols(const OpFlags &f, dim3 grid, cudaStream_t st, DenseTargets<R> tg, const R *mid, const R *nrm,
-                   const cplx<R> *B, cplx<R> *C, const typename Prm<R>::type *p, int n, int wc, int wcs)
+void boundary_cols(int code, dim3 grid, cudaStream_t st, DenseTargets<R> tg, const R *mid, const R *nrm,
+                   const cplx<R> *B, cplx<R> *C, const typename Prm<R>::type *p, int n, int wc, int wcs, int per_split)
 {
-    const int code = (f.sl() ? 1 : 0) | (f.dl() ? 2 : 0) | (f.adl() ? 4 : 0);
-#define BAEMM_BK(SL, DL, ADL) boundary_dense_kernel<R, COLS, SL, DL, ADL><<<grid, kTargets, 0, st>>>(tg, mid, nrm, B, C, p, n, wc, wcs)
+#define BAEMM_BK(SL, DL, ADL) \
+    boundary_dense_kernel<R, COLS, SL, DL, ADL><<<grid, kTargets, 0, st>>>(tg, mid, nrm, B, C, p, n, wc, wcs, per_split)
     switch (code)
     {
         case 1: BAEMM_BK(true, false, false); break;
@@ -610,12 +773,11 @@ template <> const double *geo_meas<double>(const MeshDev &m) { return m.meas_d; 
 
 inline int cols_for(int wcs) { return wcs < 16 ? wcs : 16; }
 
-template <int TT>
-void packed_dispatch(int code, DenseTargets<float> tg, int n, int wc, int wcs, const float *mid, const float *nrm,
-                     const float2 *B, float2 *C, const ChunkParamsF *p, cudaStream_t st)
+void packed_dispatch(int code, dim3 grid, cudaStream_t st, DenseTargets<float> tg, const float *mid, const float *nrm,
+                     const float2 *B, float2 *C, const ChunkParamsF *p, int n, int wc, int wcs, int per_split)
 {
-    dim3 grid(ceil_div(tg.m, kTargets * TT), wc / kPackedCols);
-#define BAEMM_PK(SL, DL, ADL) boundary_packed_kernel<TT, SL, DL, ADL><<<grid, kTargets, 0, st>>>(tg, mid, nrm, B, C, p, n, wc, wcs)
+#define BAEMM_PK(SL, DL, ADL) \
+    boundary_packed_kernel<SL, DL, ADL><<<grid, kTargets, 0, st>>>(tg, mid, nrm, B, C, p, n, wc, wcs, per_split)
     switch (code)
     {
         case 1: BAEMM_PK(true, false, false); break;
@@ -630,61 +792,146 @@ void packed_dispatch(int code, DenseTargets<float> tg, int n, int wc, int wcs, c
 #undef BAEMM_PK
 }
 
-// Ctri (tg.m x wc) = K Btri over all nt sources for the targets tg.
+template <int COLS, bool RI>
+void pair_dispatch(int code, dim3 grid, cudaStream_t st, DenseTargets<float> tg, const float *mid, const float *nrm,
+                   const float2 *B, float2 *C, const ChunkParamsF *p, int n, int wc, int wcs, int per_split)
+{
+#define BAEMM_PR(SL, DL, ADL) \
+    boundary_pair_kernel<COLS, SL, DL, ADL, RI><<<grid, kTargets, 0, st>>>(tg, mid, nrm, B, C, p, n, wc, wcs, per_split)
+    switch (code)
+    {
+        case 1: BAEMM_PR(true, false, false); break;
+        case 2: BAEMM_PR(false, true, false); break;
+        case 3: BAEMM_PR(true, true, false); break;
+        case 4: BAEMM_PR(false, false, true); break;
+        case 5: BAEMM_PR(true, false, true); break;
+        case 6: BAEMM_PR(false, true, true); break;
+        case 7: BAEMM_PR(true, true, true); break;
+        default: break;
+    }
+#undef BAEMM_PR
+}
+
+// Source splits of a launch of `ctas` CTAs over n sources (each split writes a
+// partial block, split_sum_kernel adds them): the s that minimises
+//     (n / s + kSplitCost) * max(ceil(ctas s / SMs), 2),
+// the sources of one CTA times the CTAs of the busiest SM.  An SM needs about
+// two CTAs before its FP32 pipe is shared rather than idle (hence the 2), and
+// a CTA costs about kSplitCost sources to start, drain and sum.  Without it a
+// launch of a few CTAs leaves most SMs idle, and one of 1.1 CTAs per SM runs
+// at half speed: 320 triangles x 16 columns ran 44 us as 3 CTAs of the scalar
+// kernel and 7.3 + 3.1 us (the sum) as 2 x 10 of the pair kernel, 5120 x 16
+// 480 us as 80 CTAs and 157 + 2.9 us split.
+constexpr int kSplitCost = 24, kSplitMin = 16, kSplitMax = 64;
+
+int dense_splits(int64_t ctas, int64_t n, int sms)
+{
+    int best = 1;
+    double best_cost = 0.0;
+    for (int s = 1; s <= kSplitMax && (s == 1 || n >= (int64_t)s * kSplitMin); ++s)
+    {
+        const int64_t per_sm = std::max<int64_t>((ctas * s + sms - 1) / sms, 2);
+        const double cost = ((double)n / s + (s > 1 ? kSplitCost : 0)) * (double)per_sm;
+        if (s == 1 || cost < 0.97 * best_cost) { best = s; best_cost = cost; }
+    }
+    return best;
+}
+
+// Ctri (tg.m x wc) = K Btri over all nt sources for the targets tg, in as many
+// splits as ws can hold.
 template <class R>
 void dense_dispatch(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
-                    DenseTargets<R> tg, const cplx<R> *Btri, cplx<R> *Ctri, cudaStream_t st, int variant)
+                    DenseTargets<R> tg, const cplx<R> *Btri, cplx<R> *Ctri, cudaStream_t st, int variant,
+                    SplitSpace<R> ws)
 {
     if (!f.any_layer() || m.nt == 0 || tg.m == 0) return;
     const int n = (int)m.nt;
     const int cols = cols_for(wcs);
-    dim3 grid(ceil_div(tg.m, kTargets), wc / cols);
+    const int code = (f.sl() ? 1 : 0) | (f.dl() ? 2 : 0) | (f.adl() ? 4 : 0);
     const auto *p = static_cast<const typename Prm<R>::type *>(chunk_params);
     const R *mid = geo_mid<R>(m), *nrm = geo_nrm<R>(m);
-    if constexpr (std::is_same<R, float>::value)
+    // plain FP32: the pair kernel unless a variant was set (its entry is shared by
+    // too few columns below 4 per chunk)
+    const bool pair = std::is_same<R, float>::value && (variant < 0 || variant == 2) && cols >= 4;
+    const bool packed = std::is_same<R, float>::value && variant == 1 && cols == kPackedCols;
+    dim3 grid(ceil_div(tg.m, pair ? 2 * kTargets : kTargets), wc / cols);
+    const int64_t elems = (int64_t)tg.m * wc;
+    int splits = dense_splits((int64_t)grid.x * grid.y, n, tc_sm_count());
+    cplx<R> *out = Ctri;
+    if (splits > 1 && ws.grow)
     {
-        if (cols == kPackedCols && variant > 0)
+        try
         {
-            const int code = (f.sl() ? 1 : 0) | (f.dl() ? 2 : 0) | (f.adl() ? 4 : 0);
-            if (variant == 2) packed_dispatch<2>(code, tg, n, wc, wcs, mid, nrm, Btri, Ctri, p, st);
-            else packed_dispatch<1>(code, tg, n, wc, wcs, mid, nrm, Btri, Ctri, p, st);
-            BAEMM_LAUNCH_CHECK();
-            return;
+            out = ws.grow->reserve((size_t)splits * elems);
+        }
+        catch (const Error &)
+        {
+            splits = 1;   // no memory for the partial blocks: one sweep per target
         }
     }
-    switch (cols)
+    else if (splits > 1)
     {
-        case 1: boundary_cols<R, 1>(f, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs); break;
-        case 2: boundary_cols<R, 2>(f, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs); break;
-        case 4: boundary_cols<R, 4>(f, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs); break;
-        case 8: boundary_cols<R, 8>(f, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs); break;
-        case 16: boundary_cols<R, 16>(f, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs); break;
-        default: throw Error(BAEMM_ERR_SIZE, "wave_chunk_size must be a power of two <= 64");
+        splits = (int)std::max<size_t>(1, std::min<size_t>(splits, ws.elems / elems));
+        out = ws.fixed;
     }
+    const int per_split = ceil_div(n, splits);
+    grid.z = ceil_div(n, per_split);   // every split has sources
+    if (grid.z == 1) out = Ctri;
+    if constexpr (std::is_same<R, float>::value)
+    {
+        // single layer imaginary, double layers real (the tuples of the solves): RI
+        const bool ri = !f.re_sl && !f.im_dl && !f.im_adl;
+#define BAEMM_PC(COLS) \
+    ri ? pair_dispatch<COLS, true>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split) \
+       : pair_dispatch<COLS, false>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split)
+        if (pair)
+        {
+            if (cols == 16) BAEMM_PC(16);
+            else if (cols == 8) BAEMM_PC(8);
+            else BAEMM_PC(4);
+        }
+        else if (packed) packed_dispatch(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split);
+#undef BAEMM_PC
+    }
+    if (!pair && !packed)
+        switch (cols)
+        {
+            case 1: boundary_cols<R, 1>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split); break;
+            case 2: boundary_cols<R, 2>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split); break;
+            case 4: boundary_cols<R, 4>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split); break;
+            case 8: boundary_cols<R, 8>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split); break;
+            case 16: boundary_cols<R, 16>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split); break;
+            default: throw Error(BAEMM_ERR_SIZE, "wave_chunk_size must be a power of two <= 64");
+        }
     BAEMM_LAUNCH_CHECK();
+    if (grid.z > 1)
+    {
+        split_sum_kernel<R><<<ceil_div(elems, 256), 256, 0, st>>>(out, (int)grid.z, elems, Ctri);
+        BAEMM_LAUNCH_CHECK();
+    }
 }
 
 } // namespace
 
 template <class R>
 void launch_boundary_dense(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
-                           const cplx<R> *Btri, cplx<R> *Ctri, cudaStream_t st, int variant, int64_t row_begin,
-                           int64_t row_end)
+                           const cplx<R> *Btri, cplx<R> *Ctri, cudaStream_t st, SplitSpace<R> ws, int variant,
+                           int64_t row_begin, int64_t row_end)
 {
     const int64_t r0 = std::max<int64_t>(0, row_begin), r1 = row_end < 0 ? m.nt : std::min<int64_t>(row_end, m.nt);
     if (r1 <= r0) return;
     dense_dispatch<R>(m, f, chunk_params, wc, wcs, DenseTargets<R>{geo_mid<R>(m) + 4 * r0, (int)(r1 - r0), 1, (int)r0},
-                      Btri, Ctri + r0 * wc, st, variant);
+                      Btri, Ctri + r0 * wc, st, variant, ws);
 }
 
 template <class R>
 void launch_nearfield_dense(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
                             const R *pts4, int64_t npts, const cplx<R> *Btri, cplx<R> *Cpts, cudaStream_t st,
-                            int variant)
+                            SplitSpace<R> ws, int variant)
 {
     BAEMM_REQUIRE(!f.adl() && !f.mass(), BAEMM_ERR_ARG, "near field: single and double layer only");
     BAEMM_REQUIRE(npts <= INT32_MAX, BAEMM_ERR_SIZE, "too many evaluation points");
-    dense_dispatch<R>(m, f, chunk_params, wc, wcs, DenseTargets<R>{pts4, (int)npts, 0, 0}, Btri, Cpts, st, variant);
+    dense_dispatch<R>(m, f, chunk_params, wc, wcs, DenseTargets<R>{pts4, (int)npts, 0, 0}, Btri, Cpts, st, variant, ws);
 }
 
 template <class R>
@@ -775,15 +1022,15 @@ void launch_incident(const MeshDev &m, const void *chunk_params, int wc, int wcs
 }
 
 template void launch_boundary_dense<float>(const MeshDev &, const OpFlags &, const void *, int, int, const float2 *,
-                                           float2 *, cudaStream_t, int, int64_t, int64_t);
+                                           float2 *, cudaStream_t, SplitSpace<float>, int, int64_t, int64_t);
 template void launch_pack_points<float>(int64_t, const double *, float *, cudaStream_t);
 template void launch_pack_points<double>(int64_t, const double *, double *, cudaStream_t);
 template void launch_nearfield_dense<float>(const MeshDev &, const OpFlags &, const void *, int, int, const float *,
-                                            int64_t, const float2 *, float2 *, cudaStream_t, int);
+                                            int64_t, const float2 *, float2 *, cudaStream_t, SplitSpace<float>, int);
 template void launch_nearfield_dense<double>(const MeshDev &, const OpFlags &, const void *, int, int, const double *,
-                                             int64_t, const double2 *, double2 *, cudaStream_t, int);
+                                             int64_t, const double2 *, double2 *, cudaStream_t, SplitSpace<double>, int);
 template void launch_boundary_dense<double>(const MeshDev &, const OpFlags &, const void *, int, int, const double2 *,
-                                            double2 *, cudaStream_t, int, int64_t, int64_t);
+                                            double2 *, cudaStream_t, SplitSpace<double>, int, int64_t, int64_t);
 template void launch_farfield<float>(const MeshDev &, const OpFlags &, const void *, int, int, const float2 *, float2 *,
                                      size_t, double2, double2, double2 *, int64_t, cudaStream_t);
 template void launch_farfield<double>(const MeshDev &, const OpFlags &, const void *, int, int, const double2 *,

@@ -108,14 +108,24 @@ void launch_axpby(int64_t rows, int cols, T a, const T *x, int64_t ldx, T b, T *
 // ---- dense.cu ------------------------------------------------------------------
 // Dense boundary kernel (BoundaryOperatorKernel.cl:5-239): Ctri = K(kappa) Btri
 // chunk by chunk, the self pair excluded.  R = float (plain FP32) or double.
-// variant (FP32, 16-column groups): 0 scalar FMA kernel, 1 / 2 packed FP32x2
-// kernel with 1 / 2 targets per thread.  [row_begin, row_end) restricts the
-// targets to those triangles (rows of Ctri outside are not written; row_end
-// < 0: all).
+// variant (FP32): 0 scalar FMA kernel, 1 packed FP32x2 kernel (16-column
+// groups), 2 FP32x2 kernel over pairs of targets (groups of 4 columns and
+// more), -1 the library's choice (2 where it applies); where a variant does not
+// apply, 0.  [row_begin, row_end) restricts the targets to those triangles
+// (rows of Ctri outside are not written; row_end < 0: all).
 constexpr int kDenseVariants = 3;
+// Where a launch that is split over the sources keeps its partial blocks: a
+// context's buffer that grows as needed, or a fixed block of `elems` elements.
+template <class R>
+struct SplitSpace
+{
+    DevBuf<cplx<R>> *grow = nullptr;
+    cplx<R> *fixed = nullptr;
+    size_t elems = 0;
+};
 template <class R>
 void launch_boundary_dense(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
-                           const cplx<R> *Btri, cplx<R> *Ctri, cudaStream_t st, int variant = 2,
+                           const cplx<R> *Btri, cplx<R> *Ctri, cudaStream_t st, SplitSpace<R> ws, int variant = -1,
                            int64_t row_begin = 0, int64_t row_end = -1);
 // Near-field kernel (NearFieldOperatorKernel.cl:5-194): Cpts (npts x wc) =
 // K(kappa) Btri at the points pts4 (npts x 4 reals), single and double layer
@@ -123,7 +133,7 @@ void launch_boundary_dense(const MeshDev &m, const OpFlags &f, const void *chunk
 template <class R>
 void launch_nearfield_dense(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
                             const R *pts4, int64_t npts, const cplx<R> *Btri, cplx<R> *Cpts, cudaStream_t st,
-                            int variant = 2);
+                            SplitSpace<R> ws, int variant = -1);
 // Evaluation points (m x 3 doubles, device) -> m x 4 reals, w = 0.
 template <class R>
 void launch_pack_points(int64_t m, const double *pts3, R *pts4, cudaStream_t st);

@@ -70,7 +70,7 @@ void Ctx::autotune(int mode, int repeats, baemm_tune_result *out)
                      (tc_tune.share << 5);
     const TuneKey key{device, mesh.nt, mesh.nv, wave_count, wave_chunk_size, mode, code, form};
     auto report = [&](const TuneChoice &ch, double before, int cached) {
-        out->dense_variant = dense_variant;
+        out->dense_variant = std::max(0, dense_variant);
         out->tc_segment = tc_tune.seg_tiles;
         out->tc_ctas = tc_tune.ctas;
         out->tc_stagger = tc_tune.stagger;

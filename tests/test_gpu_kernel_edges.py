@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from baemm_b200 import _capi, meshes
-from baemm_b200.helmholtz import APPLY_TC, Helmholtz_CUDA
+from baemm_b200.helmholtz import APPLY_FP32, APPLY_FP64, APPLY_TC, Helmholtz_CUDA
 from oracle import oracle as O
 
 from tests.helpers import crandn, relerr
@@ -40,3 +40,25 @@ def test_tensor_core_split_blocks(ctas):
     """Target blocks shared by one, a few and many CTAs (the sums of their workspace slots)."""
     got, ref = _apply(APPLY_TC, (13, 23), 64, 32, "bie", lambda H: H.SetTuning(_capi.TUNE_TC_CTAS, ctas))
     assert relerr(got, ref) < TOL32
+
+
+@pytest.mark.parametrize("variant", [None, 0, 1, 2])
+@pytest.mark.parametrize("grid", [(3, 3), (4, 4), (5, 13), (16, 8), (15, 17), (16, 16), (19, 54)])
+@pytest.mark.parametrize("wc,wcs,cname", [(16, 16, "bie"), (32, 32, "all"), (24, 8, "dtn"), (8, 4, "all"), (4, 2, "bie"),
+                                          (3, 1, "sl")])
+def test_plain_fp32_variants(variant, grid, wc, wcs, cname):
+    """18 to 2052 triangles: less than a tile, whole tiles and one more, one and
+    many source splits, blocks of targets that are full, partly filled and half
+    empty, in every chunk size's kernel."""
+    got, ref = _apply(APPLY_FP32, grid, wc, wcs, cname,
+                      lambda H: variant is not None and H.SetKernelVariant(variant))
+    assert relerr(got, ref) < TOL32
+
+
+def test_kernel_variant_reads_back():
+    coords, tris = meshes.icosphere(1)
+    with Helmholtz_CUDA(coords, tris, meshes.fibonacci_sphere(4)) as H:
+        assert H.GetKernelVariant() == 0
+        for v in (2, 0, 1):
+            H.SetKernelVariant(v)
+            assert H.GetKernelVariant() == v
