@@ -515,7 +515,7 @@ void Ctx::apply_farfield(zc alpha, const double2 *B, int64_t ldB, zc beta, doubl
     BAEMM_REQUIRE(mesh.nm > 0, BAEMM_ERR_SIZE, "no measurement directions");
     BAEMM_REQUIRE(ldB >= wave_count && ldC >= wave_count, BAEMM_ERR_ARG, "leading dimension smaller than wave_count");
     const int64_t tri_elems = mesh.nt * wave_count;
-    const size_t pe = farfield_partial_elems(mesh, wave_count, wave_chunk_size);
+    const size_t pe = farfield_partial_elems(mesh, wave_count, wave_chunk_size, aux_fp64());
     const double2 be = make_double2(beta.real(), beta.imag());
     if (aux_fp64())
     {

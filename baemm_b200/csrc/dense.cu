@@ -83,12 +83,9 @@ __device__ __forceinline__ void stage_tile(Tile<R, COLS> &t, const R *__restrict
     }
 }
 
-// FP64: 4 CTAs of 128 threads per SM (<= 128 registers; a few bytes spill)
-// keep more warps in flight for the FP64 pipe than the 3 CTAs that the 134
-// registers of an unbounded build allow: 916 vs 946 ms on the 153,600-triangle
-// torus with 64 right-hand sides, identical results.
+// In FP64 only chunks of fewer than 8 columns come here (dense64.cu takes the others).
 template <class R, int COLS, bool SL, bool DL, bool ADL>
-__global__ void __launch_bounds__(kTargets, std::is_same<R, double>::value ? 4 : 1)
+__global__ void __launch_bounds__(kTargets)
 boundary_dense_kernel(DenseTargets<R> tg, const R *__restrict__ mid4, const R *__restrict__ nrm4,
                       const cplx<R> *__restrict__ B, cplx<R> *__restrict__ C,
                       const typename Prm<R>::type *__restrict__ prm, int n, int wc, int wcs, int per_split)
@@ -568,23 +565,41 @@ farfield_partial_kernel(const R *__restrict__ meas4, const R *__restrict__ mid4,
     }
 }
 
+// Sum of the splits' partial blocks in double, times alpha, plus beta C.  One
+// block per 32 elements: 8 rows of threads take every eighth split each (four
+// loads in flight), added in row order.  (One thread per element over all
+// splits: 42 us for 148 x 256 x 32 double values, now 3.3 us for 74.)
+constexpr int kReduceRows = 8;
 template <class R>
-__global__ void farfield_reduce_kernel(const cplx<R> *__restrict__ partial, int splits, int m, int wc, double2 alpha,
-                                       double2 beta, double2 *__restrict__ Cout, int64_t ldC)
+__global__ void __launch_bounds__(32 * kReduceRows)
+farfield_reduce_kernel(const cplx<R> *__restrict__ partial, int splits, int m, int wc, double2 alpha, double2 beta,
+                       double2 *__restrict__ Cout, int64_t ldC)
 {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (int64_t)m * wc) return;
-    const int64_t i = idx / wc;
-    const int k = (int)(idx - i * wc);
-    double sx = 0.0, sy = 0.0;
-    for (int s = 0; s < splits; ++s)
+    __shared__ double2 row[kReduceRows][32];
+    const int64_t elems = (int64_t)m * wc, idx = (int64_t)blockIdx.x * 32 + threadIdx.x;
+    double2 t = make_double2(0.0, 0.0);
+    if (idx < elems)
     {
-        const cplx<R> p = partial[((int64_t)s * m + i) * wc + k];
-        sx += (double)p.x;
-        sy += (double)p.y;
+        #pragma unroll 4
+        for (int s = threadIdx.y; s < splits; s += kReduceRows)
+        {
+            const cplx<R> p = partial[s * elems + idx];
+            t.x += (double)p.x;
+            t.y += (double)p.y;
+        }
     }
-    double2 o = make_double2(alpha.x * sx - alpha.y * sy, alpha.x * sy + alpha.y * sx);
-    double2 *c = &Cout[i * ldC + k];
+    row[threadIdx.y][threadIdx.x] = t;
+    __syncthreads();
+    if (threadIdx.y != 0 || idx >= elems) return;
+    #pragma unroll
+    for (int s = 1; s < kReduceRows; ++s)
+    {
+        t.x += row[s][threadIdx.x].x;
+        t.y += row[s][threadIdx.x].y;
+    }
+    const int64_t i = idx / wc;
+    double2 o = make_double2(alpha.x * t.x - alpha.y * t.y, alpha.x * t.y + alpha.y * t.x);
+    double2 *c = &Cout[i * ldC + (idx - i * wc)];
     if (beta.x != 0.0 || beta.y != 0.0)
     {
         const double2 b = *c;
@@ -822,7 +837,7 @@ void pair_dispatch(int code, dim3 grid, cudaStream_t st, DenseTargets<float> tg,
 // at half speed: 320 triangles x 16 columns ran 44 us as 3 CTAs of the scalar
 // kernel and 7.3 + 3.1 us (the sum) as 2 x 10 of the pair kernel, 5120 x 16
 // 480 us as 80 CTAs and 157 + 2.9 us split.
-constexpr int kSplitCost = 24, kSplitMin = 16, kSplitMax = 64;
+constexpr int kSplitCost = 24, kSplitMin = 16, kSplitMax = 128;
 
 int dense_splits(int64_t ctas, int64_t n, int sms)
 {
@@ -854,9 +869,10 @@ void dense_dispatch(const MeshDev &m, const OpFlags &f, const void *chunk_params
     // too few columns below 4 per chunk)
     const bool pair = std::is_same<R, float>::value && (variant < 0 || variant == 2) && cols >= 4;
     const bool packed = std::is_same<R, float>::value && variant == 1 && cols == kPackedCols;
+    const bool d64 = std::is_same<R, double>::value && cols >= 8;
     dim3 grid(ceil_div(tg.m, pair ? 2 * kTargets : kTargets), wc / cols);
     const int64_t elems = (int64_t)tg.m * wc;
-    int splits = dense_splits((int64_t)grid.x * grid.y, n, tc_sm_count());
+    int splits = dense_splits(d64 ? d64_ctas(d64_unit(wc, wcs), tg.m, wc) : (int64_t)grid.x * grid.y, n, tc_sm_count());
     cplx<R> *out = Ctri;
     if (splits > 1 && ws.grow)
     {
@@ -874,7 +890,7 @@ void dense_dispatch(const MeshDev &m, const OpFlags &f, const void *chunk_params
         splits = (int)std::max<size_t>(1, std::min<size_t>(splits, ws.elems / elems));
         out = ws.fixed;
     }
-    const int per_split = ceil_div(n, splits);
+    const int per_split = ceil_div(ceil_div(n, splits), 8) * 8;
     grid.z = ceil_div(n, per_split);   // every split has sources
     if (grid.z == 1) out = Ctri;
     if constexpr (std::is_same<R, float>::value)
@@ -893,17 +909,24 @@ void dense_dispatch(const MeshDev &m, const OpFlags &f, const void *chunk_params
         else if (packed) packed_dispatch(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split);
 #undef BAEMM_PC
     }
-    if (!pair && !packed)
+    else if (d64) launch_boundary_d64(m, f, p, wc, wcs, tg, Btri, out, per_split, st);
+    if (!pair && !packed && !d64)
         switch (cols)
         {
             case 1: boundary_cols<R, 1>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split); break;
             case 2: boundary_cols<R, 2>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split); break;
             case 4: boundary_cols<R, 4>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split); break;
-            case 8: boundary_cols<R, 8>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split); break;
-            case 16: boundary_cols<R, 16>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split); break;
+            case 8:
+                if constexpr (std::is_same<R, float>::value)
+                    boundary_cols<R, 8>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split);
+                break;
+            case 16:
+                if constexpr (std::is_same<R, float>::value)
+                    boundary_cols<R, 16>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split);
+                break;
             default: throw Error(BAEMM_ERR_SIZE, "wave_chunk_size must be a power of two <= 64");
         }
-    BAEMM_LAUNCH_CHECK();
+    if (!d64) BAEMM_LAUNCH_CHECK();
     if (grid.z > 1)
     {
         split_sum_kernel<R><<<ceil_div(elems, 256), 256, 0, st>>>(out, (int)grid.z, elems, Ctri);
@@ -942,9 +965,10 @@ void launch_pack_points(int64_t m, const double *pts3, R *pts4, cudaStream_t st)
     BAEMM_LAUNCH_CHECK();
 }
 
-static int farfield_splits(const MeshDev &m, int wc, int wcs)
+static int farfield_splits(const MeshDev &m, int wc, int wcs, bool fp64)
 {
     const int cols = cols_for(wcs);
+    if (fp64 && cols >= 8) return dense_splits(d64_ctas(d64_unit(wc, wcs), m.nm, wc), m.nt, tc_sm_count());
     const int ctas = ceil_div(m.nm, kTargets) * (wc / cols);
     int splits = ceil_div(4 * 148, ctas);
     const int max_splits = ceil_div(m.nt, kTile);
@@ -953,9 +977,9 @@ static int farfield_splits(const MeshDev &m, int wc, int wcs)
     return splits;
 }
 
-size_t farfield_partial_elems(const MeshDev &m, int wc, int wcs)
+size_t farfield_partial_elems(const MeshDev &m, int wc, int wcs, bool fp64)
 {
-    return (size_t)farfield_splits(m, wc, wcs) * (size_t)m.nm * (size_t)wc;
+    return (size_t)farfield_splits(m, wc, wcs, fp64) * (size_t)m.nm * (size_t)wc;
 }
 
 template <class R>
@@ -964,26 +988,35 @@ void launch_farfield(const MeshDev &m, const OpFlags &f, const void *chunk_param
                      double2 *Cout, int64_t ldC, cudaStream_t st)
 {
     if (!(f.sl() || f.dl()) || m.nm == 0) return;
-    const int splits = farfield_splits(m, wc, wcs);
+    constexpr bool fp64 = std::is_same<R, double>::value;
+    int splits = farfield_splits(m, wc, wcs, fp64);
     BAEMM_REQUIRE((size_t)splits * m.nm * wc <= partial_cap, BAEMM_ERR_SIZE, "far-field partial buffer too small");
-    const int per_split = ceil_div(ceil_div(m.nt, splits), kTile) * kTile;
     const int cols = cols_for(wcs);
-    dim3 grid(ceil_div(m.nm, kTargets), wc / cols, splits);
     const auto *p = static_cast<const typename Prm<R>::type *>(chunk_params);
     const R *mid = geo_mid<R>(m), *nrm = geo_nrm<R>(m), *meas = geo_meas<R>(m);
     const int mm = (int)m.nm, n = (int)m.nt;
+    const int unit = fp64 && cols >= 8 ? 8 : kTile;   // sources a split is rounded up to
+    const int per_split = ceil_div(ceil_div(m.nt, splits), unit) * unit;
+    splits = ceil_div(m.nt, per_split);
+    dim3 grid(ceil_div(m.nm, kTargets), wc / cols, splits);
     switch (cols)
     {
         case 1: farfield_cols<R, 1>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial); break;
         case 2: farfield_cols<R, 2>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial); break;
         case 4: farfield_cols<R, 4>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial); break;
-        case 8: farfield_cols<R, 8>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial); break;
-        case 16: farfield_cols<R, 16>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial); break;
+        case 8:
+            if constexpr (fp64) launch_farfield_d64(m, f, p, wc, wcs, Btri, partial, per_split, st);
+            else farfield_cols<R, 8>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial);
+            break;
+        case 16:
+            if constexpr (fp64) launch_farfield_d64(m, f, p, wc, wcs, Btri, partial, per_split, st);
+            else farfield_cols<R, 16>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial);
+            break;
         default: throw Error(BAEMM_ERR_SIZE, "wave_chunk_size must be a power of two <= 64");
     }
-    BAEMM_LAUNCH_CHECK();
-    farfield_reduce_kernel<R><<<ceil_div((int64_t)mm * wc, 256), 256, 0, st>>>(partial, splits, mm, wc, alpha, beta,
-                                                                               Cout, ldC);
+    if (!(fp64 && cols >= 8)) BAEMM_LAUNCH_CHECK();
+    farfield_reduce_kernel<R><<<ceil_div((int64_t)mm * wc, 32), dim3(32, kReduceRows), 0, st>>>(partial, splits, mm, wc,
+                                                                                             alpha, beta, Cout, ldC);
     BAEMM_LAUNCH_CHECK();
 }
 

@@ -127,6 +127,22 @@ template <class R>
 void launch_boundary_dense(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
                            const cplx<R> *Btri, cplx<R> *Ctri, cudaStream_t st, SplitSpace<R> ws, int variant = -1,
                            int64_t row_begin = 0, int64_t row_end = -1);
+// ---- dense64.cu: the FP64 forms on the FP64 matrix instructions --------------------
+// They take chunks of 8 columns and more.  A work unit is `sets` wavenumbers of
+// tiles * 8 columns each; splits of `per_split` sources write partial blocks
+// (ceil(n / per_split) x m x wc), summed by the caller.
+struct D64Unit
+{
+    int sets = 1, tiles = 1;
+    int columns() const { return sets * tiles * 8; }
+};
+D64Unit d64_unit(int wc, int wcs);
+int64_t d64_ctas(const D64Unit &u, int64_t m, int wc);
+void launch_boundary_d64(const MeshDev &m, const OpFlags &f, const ChunkParamsD *prm, int wc, int wcs,
+                         const DenseTargets<double> &tg, const double2 *Btri, double2 *out, int per_split,
+                         cudaStream_t st);
+void launch_farfield_d64(const MeshDev &m, const OpFlags &f, const ChunkParamsD *prm, int wc, int wcs,
+                         const double2 *Btri, double2 *partial, int per_split, cudaStream_t st);
 // Near-field kernel (NearFieldOperatorKernel.cl:5-194): Cpts (npts x wc) =
 // K(kappa) Btri at the points pts4 (npts x 4 reals), single and double layer
 // (c1, c2) only, no pair excluded.  Same kernels and variants as the boundary form.
@@ -251,7 +267,7 @@ template <class R>
 void launch_farfield(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
                      const cplx<R> *Btri, cplx<R> *partial, size_t partial_cap, double2 alpha, double2 beta,
                      double2 *Cout, int64_t ldC, cudaStream_t st);
-size_t farfield_partial_elems(const MeshDev &m, int wc, int wcs);
+size_t farfield_partial_elems(const MeshDev &m, int wc, int wcs, bool fp64);
 // Herglotz kernel (HerglotzWaveKernel.cl:5-176) applied to conj(g).
 template <class R>
 void launch_herglotz(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,

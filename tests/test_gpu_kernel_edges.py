@@ -62,3 +62,53 @@ def test_kernel_variant_reads_back():
         for v in (2, 0, 1):
             H.SetKernelVariant(v)
             assert H.GetKernelVariant() == v
+
+
+GRIDS64 = [(3, 3), (4, 4), (5, 13), (8, 8), (15, 17), (19, 54)]
+
+
+@pytest.mark.parametrize("grid", GRIDS64)
+@pytest.mark.parametrize("wc,wcs,cname", [(16, 16, "bie"), (32, 16, "all"), (48, 16, "dtn"), (32, 32, "sl"), (64, 64, "all"),
+                                          (16, 8, "dtn"), (24, 8, "bie"), (8, 8, "all"), (8, 4, "all"), (2, 1, "sl")])
+def test_fp64_units(grid, wc, wcs, cname):
+    """18 to 2052 triangles (remainders of 8 sources and 16 targets, split and
+    unsplit) in every work unit of the FP64 form and in the chunk sizes below 8."""
+    got, ref = _apply(APPLY_FP64, grid, wc, wcs, cname)
+    assert relerr(got, ref) < TOL64
+
+
+def test_fp64_large_arguments():
+    """Phases beyond the fast argument reduction: kappa r up to about 1e6.  A
+    relative rounding of 1e-16 in r is 1e-10 in the phase there; 1e-8 leaves two digits."""
+    coords, tris = meshes.torus(n_minor=5, n_major=13)
+    B = crandn(np.random.default_rng(3), coords.shape[0], 16)
+    got, ref = np.zeros_like(B), np.zeros_like(B)
+    kap, coeff = np.array([2.0, 4e5]), np.array([COEFF["bie"](2.0), COEFF["all"](3.0)], np.complex128)
+    with Helmholtz_CUDA(coords, tris, meshes.fibonacci_sphere(4)) as H:
+        H.SetApplyMode(APPLY_FP64)
+        H.ApplyBoundaryOperators_PL(1.0, B, 0.0, got, kap, coeff, 16, 8)
+    O.Oracle(coords, tris, meshes.fibonacci_sphere(4), precision=64).ApplyBoundaryOperators_PL(
+        1.0, B, 0.0, ref, kap, coeff, 16, 8)
+    assert relerr(got, ref) < 1e-8
+
+
+@pytest.mark.parametrize("count", [1, 15, 17, 64, 65, 300])
+@pytest.mark.parametrize("wc,wcs", [(16, 16), (32, 16), (64, 32), (16, 8), (8, 8), (4, 2)])
+def test_fp64_far_and_near(count, wc, wcs):
+    """Directions and evaluation points that are not multiples of a block, beta on."""
+    coords, tris = meshes.torus(n_minor=7, n_major=19)
+    meas = meshes.fibonacci_sphere(count)
+    points = meshes.points_off_torus(count, seed=5)
+    kap = np.linspace(1.0, 5.0, wc // wcs)
+    rng = np.random.default_rng(11)
+    B, C0 = crandn(rng, coords.shape[0], wc), crandn(rng, count, wc)
+    coeff = np.array([COEFF["all"](k) for k in kap], np.complex128)
+    coeff[:, 3] = 0.0
+    orc = O.Oracle(coords, tris, meas, precision=64)
+    with Helmholtz_CUDA(coords, tris, meas) as H:
+        H.SetApplyMode(APPLY_FP64)
+        for name, extra in (("ApplyFarFieldOperators_PL", ()), ("ApplyNearFieldOperators_PL", (points,))):
+            got, ref = C0.copy(), C0.copy()
+            getattr(H, name)(0.7, B, 0.3, got, kap, coeff, wc, wcs, *extra)
+            getattr(orc, name)(0.7, B, 0.3, ref, kap, coeff, wc, wcs, *extra)
+            assert relerr(got, ref) < TOL64, name
