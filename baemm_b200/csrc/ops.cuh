@@ -23,7 +23,7 @@ struct MeshDev
     DevBuf<int32_t> avt_outer, avt_inner;
     DevBuf<int32_t> mass_outer, mass_inner;
     DevBuf<float> mid_f, nrm_f, area_f, a3_f, diag_f, mass_f, lumped_f, meas_f;
-    DevBuf<float> tgeo_f;        // tensor-core form: source geometry per 16-source tile (lazily built)
+    DevBuf<float> tgeo_f;        // tensor-core form: source geometry per source tile (lazily built)
     DevBuf<double> mid_d, nrm_d, area_d, a3_d, diag_d, mass_d, lumped_d, meas_d;
 };
 
@@ -169,7 +169,8 @@ struct TcCoeffForm
 };
 TcCoeffForm tc_coeff_form(const ChunkParamsF *host_params, int groups);
 // Settings of the tensor-core form (the autotuner's search space):
-//   seg_tiles  16-source tiles accumulated in TMEM before the partial sum is
+//   seg_tiles  groups of 16 sources accumulated in TMEM (rounded up to whole
+//              tiles of 32) before the partial sum is
 //              added to FP32 registers (bounds the tensor-core accumulation chain);
 //   ctas       persistent grid size (0: one CTA per SM);
 //   stagger    sweep offset between CTAs (tiles; -1: spread evenly);
@@ -200,9 +201,9 @@ void launch_nearfield_tc(const MeshDev &m, const OpFlags &f, const void *chunk_p
                          int wc, int wcs, const float *tgeo, const float *pts4, int64_t npts, const float2 *Btri,
                          float2 *Cpts, float2 *ws, size_t ws_elems, DevBuf<uint8_t> &img, int *err, cudaStream_t st,
                          const TcTuning &tune);
-// The tensor-core form's B operand: every 16-source tile's hi / lo images of
+// The tensor-core form's B operand: every source tile's hi / lo images of
 // B_tri (n x wc) per 16-column group, as the kernel's B stages hold them
-// (8 KB each); returns img's device block (grown as needed).
+// (16 KB each); returns img's device block (grown as needed).
 // Self-test of the bounded pipeline waits: one warp waits on an mbarrier that
 // nothing arrives on; returns the error code the wait wrote and its duration.
 void tc_bounded_wait_probe(int code, double *elapsed_ms, int *code_out);
@@ -255,7 +256,7 @@ int tc_pack_class(const OpFlags &f, int wc, const TcTuning &tune);
 // whatever it is packed with.
 void launch_boundary_tc_packed(const TcPackItem *items, int count, const OpFlags &f, const TcTuning &tune,
                                TcPackScratch &scratch, int *err, cudaStream_t st);
-// Source geometry of the tensor-core form, per 16-source tile (built once per mesh).
+// Source geometry of the tensor-core form, per source tile (built once per mesh).
 size_t tc_tile_geometry_floats(int64_t nt);
 void launch_tc_tile_geometry(const MeshDev &m, float *tgeo, cudaStream_t st);
 // float2 elements of the tensor-core workspace for a persistent grid of `ctas`

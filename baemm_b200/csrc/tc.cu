@@ -16,7 +16,7 @@
 // correction half); a tcgen05.mma costs about the same for N = 32 and 64.
 // which keeps ~21 bits per product (TF32 hi+lo), well inside 1e-5 relative.
 //
-// Work unit = (group of up to 4 chunks, block of 128 targets, 16-source tile).
+// Work unit = (group of up to 4 chunks, block of 128 targets, 32-source tile).
 // The grid is persistent (one CTA per SM, it holds all 512 TMEM columns).
 // Whole target blocks are dealt out in waves (all CTAs sweep the source tiles
 // in step, so the tiles in use stay cached); the blocks left over after the
@@ -27,8 +27,8 @@
 // (deterministic).
 // Warp roles (GW generator warps + 1 + 2 = 19 or 11 warps):
 //   warps 0 .. GW-1  generators: thread (lane quarter q = warp % 4, group
-//               g = warp / 4) owns target row 32 q + lane and 16 / (GW / 4)
-//               sources of each 16-source K tile; it evaluates the kernel
+//               g = warp / 4) owns target row 32 q + lane and 32 / (GW / 4)
+//               sources of each 32-source K tile; it evaluates the kernel
 //               entries in registers, two sources per FP32x2 instruction
 //               (geometry shared by all chunks), splits them into hi / lo and
 //               writes them straight into TMEM (tcgen05.st), so the A operand
@@ -43,6 +43,14 @@
 // Pipelines use mbarriers (A stages in TMEM, B and geometry stages in shared
 // memory).  All roles wait with mbarrier.try_wait, which suspends the warp in
 // hardware.
+// The generators bound it (instruction issue and the MUFU pipe, 60 % and 57 %
+// busy with 38400 triangles x 64 columns, the tensor pipe 38 %) unless four
+// groups share their entries (then the tensor pipe).  A tile of 32 sources
+// gives a thread eight entries per wait for a stage, publication and barrier
+// round, instead of four with tiles of 16: 19.0 instead of 27.0 instructions
+// per entry; 153600 triangles x 64 columns 95.0 -> 89.3 ms, 20480 x 64 (two
+// wavenumbers) 1343 -> 1105 us, the near field of 30246 triangles at 20011
+// points 1709 -> 1390 us, 5120 x 32 86 -> 76 us.
 // Every wait is bounded: on time-out the CTA raises a shared abort flag, writes
 // an error code for the host, waits (bounded) for its issued MMAs and frees
 // its TMEM before returning.
@@ -62,7 +70,7 @@ namespace
 {
 
 constexpr int TC_M = 128;          // targets per CTA (TMEM lanes)
-constexpr int TC_SRC = 16;         // sources per K tile
+constexpr int TC_SRC = 32;         // sources per K tile (two K halves of 16: a half is one swizzle row of the B images)
 constexpr int TC_N = 32;           // MMA N: 16 columns as (re | im)
 constexpr int TC_CHMAX = 4;        // chunks per work unit
 constexpr int TC_MAXCHUNKS = 32;   // wave_count <= 512 with wave_chunk_size 16
@@ -75,9 +83,9 @@ struct TcShape
     static_assert(GW == 8 || GW == 16, "8 or 16 generator warps");
     static constexpr int GEN_THREADS = 32 * GW;
     static constexpr int GROUPS = GW / 4;        // source groups of a tile (4 warps cover the 128 rows)
-    static constexpr int SPT = 16 / GROUPS;      // sources per generator thread and tile
+    static constexpr int SPT = TC_SRC / GROUPS;  // sources per generator thread and tile
     static constexpr int PPT = SPT / 2;          // their pairs
-    static constexpr int KPT = 2 * SPT;          // their K columns of an A stage
+    static constexpr int SPK = SPT / 4;          // their K steps (4 sources = 8 K columns each)
     static constexpr int CPG = 16 / GROUPS;      // right-hand sides per thread in the drain
 };
 // MMA-issuing warps of a block: two (each takes every other chunk), so that
@@ -95,25 +103,26 @@ constexpr int tc_mma_warps() { return CH / R >= 2 ? 2 : 1; }
 // generators + the bulk-copy warp + the MMA issuers
 template <int GW, int CH, int R>
 constexpr int tc_threads() { return 32 * GW + 32 + 32 * tc_mma_warps<GW, CH, R>(); }
-constexpr int TC_BSTAGES = 4;      // B image stages in shared memory (bulk copies of the expanded images)
-constexpr int TC_RSTAGES = 6;      // tile geometry stages (bulk copies)
+constexpr int TC_BSTAGES = 2;      // B image stages in shared memory (bulk copies of the expanded images)
+constexpr int TC_RSTAGES = 4;      // tile geometry stages (bulk copies)
 constexpr uint32_t TC_TMEM_COLS = 512;
 // per chunk: main (Ahi Bhi) and correction (Ahi Blo + Alo Bhi) accumulators;
 // an entry set of R chunks holds its R main parts, then its R corrections
 constexpr uint32_t TC_DCOLS = 2 * TC_N;
-// A stages in TMEM (one chunk of one tile each, 64 columns) take the columns
-// after the accumulator of a CH-chunk work unit: 4 stages for 4 chunks, 6 for
-// 2, 7 for 1.  Within a stage, K step ks (8 K columns) has its hi part at
+// A stages in TMEM (one entry set of one tile each, 128 columns) take the
+// columns after the accumulator of a CH-chunk work unit: 2 stages for 4 chunks,
+// 3 for 2 and for 1.  Within a stage, K step ks (8 K columns) has its hi part at
 // columns 16 ks .. 16 ks + 7 and its lo part right after, so a generator
-// thread writes the hi and lo parts of its K step with one 16-column store
+// thread writes the hi and lo parts of a K step with one 16-column store
 // (1.3 % faster than separate hi and lo halves of the stage).
+constexpr uint32_t TC_ACOLS = 4 * TC_SRC;
 template <int CH>
-constexpr int tc_astages() { return (int)(TC_TMEM_COLS / TC_DCOLS) - CH; }
-constexpr int TC_ASTAGES_MAX = (int)(TC_TMEM_COLS / TC_DCOLS) - 1;
+constexpr int tc_astages() { return (int)((TC_TMEM_COLS - CH * TC_DCOLS) / TC_ACOLS); }
+constexpr int TC_ASTAGES_MAX = (int)((TC_TMEM_COLS - TC_DCOLS) / TC_ACOLS);
 constexpr int TC_IMG = TC_N * 128;                   // one K-major SW128 image: 32 rows x 128 B
 constexpr uint64_t kWaitNs = 200ull * 1000 * 1000;   // 200 ms per wait (a pipeline stage takes microseconds)
 
-// Source geometry of one 16-source tile, structure of arrays (built once per
+// Source geometry of one tile, structure of arrays (built once per
 // mesh by tc_tile_geometry_kernel; padding sources past the end are zero).
 struct TcTileGeo
 {
@@ -122,15 +131,16 @@ struct TcTileGeo
 };
 static_assert(sizeof(TcTileGeo) % 16 == 0, "bulk copies move multiples of 16 bytes");
 
-// The right-hand sides of one 16-source tile and one 16-column group as the
-// MMA's B operand: the hi and the lo image (32 rows each, 8 KB; ordered within
-// an entry set as tc_expand_kernel describes), expanded once per apply into
-// global memory and bulk-copied into a B stage as they are.
-constexpr int TC_GROUP_BYTES = 2 * TC_IMG;
+// The right-hand sides of one tile and one 16-column group as the MMA's B
+// operand: per K half the hi and the lo image (32 rows of 128 bytes each;
+// ordered within an entry set as tc_expand_kernel describes), expanded once per
+// apply into global memory and bulk-copied into a B stage as they are.
+constexpr int TC_HALVES = TC_SRC / 16;
+constexpr int TC_GROUP_BYTES = TC_HALVES * 2 * TC_IMG;
 
 struct __align__(1024) TcSmem
 {
-    uint8_t img[TC_BSTAGES][TC_CHMAX][2][TC_IMG];   // per stage the unit's images as tc_expand_kernel lays them out
+    uint8_t img[TC_BSTAGES][TC_CHMAX][TC_HALVES * 2][TC_IMG];   // per stage the unit's images as tc_expand_kernel lays them out
     TcTileGeo geo[TC_RSTAGES];
     uint64_t a_full[TC_ASTAGES_MAX], a_empty[TC_ASTAGES_MAX];
     uint64_t b_full[TC_BSTAGES], b_empty[TC_BSTAGES];
@@ -365,7 +375,7 @@ __device__ __forceinline__ uint32_t img_off16(int row, int sp) { return (uint32_
 // pieces, CTA k taking blocks k, k + ctas, ...: in each wave every CTA sweeps
 // the source tiles from the first, in step with the others, so the tiles being
 // read at any time stay few and cached.  The remaining blocks ("tail") are
-// split evenly by 16-source tiles ("stream-K"): CTA k takes the tail units
+// split evenly by tiles ("stream-K"): CTA k takes the tail units
 // [tail_start(k), tail_start(k + 1)), where a unit is one tile of one block.
 // One problem of a packed launch (device memory; the fields of a single
 // launch's plan and arguments, per problem).  prm: the broadcast parameter
@@ -514,12 +524,30 @@ struct Pieces
     }
 };
 
-// The kernel entries of one wave chunk for this thread's PPT source pairs,
-// in the A operand's K order (Re A_s0, Re A_s1, Im A_s0, Im A_s1) per pair,
-// split into hi (the FP32 bits; the tensor core reads their top 19 as TF32)
-// and lo = x - trunc_tf32(x).  P: the chunk's broadcast pairs kappa, -kappa,
-// c1.x, c1.y, -c2.x, -c2.y, c3.x, c3.y.  Per pair: rinv = 1/r, r, dmu =
-// (z.mu_j)/r^3, dnu = (z.nu_i)/r^3 (zero rinv masks a pair).
+// (ax, ay) of a source pair in the A operand's K order (Re A_s0, Re A_s1,
+// Im A_s0, Im A_s1), split into hi (the FP32 bits; the tensor core reads their
+// top 19 as TF32) and lo = x - trunc_tf32(x).
+__device__ __forceinline__ void tc_split_pair(float2 ax, float2 ay, uint32_t *hi, uint32_t *lo)
+{
+    const float2 m1 = make_float2(-1.f, -1.f);
+    const float2 tx = make_float2(__uint_as_float(__float_as_uint(ax.x) & 0xffffe000u),
+                                  __uint_as_float(__float_as_uint(ax.y) & 0xffffe000u));
+    const float2 ty = make_float2(__uint_as_float(__float_as_uint(ay.x) & 0xffffe000u),
+                                  __uint_as_float(__float_as_uint(ay.y) & 0xffffe000u));
+    const float2 lx = __ffma2_rn(tx, m1, ax), ly = __ffma2_rn(ty, m1, ay);
+    hi[0] = __float_as_uint(ax.x);
+    hi[1] = __float_as_uint(ax.y);
+    hi[2] = __float_as_uint(ay.x);
+    hi[3] = __float_as_uint(ay.y);
+    lo[0] = __float_as_uint(lx.x);
+    lo[1] = __float_as_uint(lx.y);
+    lo[2] = __float_as_uint(ly.x);
+    lo[3] = __float_as_uint(ly.y);
+}
+
+// The kernel entries of one wave chunk for a source pair.  P: the chunk's
+// broadcast pairs kappa, -kappa, c1.x, c1.y, -c2.x, -c2.y, c3.x, c3.y.  Per
+// pair: rinv = 1/r, r, dmu = (z.mu_j)/r^3, dnu = (z.nu_i)/r^3 (zero rinv masks a pair).
 //   A = e^{i k r} h,  h = c1 / r + u + i k r (-u),  u = -(c2 dmu - c3 dnu):
 //   hx = c1x / r + ux + k r uy,   hy = c1y / r + uy - k r ux.
 // RI: every chunk's single-layer coefficient is imaginary and its double- and
@@ -527,119 +555,82 @@ struct Pieces
 // FarField.hpp), so u is real: hx = ux, hy = c1y / r - k r ux.  The sincos is
 // taken of -k r there, which gives -sin(k r) and saves the negation of the
 // rotation's real part.
-template <int PPT, bool SL, bool DL, bool ADL, bool RI>
-__device__ __forceinline__ void tc_entries(const float2 *__restrict__ P, const float2 (&rinv)[PPT],
-                                           const float2 (&r)[PPT], const float2 (&dmu)[PPT],
-                                           const float2 (&dnu)[PPT], uint32_t (&hi)[4 * PPT],
-                                           uint32_t (&lo)[4 * PPT])
+template <bool SL, bool DL, bool ADL, bool RI>
+__device__ __forceinline__ void tc_entry(const float2 *__restrict__ P, float2 rinv, float2 r, float2 dmu, float2 dnu,
+                                         uint32_t *hi, uint32_t *lo)
 {
     const float2 m1 = make_float2(-1.f, -1.f);
-    #pragma unroll
-    for (int p = 0; p < PPT; ++p)
+    float2 ax, ay;
+    if (RI)
     {
-        float2 ax, ay;
-        if (RI)
-        {
-            const float2 nkr = __fmul2_rn(P[1], r[p]);   // -k r
-            float sn0, cs0, sn1, cs1;
-            __sincosf(nkr.x, &sn0, &cs0);
-            __sincosf(nkr.y, &sn1, &cs1);
-            const float2 cs = make_float2(cs0, cs1), nsn = make_float2(sn0, sn1);   // cos(k r), -sin(k r)
-            float2 ux = make_float2(0.f, 0.f);
-            if (DL) ux = __fmul2_rn(P[4], dmu[p]);
-            if (ADL) ux = DL ? __ffma2_rn(P[6], dnu[p], ux) : __fmul2_rn(P[6], dnu[p]);
-            float2 hy;
-            if (DL || ADL) hy = SL ? __ffma2_rn(nkr, ux, __fmul2_rn(P[3], rinv[p])) : __fmul2_rn(nkr, ux);
-            else hy = __fmul2_rn(P[3], rinv[p]);
-            // (ax, ay) = (ux cs - hy sn, ux sn + hy cs)
-            ax = __ffma2_rn(hy, nsn, __fmul2_rn(ux, cs));
-            ay = __ffma2_rn(hy, cs, __fmul2_rn(ux, __fmul2_rn(m1, nsn)));
-            if (!(DL || ADL)) ax = __fmul2_rn(hy, nsn);
-        }
-        else
-        {
-            const float2 kr = __fmul2_rn(P[0], r[p]);
-            float sn0, cs0, sn1, cs1;
-            __sincosf(kr.x, &sn0, &cs0);
-            __sincosf(kr.y, &sn1, &cs1);
-            const float2 cs = make_float2(cs0, cs1), sn = make_float2(sn0, sn1);
-            float2 hx = make_float2(0.f, 0.f), hy = make_float2(0.f, 0.f);
-            if (SL)
-            {
-                hx = __fmul2_rn(P[2], rinv[p]);
-                hy = __fmul2_rn(P[3], rinv[p]);
-            }
-            if (DL || ADL)
-            {
-                float2 ux = make_float2(0.f, 0.f), uy = make_float2(0.f, 0.f);
-                if (DL) { ux = __fmul2_rn(P[4], dmu[p]); uy = __fmul2_rn(P[5], dmu[p]); }
-                if (ADL) { ux = __ffma2_rn(P[6], dnu[p], ux); uy = __ffma2_rn(P[7], dnu[p], uy); }
-                const float2 nkr = __fmul2_rn(P[1], r[p]);
-                hx = __ffma2_rn(kr, uy, __fadd2_rn(hx, ux));
-                hy = __ffma2_rn(nkr, ux, __fadd2_rn(hy, uy));
-            }
-            // (ax, ay) = (hx cs - hy sn, hx sn + hy cs)
-            ax = __ffma2_rn(hy, __fmul2_rn(m1, sn), __fmul2_rn(hx, cs));
-            ay = __ffma2_rn(hy, cs, __fmul2_rn(hx, sn));
-        }
-        const float2 tx = make_float2(__uint_as_float(__float_as_uint(ax.x) & 0xffffe000u),
-                                      __uint_as_float(__float_as_uint(ax.y) & 0xffffe000u));
-        const float2 ty = make_float2(__uint_as_float(__float_as_uint(ay.x) & 0xffffe000u),
-                                      __uint_as_float(__float_as_uint(ay.y) & 0xffffe000u));
-        const float2 lx = __ffma2_rn(tx, m1, ax), ly = __ffma2_rn(ty, m1, ay);
-        hi[4 * p + 0] = __float_as_uint(ax.x);
-        hi[4 * p + 1] = __float_as_uint(ax.y);
-        hi[4 * p + 2] = __float_as_uint(ay.x);
-        hi[4 * p + 3] = __float_as_uint(ay.y);
-        lo[4 * p + 0] = __float_as_uint(lx.x);
-        lo[4 * p + 1] = __float_as_uint(lx.y);
-        lo[4 * p + 2] = __float_as_uint(ly.x);
-        lo[4 * p + 3] = __float_as_uint(ly.y);
+        const float2 nkr = __fmul2_rn(P[1], r);   // -k r
+        float sn0, cs0, sn1, cs1;
+        __sincosf(nkr.x, &sn0, &cs0);
+        __sincosf(nkr.y, &sn1, &cs1);
+        const float2 cs = make_float2(cs0, cs1), nsn = make_float2(sn0, sn1);   // cos(k r), -sin(k r)
+        float2 ux = make_float2(0.f, 0.f);
+        if (DL) ux = __fmul2_rn(P[4], dmu);
+        if (ADL) ux = DL ? __ffma2_rn(P[6], dnu, ux) : __fmul2_rn(P[6], dnu);
+        float2 hy;
+        if (DL || ADL) hy = SL ? __ffma2_rn(nkr, ux, __fmul2_rn(P[3], rinv)) : __fmul2_rn(nkr, ux);
+        else hy = __fmul2_rn(P[3], rinv);
+        // (ax, ay) = (ux cs - hy sn, ux sn + hy cs)
+        ax = __ffma2_rn(hy, nsn, __fmul2_rn(ux, cs));
+        ay = __ffma2_rn(hy, cs, __fmul2_rn(ux, __fmul2_rn(m1, nsn)));
+        if (!(DL || ADL)) ax = __fmul2_rn(hy, nsn);
     }
+    else
+    {
+        const float2 kr = __fmul2_rn(P[0], r);
+        float sn0, cs0, sn1, cs1;
+        __sincosf(kr.x, &sn0, &cs0);
+        __sincosf(kr.y, &sn1, &cs1);
+        const float2 cs = make_float2(cs0, cs1), sn = make_float2(sn0, sn1);
+        float2 hx = make_float2(0.f, 0.f), hy = make_float2(0.f, 0.f);
+        if (SL)
+        {
+            hx = __fmul2_rn(P[2], rinv);
+            hy = __fmul2_rn(P[3], rinv);
+        }
+        if (DL || ADL)
+        {
+            float2 ux = make_float2(0.f, 0.f), uy = make_float2(0.f, 0.f);
+            if (DL) { ux = __fmul2_rn(P[4], dmu); uy = __fmul2_rn(P[5], dmu); }
+            if (ADL) { ux = __ffma2_rn(P[6], dnu, ux); uy = __ffma2_rn(P[7], dnu, uy); }
+            const float2 nkr = __fmul2_rn(P[1], r);
+            hx = __ffma2_rn(kr, uy, __fadd2_rn(hx, ux));
+            hy = __ffma2_rn(nkr, ux, __fadd2_rn(hy, uy));
+        }
+        // (ax, ay) = (hx cs - hy sn, hx sn + hy cs)
+        ax = __ffma2_rn(hy, __fmul2_rn(m1, sn), __fmul2_rn(hx, cs));
+        ay = __ffma2_rn(hy, cs, __fmul2_rn(hx, sn));
+    }
+    tc_split_pair(ax, ay, hi, lo);
 }
 
 // KI: RI with the structure of the BIE and DtN tuples over all chunks:
 // c1 = i s kappa with s common, c2 and c3 real and common.  Then
 //   hy = c1y / r - k r ux = kappa v,   v = s / r - r ux,
-// and ux, -ux and v are per source pair, shared by every chunk (computed with
-// the pair geometry): a chunk costs the phase, its sincos, hy, the rotation
-// and the split.
-template <int PPT>
-__device__ __forceinline__ void tc_entries_ki(const float2 *__restrict__ P, const float2 (&r)[PPT],
-                                              const float2 (&ux)[PPT], const float2 (&nux)[PPT],
-                                              const float2 (&v)[PPT], uint32_t (&hi)[4 * PPT],
-                                              uint32_t (&lo)[4 * PPT])
+// and ux and v are per source pair, shared by every chunk (computed with the
+// pair geometry): a chunk costs the phase, its sincos, hy, the rotation and the
+// split.  (A shared -ux would save one of its instructions, but its registers
+// for four pairs spill.)
+__device__ __forceinline__ void tc_entry_ki(const float2 *__restrict__ P, float2 r, float2 ux, float2 v, uint32_t *hi,
+                                            uint32_t *lo)
 {
     const float2 m1 = make_float2(-1.f, -1.f);
-    #pragma unroll
-    for (int p = 0; p < PPT; ++p)
-    {
-        const float2 nkr = __fmul2_rn(P[1], r[p]);   // -k r
-        float sn0, cs0, sn1, cs1;
-        __sincosf(nkr.x, &sn0, &cs0);
-        __sincosf(nkr.y, &sn1, &cs1);
-        const float2 cs = make_float2(cs0, cs1), nsn = make_float2(sn0, sn1);   // cos(k r), -sin(k r)
-        const float2 hy = __fmul2_rn(P[0], v[p]);
-        // (ax, ay) = (ux cs - hy sn, ux sn + hy cs)
-        const float2 ax = __ffma2_rn(hy, nsn, __fmul2_rn(ux[p], cs));
-        const float2 ay = __ffma2_rn(hy, cs, __fmul2_rn(nux[p], nsn));
-        const float2 tx = make_float2(__uint_as_float(__float_as_uint(ax.x) & 0xffffe000u),
-                                      __uint_as_float(__float_as_uint(ax.y) & 0xffffe000u));
-        const float2 ty = make_float2(__uint_as_float(__float_as_uint(ay.x) & 0xffffe000u),
-                                      __uint_as_float(__float_as_uint(ay.y) & 0xffffe000u));
-        const float2 lx = __ffma2_rn(tx, m1, ax), ly = __ffma2_rn(ty, m1, ay);
-        hi[4 * p + 0] = __float_as_uint(ax.x);
-        hi[4 * p + 1] = __float_as_uint(ax.y);
-        hi[4 * p + 2] = __float_as_uint(ay.x);
-        hi[4 * p + 3] = __float_as_uint(ay.y);
-        lo[4 * p + 0] = __float_as_uint(lx.x);
-        lo[4 * p + 1] = __float_as_uint(lx.y);
-        lo[4 * p + 2] = __float_as_uint(ly.x);
-        lo[4 * p + 3] = __float_as_uint(ly.y);
-    }
+    const float2 nkr = __fmul2_rn(P[1], r);   // -k r
+    float sn0, cs0, sn1, cs1;
+    __sincosf(nkr.x, &sn0, &cs0);
+    __sincosf(nkr.y, &sn1, &cs1);
+    const float2 cs = make_float2(cs0, cs1), nsn = make_float2(sn0, sn1);   // cos(k r), -sin(k r)
+    const float2 hy = __fmul2_rn(P[0], v);
+    // (ax, ay) = (ux cs - hy sn, ux sn + hy cs)
+    tc_split_pair(__ffma2_rn(hy, nsn, __fmul2_rn(ux, cs)), __ffma2_rn(hy, cs, __fmul2_rn(m1, __fmul2_rn(ux, nsn))), hi,
+                  lo);
 }
 
-// RI, KI: see tc_entries and tc_entries_ki.  GW: generator warps (TcShape).
+// RI, KI: see tc_entry and tc_entry_ki.  GW: generator warps (TcShape).
 // PACK: a packed launch over plan.probs (the pointer arguments are unused).
 // R: groups of 16 columns that share one evaluation of the kernel entries (the
 // KI form, whose entries depend on a group only through its wavenumber, with
@@ -657,7 +648,7 @@ boundary_tc_kernel(const float *__restrict__ mid4, const float *__restrict__ nrm
                    const ChunkParamsF *__restrict__ prm, const TcPlan plan, int *err)
 {
     constexpr int TC_GEN_THREADS = TcShape<GW>::GEN_THREADS;
-    constexpr int TC_SPT = TcShape<GW>::SPT, TC_PPT = TcShape<GW>::PPT, TC_KPT = TcShape<GW>::KPT;
+    constexpr int TC_SPT = TcShape<GW>::SPT, TC_PPT = TcShape<GW>::PPT, TC_SPK = TcShape<GW>::SPK;
     constexpr int TC_CPG = TcShape<GW>::CPG;
     static_assert(R == 1 || (KI && !PACK && CH % R == 0), "shared entry sets need the KI form and R | CH");
     constexpr int E = CH / R;   // entry sets per tile
@@ -727,7 +718,7 @@ boundary_tc_kernel(const float *__restrict__ mid4, const float *__restrict__ nrm
         const int row = q * 32 + lane;
         const uint32_t lane_addr = tbase + ((uint32_t)(q * 32) << 16);
         constexpr int AS = tc_astages<CH>();
-        const uint32_t a_addr = lane_addr + (uint32_t)(CH * TC_DCOLS + g * 2 * TC_KPT);
+        const uint32_t a_addr = lane_addr + (uint32_t)(CH * TC_DCOLS + g * 16 * TC_SPK);
         float2 *acc_row = &sm.acc[row][g * TC_CPG];
         bool ok = true;
         bool pend = false;          // an A stage is written and not yet published
@@ -848,8 +839,8 @@ boundary_tc_kernel(const float *__restrict__ mid4, const float *__restrict__ nrm
                     }
                 }
                 mbar_arrive(&sm.r_empty[rs]);
-                // KI: ux = -(c2 dmu - c3 dnu), -ux and v = s / r - r ux per pair (every chunk's c2, c3 and s)
-                float2 kux[TC_PPT], knux[TC_PPT], kv[TC_PPT];
+                // KI: ux = -(c2 dmu - c3 dnu) and v = s / r - r ux per pair (every chunk's c2, c3 and s)
+                float2 kux[TC_PPT], kv[TC_PPT];
                 if (KI)
                 {
                     const float2 s2 = make_float2(V.ki_s, V.ki_s);
@@ -860,35 +851,37 @@ boundary_tc_kernel(const float *__restrict__ mid4, const float *__restrict__ nrm
                         if (DL) ux = __fmul2_rn(Pg[4], dmu[p]);
                         if (ADL) ux = DL ? __ffma2_rn(Pg[6], dnu[p], ux) : __fmul2_rn(Pg[6], dnu[p]);
                         kux[p] = ux;
-                        knux[p] = make_float2(-ux.x, -ux.y);
-                        kv[p] = __ffma2_rn(r[p], knux[p], __fmul2_rn(s2, rinv[p]));
+                        kv[p] = __ffma2_rn(r[p], make_float2(-ux.x, -ux.y), __fmul2_rn(s2, rinv[p]));
                     }
                 }
                 #pragma unroll
                 for (int e = 0; e < E; ++e)
                 {
-                    uint32_t hi[TC_KPT], lo[TC_KPT];
-                    if (KI) tc_entries_ki<TC_PPT>(Pg + 8 * (e * R), r, kux, knux, kv, hi, lo);
-                    else tc_entries<TC_PPT, SL, DL, ADL, RI>(Pg + 8 * e, rinv, r, dmu, dnu, hi, lo);
                     const uint32_t u = (uint32_t)T * E + e;
                     const uint32_t stage = u % AS;
-                    // (8 warps) publish the previous set's stage now that its stores had this math to land
-                    publish();
-                    // the stage is free once the MMAs that read it AS sets ago completed
-                    if (!warp_wait(&sm.a_empty[stage], ((u / AS) & 1u) ^ 1u, abort_flag, err, 3))
-                    {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
                     #pragma unroll
-                    for (int h = 0; h < TC_KPT / 8; ++h)
+                    for (int h = 0; h < TC_SPK; ++h)
                     {
-                        uint32_t v[16];
+                        uint32_t v[16];   // the K step's hi part, then its lo part
                         #pragma unroll
-                        for (int k = 0; k < 8; ++k) { v[k] = hi[8 * h + k]; v[8 + k] = lo[8 * h + k]; }
-                        tmem_st16(a_addr + stage * 64u + 16u * h, v);
+                        for (int p = 0; p < 2; ++p)
+                        {
+                            const int q2 = 2 * h + p;
+                            if (KI) tc_entry_ki(Pg + 8 * (e * R), r[q2], kux[q2], kv[q2], &v[4 * p], &v[8 + 4 * p]);
+                            else tc_entry<SL, DL, ADL, RI>(Pg + 8 * e, rinv[q2], r[q2], dmu[q2], dnu[q2], &v[4 * p],
+                                                           &v[8 + 4 * p]);
+                        }
+                        if (h == 0)
+                        {
+                            // (8 warps) publish the previous set's stage now that its stores had this math to land
+                            publish();
+                            // the stage is free once the MMAs that read it AS sets ago completed
+                            if (!warp_wait(&sm.a_empty[stage], ((u / AS) & 1u) ^ 1u, abort_flag, err, 3)) ok = false;
+                            tc_fence_after();
+                        }
+                        if (ok) tmem_st16(a_addr + stage * TC_ACOLS + 16u * h, v);
                     }
+                    if (!ok) break;
                     pend = true;
                     pend_stage = stage;
                     // 16 warps: publish at once, the issuers wait for it; the other three
@@ -1029,7 +1022,7 @@ boundary_tc_kernel(const float *__restrict__ mid4, const float *__restrict__ nrm
                     }
                     tc_fence_after();
                     const uint32_t d = tbase + (uint32_t)(c0 * TC_DCOLS);
-                    const uint32_t a_hi = tbase + (uint32_t)(CH * TC_DCOLS) + stage * 64u;
+                    const uint32_t a_hi = tbase + (uint32_t)(CH * TC_DCOLS) + stage * TC_ACOLS;
                     const uint32_t a_lo = a_hi + 8u;
                     // the set's R hi images (32 rows each) are followed by its R lo
                     // images (same 1024-byte group stride): one N = 64 R operand
@@ -1049,9 +1042,10 @@ boundary_tc_kernel(const float *__restrict__ mid4, const float *__restrict__ nrm
                     if (elect_one())
                     {
                         #pragma unroll
-                        for (int ks = 0; ks < 4; ++ks)
+                        for (int ks = 0; ks < 4 * TC_HALVES; ++ks)
                         {
-                            const uint64_t koff = (uint64_t)(ks * 32 >> 4);
+                            // 32 bytes per K step within a half's images, R hi and R lo images per half
+                            const uint64_t koff = (uint64_t)((ks % 4 * 32 + ks / 4 * (R * 2 * TC_IMG)) >> 4);
                             // [main | corr] (+)= Ahi [Bhi | Blo];  corr += Alo Bhi (each over the set's chunks)
                             mma_tf32(d, a_hi + 16u * ks, b_hilo + koff, (!first || ks > 0) ? 1u : 0u,
                                      idesc_tf32(2 * TC_N * R));
@@ -1090,30 +1084,30 @@ boundary_tc_kernel(const float *__restrict__ mid4, const float *__restrict__ nrm
     }
 }
 
-// The MMA's B operand for every 16-source tile t and 16-column group G, as the
-// bytes a B stage holds: a hi and a lo image, each 32 K-major SWIZZLE_128B
-// rows of 128 bytes.  The groups of tile t take TC_GROUP_BYTES each from
-// t * groups * TC_GROUP_BYTES; within each aligned block of `share` groups
-// (the groups that share one evaluation of the kernel entries) the hi images
-// come first, then the lo images, so that one MMA reads [Bhi | Blo] of the
-// whole block and another its Bhi (share = 1: hi, lo per group).  Row
+// The MMA's B operand for every tile t and 16-column group G, as the bytes a B
+// stage holds: per K half (16 sources) a hi and a lo image, each 32 K-major
+// SWIZZLE_128B rows of 128 bytes.  The groups of tile t take TC_GROUP_BYTES each
+// from t * groups * TC_GROUP_BYTES; within each aligned block of `share` groups
+// (the groups that share one evaluation of the kernel entries) every half's hi
+// images come first, then its lo images, so that one MMA reads [Bhi | Blo] of
+// the whole block and another its Bhi (share = 1: hi, lo per half).  Row
 // q < 16 (real part of column q's result) holds per source pair
 // sp = (s0, s1) = (2 sp, 2 sp + 1) the 16-byte group (Re b_s0, Re b_s1,
 // -Im b_s0, -Im b_s1); row 16 + q holds (Im b_s0, Im b_s1, Re b_s0, Re b_s1);
 // group sp of row r sits at ((sp ^ (r & 7)) * 16) (img_off16).  hi = tf32(x)
 // rounded to nearest, lo = x - hi (split_tf32).  Sources past n are zero.
-// Thread (t, G, q, sp), sp fastest: 8 threads fill one row's 128 bytes.
+// Thread (t, G, half, q, sp), sp fastest: 8 threads fill one row's 128 bytes.
 __global__ void tc_expand_kernel(const float2 *__restrict__ Btri, int n, int wc, int64_t total, int share,
                                  uint8_t *__restrict__ img)
 {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= total) return;
     const int groups = wc / 16;
-    const int sp = (int)(e & 7), q = (int)((e >> 3) & 15);
-    const int64_t tg = e >> 7;                       // t * groups + G
+    const int sp = (int)(e & 7), q = (int)((e >> 3) & 15), half = (int)((e >> 7) % TC_HALVES);
+    const int64_t tg = e / (128 * TC_HALVES);        // t * groups + G
     const int64_t t = tg / groups;
     const int G = (int)(tg - t * groups);
-    const int64_t j0 = t * TC_SRC + 2 * sp;
+    const int64_t j0 = t * TC_SRC + half * 16 + 2 * sp;
     const int col = G * 16 + q;
     const float2 v0 = j0 < n ? Btri[j0 * wc + col] : make_float2(0.f, 0.f);
     const float2 v1 = j0 + 1 < n ? Btri[(j0 + 1) * wc + col] : make_float2(0.f, 0.f);
@@ -1124,7 +1118,7 @@ __global__ void tc_expand_kernel(const float2 *__restrict__ Btri, int n, int wc,
     split_tf32(v1.y, hi1, li1);
     constexpr uint32_t sgn = 0x80000000u;
     const int r = G % share;   // place in the block of groups sharing the entries
-    uint8_t *blk = img + (tg - r) * TC_GROUP_BYTES;
+    uint8_t *blk = img + (tg - r) * TC_GROUP_BYTES + half * (share * 2 * TC_IMG);
     uint8_t *hi_img = blk + r * TC_IMG, *lo_img = blk + (share + r) * TC_IMG;
     *reinterpret_cast<uint4 *>(hi_img + img_off16(q, sp)) = make_uint4(hr0, hr1, hi0 ^ sgn, hi1 ^ sgn);
     *reinterpret_cast<uint4 *>(lo_img + img_off16(q, sp)) = make_uint4(lr0, lr1, li0 ^ sgn, li1 ^ sgn);
@@ -1132,7 +1126,7 @@ __global__ void tc_expand_kernel(const float2 *__restrict__ Btri, int n, int wc,
     *reinterpret_cast<uint4 *>(lo_img + img_off16(q + 16, sp)) = make_uint4(li0, li1, lr0, lr1);
 }
 
-// Midpoints and normals of each 16-source tile as structure of arrays (zeros
+// Midpoints and normals of each tile as structure of arrays (zeros
 // past the last triangle).
 __global__ void tc_tile_geometry_kernel(const float *__restrict__ mid4, const float *__restrict__ nrm4,
                                         TcTileGeo *__restrict__ out, int n, int ntiles)
@@ -1159,7 +1153,7 @@ const uint8_t *launch_tc_expand(const float2 *Btri, int64_t n, int wc, DevBuf<ui
     const int64_t ntiles = ceil_div(n, TC_SRC), groups = wc / 16;
     const size_t bytes = (size_t)(ntiles * groups) * TC_GROUP_BYTES;
     uint8_t *out = img.reserve(bytes);
-    const int64_t total = ntiles * groups * 128;
+    const int64_t total = ntiles * groups * 128 * TC_HALVES;
     if (total > 0)
     {
         tc_expand_kernel<<<ceil_div(total, 256), 256, 0, st>>>(Btri, (int)n, wc, total, share, out);
@@ -1343,6 +1337,9 @@ size_t tc_workspace_elems(int ctas)
     return (size_t)ctas * 2 * TC_M * TC_CHMAX * 16;
 }
 
+// Settings count 16-source tiles; the kernel's tiles hold TC_SRC sources.
+static int tc_tiles(int tiles16) { return ceil_div((int64_t)tiles16 * 16, TC_SRC); }
+
 size_t tc_tile_geometry_floats(int64_t nt) { return (size_t)ceil_div(nt, TC_SRC) * (sizeof(TcTileGeo) / sizeof(float)); }
 
 void launch_tc_tile_geometry(const MeshDev &m, float *tgeo, cudaStream_t st)
@@ -1409,14 +1406,14 @@ void tc_run(const MeshDev &m, const OpFlags &f, const void *chunk_params, const 
     plan.ncg = wc / (16 * CH);
     plan.nblk = ceil_div(plan.m, TC_M);
     plan.ntiles = ceil_div(plan.n, TC_SRC);
-    plan.seg_tiles = std::max(1, tune.seg_tiles);
+    plan.seg_tiles = std::max(1, tc_tiles(tune.seg_tiles));
     const int blocks = plan.ncg * plan.nblk;
     const int ctas = tune.ctas > 0 ? tune.ctas : device_sm_count();
     plan.ctas = (int)std::min<int64_t>(ctas, (int64_t)blocks * plan.ntiles);
     plan.full_waves = blocks / plan.ctas;
     plan.tail_blocks = blocks - plan.full_waves * plan.ctas;
     plan.tail_units = (int64_t)plan.tail_blocks * plan.ntiles;
-    plan.stagger = tune.stagger;
+    plan.stagger = tune.stagger < 0 ? -1 : tc_tiles(tune.stagger);
     plan.ki_s = form.s;
     BAEMM_REQUIRE(ws && ws_elems >= tc_workspace_elems(plan.ctas), BAEMM_ERR_ARG, "tensor-core workspace too small");
     const int code = (f.sl() ? 1 : 0) | (f.dl() ? 2 : 0) | (f.adl() ? 4 : 0);
@@ -1633,7 +1630,7 @@ void launch_boundary_tc_packed(const TcPackItem *items, int count, const OpFlags
     uint8_t *dev = scr.stage(host.data(), total, st);
     TcPlan plan{};
     plan.ctas = ctas;
-    plan.seg_tiles = std::max(1, tune.seg_tiles);
+    plan.seg_tiles = std::max(1, tc_tiles(tune.seg_tiles));
     plan.probs = reinterpret_cast<const TcProblem *>(dev);
     plan.cta_begin = reinterpret_cast<const int *>(dev + off_beg);
     plan.pieces = reinterpret_cast<const int2 *>(dev + off_piece);

@@ -138,8 +138,9 @@ int baemm_get_apply_mode(const baemm_ctx *ctx);
  *                             packed FP32x2 with 1 / 2 targets per thread; not
  *                             set (the default, read back as 0): the library
  *                             chooses
- *   BAEMM_TUNE_TC_SEGMENT     tensor-core form: 16-source tiles accumulated in
- *                             TMEM before each partial sum is added to the FP32
+ *   BAEMM_TUNE_TC_SEGMENT     tensor-core form: groups of 16 sources accumulated
+ *                             in TMEM (rounded up to an even number of groups)
+ *                             before each partial sum is added to the FP32
  *                             sums in shared memory (default 16; bounds the
  *                             tensor-core accumulation chain)
  *   BAEMM_TUNE_TC_CTAS        tensor-core form: persistent grid size (default 0 =

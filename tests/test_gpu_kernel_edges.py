@@ -42,6 +42,20 @@ def test_tensor_core_split_blocks(ctas):
     assert relerr(got, ref) < TOL32
 
 
+@pytest.mark.parametrize("gen_warps,seg", [(16, 1), (16, 16), (8, 3)])
+@pytest.mark.parametrize("grid", [(3, 3), (4, 4), (3, 8), (5, 13), (8, 8), (15, 17), (19, 54)])
+@pytest.mark.parametrize("wc,wcs,cname", [(16, 16, "bie"), (32, 16, "all"), (32, 32, "dtn"), (64, 16, "bie"), (64, 32, "dtn"),
+                                          (64, 64, "bie"), (64, 16, "all")])
+def test_tensor_core_tiles(gen_warps, seg, grid, wc, wcs, cname):
+    """18 to 2052 triangles: less than a 32-source tile, one half of it, whole
+    tiles and remainders, with every number of groups per entry set and per unit."""
+    def setup(H):
+        H.SetTuning(_capi.TUNE_TC_GEN_WARPS, gen_warps)
+        H.SetTuning(_capi.TUNE_TC_SEGMENT, seg)
+    got, ref = _apply(APPLY_TC, grid, wc, wcs, cname, setup)
+    assert relerr(got, ref) < TOL32
+
+
 @pytest.mark.parametrize("variant", [None, 0, 1, 2])
 @pytest.mark.parametrize("grid", [(3, 3), (4, 4), (5, 13), (16, 8), (15, 17), (16, 16), (19, 54)])
 @pytest.mark.parametrize("wc,wcs,cname", [(16, 16, "bie"), (32, 32, "all"), (24, 8, "dtn"), (8, 4, "all"), (4, 2, "bie"),
