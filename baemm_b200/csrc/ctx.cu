@@ -71,6 +71,12 @@ void Ctx::init_mesh(const double *coords, int64_t nv, const int32_t *tris, int64
     mesh.area_d.reserve(nt); mesh.a3_d.reserve(nt); mesh.diag_d.reserve(nt);
     mesh.mass_f.reserve(mass_inner_h.size()); mesh.mass_d.reserve(mass_inner_h.size());
     mesh.lumped_f.reserve(nv); mesh.lumped_d.reserve(nv);
+    if (nv <= kMassEllMaxRows)
+    {
+        mesh.mass_ell_idx.reserve(kMassEll * nv);
+        mesh.mass_ell_f.reserve(kMassEll * nv);
+        mesh.mass_ell_d.reserve(kMassEll * nv);
+    }
     launch_geometry(mesh, false, stream);
     launch_geometry(mesh, true, stream);
     launch_mass_values(mesh, false, stream);

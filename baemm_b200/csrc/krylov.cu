@@ -5,9 +5,12 @@
 // order.
 #include "krylov.cuh"
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 namespace baemm
@@ -394,142 +397,202 @@ __global__ void cg_pupdate_kernel(int64_t total, int c, const double *__restrict
     p[e] = z[e] + col[3 * c + k] * p[e];
 }
 
-// CG mass inverse on meshes of up to kCgBlockMaxRows vertices: one block per
-// column, every iteration in one launch.  The CG's columns are independent
-// (each has its own dot products and step lengths), so a block that owns a
-// column needs no other block: the phases of an iteration are separated by
-// __syncthreads only, and the 3 launches and 3 cross-block column sums of
-// an iteration of the multi-block kernels become block sums.  The block's
-// vectors are column-major in global memory (column k at x + k n),
-// L2-resident at these sizes, except the search direction p, which lives in
-// the block's shared memory (n doubles, at most 128 KB): the matvec's gathers
-// of p read shared memory instead of L2.  Same steps and stopping rule as the
-// multi-block kernels (ApplyMassInverse.hpp:48-156): x = 0, r = b, z = L r,
-// p = z; per iteration q = M p, alpha = <r,z> / <p,q>, x += alpha p,
-// r -= alpha q, z = L r, beta = <r,z>_new / <r,z>, converged once
-// ||r|| <= tol ||b|| (a column of zeros at once), p = z + beta p.  Block sums
-// add the threads' row-ordered partials by a fixed shuffle and shared-memory
-// tree, so runs are reproducible.  flags: [0] columns not converged, [1] the
-// largest iteration count (both zeroed before the launch), [2 + k] column k
-// converged.
-constexpr int kCgBlockThreads = 1024;
-// Up to this many rows one block per column is faster: on the icosphere of
-// level 5 (10242 vertices, 128 real columns) one iteration takes 26.5 us
-// against 60.3 us for the three multi-block kernels; on level 6 (40962
-// vertices, 64 columns) 130 us against 92 us, too few blocks for the rows.
-// The bound also keeps p (n doubles) within a block's shared memory.
-constexpr int64_t kCgBlockMaxRows = 16384;
+// CG mass inverse on meshes of up to kMassEllMaxRows vertices: a cluster of S = 1
+// to 8 blocks owns a column and runs every iteration in one launch (the CG's
+// columns are independent: each has its own dot products and step lengths).  Its
+// blocks split the rows.  In shared memory a block holds the whole search
+// direction p, so the matvec's gathers stay on the SM, its rows of x, r and q
+// and, where they fit, of the matrix (8 slots per row, slot-major, so that a warp
+// reads 32 rows of a slot at once; a row's entries past 8 come from the CSR
+// arrays).  Block sums and the new p go to the other blocks through distributed
+// shared memory.  An iteration has three cluster barriers: after <p, q>, after
+// the residual's dots, and after the new p.  Same steps and stopping rule as the
+// multi-block kernels (ApplyMassInverse.hpp:48-156): x = 0, r = b, p = L r; per
+// iteration q = M p, alpha = <r,z> / <p,q>, x += alpha p, r -= alpha q, z = L r,
+// beta = <r,z>_new / <r,z>, converged once ||r|| <= tol ||b|| (a column of zeros
+// at once), p = z + beta p.  All sums are in fixed orders, so runs are
+// reproducible.  flags: [0] columns not converged, [1] the largest iteration
+// count (both zeroed before the launch), [2 + k] column k converged.
+//
+// Bound by latency (barriers, block sums) on small meshes and by the matrix
+// stream from L2 where it does not fit.  One block per column, the CSR rows read
+// one thread per row (uncoalesced) and the vectors in global memory, took 28.4 us
+// per iteration on 10242 vertices x 64 columns and 9.2 us on 2562 x 64.
+// Now, per iteration of a solve's 20: 3.1 us on 642 x 64, 5.2 on 2562 x 64 (two
+// blocks a column), 14.6 on 10242 x 64 (two blocks a column, matrix from L2).
+// 512 threads: the block sums shuffle every warp's doubles through one shuffle
+// unit (1024 threads took 5.95 instead of 5.1 us per iteration on 2562 x 64);
+// the matrix rows in registers made no difference.
+constexpr int kCgThreads = 512, kCgCluster = 8;
+constexpr size_t kCgSmemBytes = 226 * 1024;   // of 227 KB, beside the static arrays
 
-// totals of a and b over the block, in every thread (red: 2 x 33 doubles)
-__device__ __forceinline__ void block_sum2(double &a, double &b, double *red)
+struct CgShape
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    int S = 0, rpc = 0;   // blocks per column, rows per block
+    int staged = 0;       // in shared memory: 1 the lumped inverse, 2 the matrix rows too
+    size_t bytes = 0;
+};
+
+// The cluster size with the least estimated time among those whose vectors fit
+// shared memory: (waves of blocks) x (cycles of an iteration), fitted to the
+// measured ones: 5000 fixed (block sums, divisions, the launch's share), 1000 for
+// the cluster's barriers, and per row of a block 2.4, 0.6 per other block that
+// its p is sent to, and 1 for a matrix row from L2.  Of clusters of 8, fewer fit
+// the chip at a time (16 of them on 148 SMs took two waves).
+template <class RV>
+CgShape cg_cluster_shape(int64_t n, int c, int sms)
+{
+    CgShape best;
+    double best_cost = 0.0;
+    for (int S = 1; S <= kCgCluster; S *= 2)
     {
-        a += __shfl_down_sync(0xffffffffu, a, o);
-        b += __shfl_down_sync(0xffffffffu, b, o);
+        CgShape h;
+        h.S = S;
+        h.rpc = ceil_div(n, S);
+        const size_t vec = ((size_t)n + 3 * (size_t)h.rpc) * 8, lump = (size_t)h.rpc * sizeof(RV);
+        const size_t mat = (size_t)h.rpc * kMassEll * (sizeof(RV) + 2);
+        if (vec > kCgSmemBytes) continue;
+        h.staged = vec + lump + mat <= kCgSmemBytes ? 2 : vec + lump <= kCgSmemBytes ? 1 : 0;
+        h.bytes = vec + (h.staged ? lump : 0) + (h.staged == 2 ? mat : 0);
+        const double cost = (double)ceil_div((int64_t)c * S, S < 8 ? sms : sms * 3 / 4) * 
+                            (5000.0 + 1000.0 * (S > 1) + h.rpc * (2.4 + 0.6 * (S - 1) + (h.staged == 2 ? 0.0 : 1.0)));
+        if (best.S == 0 || cost < best_cost) { best = h; best_cost = cost; }
     }
-    __syncthreads();   // red is free (its previous totals have been read)
-    if (lane == 0) { red[warp] = a; red[33 + warp] = b; }
-    __syncthreads();
-    if (warp == 0)
-    {
-        double ta = lane < nw ? red[lane] : 0.0, tb = lane < nw ? red[33 + lane] : 0.0;
-        #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-        {
-            ta += __shfl_down_sync(0xffffffffu, ta, o);
-            tb += __shfl_down_sync(0xffffffffu, tb, o);
-        }
-        if (lane == 0) { red[32] = ta; red[65] = tb; }
-    }
-    __syncthreads();
-    a = red[32];
-    b = red[65];
+    return best;
 }
 
 template <class RV>
-__global__ void __launch_bounds__(kCgBlockThreads, 1)
-cg_block_kernel(int64_t n, int c, const double *__restrict__ b, int64_t ldb, const int32_t *__restrict__ mo,
-                const int32_t *__restrict__ mi, const RV *__restrict__ mv, const RV *__restrict__ L, double *xs,
-                double *rs, double *zs, double *qs, double *__restrict__ y, int64_t ldy, int *flags,
-                double tol, int max_iter)
+__global__ void __launch_bounds__(kCgThreads, 1)
+cg_cluster_kernel(int64_t n, int rpc, int staged, const double *b, int64_t ldb, const int32_t *__restrict__ mo,
+                  const int32_t *__restrict__ mi, const RV *__restrict__ mv, const uint16_t *__restrict__ ell_idx,
+                  const RV *__restrict__ ell_val, const RV *__restrict__ L, double *y, int64_t ldy, int *flags,
+                  double tol, int max_iter)
 {
-    __shared__ double red[66];
-    extern __shared__ double p[];   // the column's search direction, n doubles
-    const int k = blockIdx.x;
-    const int64_t off = (int64_t)k * n;
-    // the column's vectors are separate buffers: no aliasing, so the loads of a
-    // thread's next row can be issued before the stores of its current one
-    double *__restrict__ x = xs + off;
-    double *__restrict__ r = rs + off;
-    double *__restrict__ z = zs + off;
-    double *__restrict__ q = qs + off;
-    double rz = 0.0, bb = 0.0;
-    for (int64_t row = threadIdx.x; row < n; row += blockDim.x)
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    __shared__ double red[2][kCgThreads / 32];
+    __shared__ double xch[3][kCgCluster];   // every block's sums: <p, q>, <r, z>, <r, r>
+    extern __shared__ __align__(16) uint8_t raw[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5, T = blockDim.x;
+    const int k = blockIdx.x / S;
+    const int r0 = rank * rpc, m = max(0, min(rpc, (int)n - r0));   // rows of this block
+    double *p = reinterpret_cast<double *>(raw), *x = p + n, *r = x + rpc, *q = r + rpc;
+    RV *sl = reinterpret_cast<RV *>(q + rpc);   // lumped inverse of the block's rows
+    RV *sv = sl + rpc;
+    uint16_t *si = reinterpret_cast<uint16_t *>(sv + (size_t)rpc * kMassEll);
+    const RV *lump = staged ? sl : L + r0;
+    int longer = 0;   // rows of this block with more than kMassEll entries
+    for (int row = tid; row < m; row += T)
     {
-        const double bv = b[row * ldb + k];
-        const double zv = (double)L[row] * bv;
-        x[row] = 0.0; r[row] = bv; z[row] = zv; p[row] = zv;
-        rz += bv * zv;
-        bb += bv * bv;
+        if (staged) sl[row] = L[r0 + row];
+        longer |= mo[r0 + row + 1] - mo[r0 + row] > kMassEll;
     }
-    block_sum2(rz, bb, red);   // ends with a barrier: p is complete
-    const double bn = sqrt(bb);
+    longer = __syncthreads_or(longer);
+    if (staged == 2)
+        for (int e = tid; e < m * kMassEll; e += T)
+        {
+            const int j = e / m, row = e - j * m;
+            sv[j * rpc + row] = ell_val[j * n + r0 + row];
+            si[j * rpc + row] = ell_idx[j * n + r0 + row];
+        }
+
+    // v[0 .. NV): totals over the cluster, through slots slot .. of xch
+    auto totals = [&](auto nv, int slot, double (&v)[2]) {
+        constexpr int NV = decltype(nv)::value;
+        #pragma unroll
+        for (int w = 0; w < NV; ++w)
+        {
+            #pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[w] += __shfl_xor_sync(0xffffffffu, v[w], o);
+            if (lane == 0) red[w][warp] = v[w];
+        }
+        __syncthreads();
+        if (warp < NV)
+        {
+            double t = lane < nw ? red[warp][lane] : 0.0;
+            #pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if (lane < S) *cluster.map_shared_rank(&xch[slot + warp][rank], lane) = t;
+        }
+        if (S > 1) cluster.sync();
+        else __syncthreads();
+        #pragma unroll
+        for (int w = 0; w < NV; ++w)
+        {
+            double t = 0.0;
+            for (int s = 0; s < S; ++s) t += xch[slot + w][s];
+            v[w] = t;
+        }
+    };
+    // p[row] = v in every block of the cluster
+    auto put_p = [&](int row, double v) {
+        p[row] = v;
+        for (int s = 1; s < S; ++s) cluster.map_shared_rank(p, (rank + s) & (S - 1))[row] = v;
+    };
+    constexpr std::integral_constant<int, 1> one{};
+    constexpr std::integral_constant<int, 2> two{};
+
+    double v[2] = {0.0, 0.0};
+    if (S > 1) cluster.sync();   // every block of the cluster runs before its shared memory is written
+    for (int row = tid; row < m; row += T)
+    {
+        const double bv = b[(int64_t)(r0 + row) * ldb + k];
+        const double zv = (double)lump[row] * bv;
+        x[row] = 0.0;
+        r[row] = bv;
+        put_p(r0 + row, zv);
+        v[0] += bv * zv;
+        v[1] += bv * bv;
+    }
+    totals(two, 1, v);   // its barrier also completes p
+    double rz = v[0];
+    const double bn = sqrt(v[1]);
     bool conv = bn <= tol * bn;
     int it = 0;
-    for (; it < max_iter && !conv; ++it)   // conv and it are block-uniform
+    // the totals are the same in every block of the cluster, so conv and it are cluster-uniform
+    for (; it < max_iter && !conv; ++it)
     {
-        double pq = 0.0, unused = 0.0;
-        for (int64_t row = threadIdx.x; row < n; row += blockDim.x)
-        {
-            // the row's first 8 entries (1 + the vertex degree, ~7) loaded before their gathers
-            constexpr int kPf = 8;
-            const int32_t e0 = mo[row], e1 = mo[row + 1];
-            int32_t ci[kPf];
-            double cv[kPf], pv[kPf];
-            #pragma unroll
-            for (int j = 0; j < kPf; ++j)
+        v[0] = 0.0;
+        auto matvec = [&](const RV *val, const uint16_t *idx, int64_t stride) {
+            #pragma unroll 2
+            for (int row = tid; row < m; row += T)
             {
-                const bool in = e0 + j < e1;
-                ci[j] = in ? mi[e0 + j] : 0;
-                cv[j] = in ? (double)mv[e0 + j] : 0.0;
+                double s = 0.0;
+                #pragma unroll
+                for (int j = 0; j < kMassEll; ++j) s += (double)val[j * stride + row] * p[idx[j * stride + row]];
+                if (longer)
+                    for (int32_t e = mo[r0 + row] + kMassEll; e < mo[r0 + row + 1]; ++e) s += (double)mv[e] * p[mi[e]];
+                q[row] = s;
+                v[0] += p[r0 + row] * s;
             }
-            #pragma unroll
-            for (int j = 0; j < kPf; ++j) pv[j] = e0 + j < e1 ? p[ci[j]] : 0.0;
-            double sacc = 0.0;
-            #pragma unroll
-            for (int j = 0; j < kPf; ++j)
-                if (e0 + j < e1) sacc += cv[j] * pv[j];
-            for (int32_t e = e0 + kPf; e < e1; ++e) sacc += (double)mv[e] * p[mi[e]];
-            q[row] = sacc;
-            pq += p[row] * sacc;
-        }
-        block_sum2(pq, unused, red);
-        const double alpha = pq == 0.0 ? 0.0 : rz / pq;
-        double rzn = 0.0, rr = 0.0;
-        #pragma unroll 2
-        for (int64_t row = threadIdx.x; row < n; row += blockDim.x)
+        };
+        if (staged == 2) matvec(sv, si, rpc);
+        else matvec(ell_val + r0, ell_idx + r0, n);
+        totals(one, 0, v);
+        const double alpha = v[0] == 0.0 ? 0.0 : rz / v[0];
+        v[0] = v[1] = 0.0;
+        #pragma unroll 4
+        for (int row = tid; row < m; row += T)
         {
-            x[row] += alpha * p[row];
+            x[row] += alpha * p[r0 + row];
             const double rv = r[row] - alpha * q[row];
             r[row] = rv;
-            const double zv = (double)L[row] * rv;
-            z[row] = zv;
-            rzn += rv * zv;
-            rr += rv * rv;
+            const double zv = (double)lump[row] * rv;
+            q[row] = zv;   // z, until the next matvec
+            v[0] += rv * zv;
+            v[1] += rv * rv;
         }
-        block_sum2(rzn, rr, red);
-        const double beta = rz == 0.0 ? 0.0 : rzn / rz;
-        rz = rzn;
-        conv = sqrt(rr) <= tol * bn;
-        #pragma unroll 4
-        for (int64_t row = threadIdx.x; row < n; row += blockDim.x) p[row] = z[row] + beta * p[row];
-        __syncthreads();   // p complete before the next iteration's gathers
+        totals(two, 1, v);
+        const double beta = rz == 0.0 ? 0.0 : v[0] / rz;
+        rz = v[0];
+        conv = sqrt(v[1]) <= tol * bn;
+        for (int row = tid; row < m; row += T) put_p(r0 + row, q[row] + beta * p[r0 + row]);
+        if (S > 1) cluster.sync();   // p complete before the next iteration's gathers, and no write to a block that has left
+        else __syncthreads();
     }
-    for (int64_t row = threadIdx.x; row < n; row += blockDim.x) y[row * ldy + k] = x[row];
-    if (threadIdx.x == 0)
+    for (int row = tid; row < m; row += T) y[(int64_t)(r0 + row) * ldy + k] = x[row];
+    if (rank == 0 && tid == 0)
     {
         flags[2 + k] = conv ? 1 : 0;
         if (!conv) atomicAdd(&flags[0], 1);
@@ -537,14 +600,11 @@ cg_block_kernel(int64_t n, int c, const double *__restrict__ b, int64_t ldb, con
     }
 }
 
-// One block per column with p (n doubles) in dynamic shared memory; the limit
-// above 48 KB is a per-device attribute of each instantiation, set once.
 template <class RV>
-void launch_cg_block(cudaStream_t st, int64_t n, int c, const double *b, int64_t ldb, const int32_t *mo,
-                     const int32_t *mi, const RV *mv, const RV *L, double *x, double *r, double *z, double *q,
-                     double *y, int64_t ldy, int *flags, double tol, int max_iter)
+void launch_cg_cluster(cudaStream_t st, const MeshDev &mesh, int c, const double *b, int64_t ldb, const RV *mv,
+                       const RV *ell_val, const RV *L, double *y, int64_t ldy, int *flags, double tol, int max_iter)
 {
-    constexpr int kMaxBytes = (int)(kCgBlockMaxRows * sizeof(double));
+    // the limit above 48 KB is a per-device attribute of each instantiation, set once
     int dev = 0;
     BAEMM_CUDA(cudaGetDevice(&dev));
     static std::mutex mu;
@@ -553,12 +613,26 @@ void launch_cg_block(cudaStream_t st, int64_t n, int c, const double *b, int64_t
         std::lock_guard<std::mutex> lock(mu);
         if (dev < 0 || dev >= 64 || !done[dev])
         {
-            BAEMM_CUDA(cudaFuncSetAttribute(cg_block_kernel<RV>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBytes));
+            BAEMM_CUDA(cudaFuncSetAttribute(cg_cluster_kernel<RV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)kCgSmemBytes));
             if (dev >= 0 && dev < 64) done[dev] = true;
         }
     }
-    cg_block_kernel<<<c, kCgBlockThreads, (size_t)n * sizeof(double), st>>>(n, c, b, ldb, mo, mi, mv, L, x, r, z, q,
-                                                                              y, ldy, flags, tol, max_iter);
+    const CgShape h = cg_cluster_shape<RV>(mesh.nv, c, tc_sm_count());
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(c * h.S);
+    cfg.blockDim = dim3(std::min(kCgThreads, ceil_div(h.rpc, 128) * 128));
+    cfg.dynamicSmemBytes = h.bytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = h.S;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    BAEMM_CUDA(cudaLaunchKernelEx(&cfg, cg_cluster_kernel<RV>, mesh.nv, h.rpc, h.staged, b, ldb,
+                                  (const int32_t *)mesh.mass_outer.p, (const int32_t *)mesh.mass_inner.p, mv,
+                                  (const uint16_t *)mesh.mass_ell_idx.p, ell_val, L, y, ldy, flags, tol, max_iter));
 }
 
 __global__ void cg_output_kernel(int64_t n, int c, const double *__restrict__ x, double *__restrict__ y, int64_t ldy)
@@ -847,8 +921,8 @@ bool CgSolver::finish(cudaStream_t st, int *iterations)
 {
     BAEMM_CUDA(cudaStreamSynchronize(st));
     if (iterations) *iterations = host_flags_[1];
-    // flags[0]: all converged (multi-block kernels) or columns not converged (cg_block_kernel)
-    return block_path_ ? host_flags_[0] == 0 : host_flags_[0] != 0;
+    // flags[0]: all converged (multi-block kernels) or columns not converged (cg_cluster_kernel)
+    return cluster_path_ ? host_flags_[0] == 0 : host_flags_[0] != 0;
 }
 
 void CgSolver::reserve_totals(int nblk, int S, cudaStream_t st)
@@ -869,25 +943,23 @@ void CgSolver::enqueue_mass(const MeshDev &m, bool fp64_values, const double *b,
     const int64_t n = m.nv;
     BAEMM_REQUIRE(c >= 1 && c <= kMaxKrylovColumns, BAEMM_ERR_SIZE, "CG column count out of range");
     const int64_t N = n * c;
-    x_.reserve(N); r_.reserve(N); z_.reserve(N); p_.reserve(N); q_.reserve(N);
-    col_.reserve(4 * (size_t)c);
     flags_.reserve(2 + (size_t)c);
     if (!host_flags_) BAEMM_CUDA(cudaMallocHost(&host_flags_, 2 * sizeof(int)));
-    block_path_ = n <= kCgBlockMaxRows;
-    if (block_path_)
+    cluster_path_ = n <= kMassEllMaxRows;
+    if (cluster_path_)
     {
-        // one block per column, all iterations in one launch
+        // all iterations in one launch
         BAEMM_CUDA(cudaMemsetAsync(flags_.p, 0, 2 * sizeof(int), st));
-        auto runb = [&](auto Lv, auto Mv) {
-            launch_cg_block(st, n, c, b, ldb, m.mass_outer, m.mass_inner, Mv, Lv, x_.p, r_.p, z_.p, q_.p, y, ldy,
-                            flags_.p, tol, max_iter);
-        };
-        if (fp64_values) runb(m.lumped_d.p, m.mass_d.p);
-        else runb(m.lumped_f.p, m.mass_f.p);
+        if (fp64_values)
+            launch_cg_cluster<double>(st, m, c, b, ldb, m.mass_d, m.mass_ell_d, m.lumped_d, y, ldy, flags_.p, tol, max_iter);
+        else
+            launch_cg_cluster<float>(st, m, c, b, ldb, m.mass_f, m.mass_ell_f, m.lumped_f, y, ldy, flags_.p, tol, max_iter);
         BAEMM_LAUNCH_CHECK();
         BAEMM_CUDA(cudaMemcpyAsync(host_flags_, flags_.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
         return;
     }
+    x_.reserve(N); r_.reserve(N); z_.reserve(N); p_.reserve(N); q_.reserve(N);
+    col_.reserve(4 * (size_t)c);
     const Layout L = make_layout(n, c);
     reserve_totals(L.nblk, 2 * c, st);
     dim3 grid(L.nblk, L.nchunk);
@@ -918,32 +990,29 @@ double CgSolver::profile_block(const MeshDev &m, bool fp64_values, int c, int it
     const int64_t n = m.nv;
     BAEMM_REQUIRE(c >= 1 && c <= kMaxKrylovColumns, BAEMM_ERR_SIZE, "CG column count out of range");
     BAEMM_REQUIRE(iterations >= 1, BAEMM_ERR_ARG, "at least one iteration");
-    if (n > kCgBlockMaxRows) return 0.0;
+    if (n > kMassEllMaxRows) return 0.0;
     const int64_t N = n * c;
     DevBuf<double> b, y;
     b.reserve(N);
     y.reserve(N);
     std::vector<double> ones((size_t)N, 1.0);
     BAEMM_CUDA(cudaMemcpyAsync(b.p, ones.data(), N * sizeof(double), cudaMemcpyHostToDevice, st));
-    x_.reserve(N); r_.reserve(N); z_.reserve(N); p_.reserve(N); q_.reserve(N);
     flags_.reserve(2 + (size_t)c);
     cudaEvent_t e0, e1;
     BAEMM_CUDA(cudaEventCreate(&e0));
     BAEMM_CUDA(cudaEventCreate(&e1));
     float ms = 0.f;
-    auto runb = [&](auto Lv, auto Mv) {
-        // tol < 0: no column converges, every iteration does its work; a first launch warms up
-        for (int rep = 0; rep < 2; ++rep)
-        {
-            BAEMM_CUDA(cudaMemsetAsync(flags_.p, 0, 2 * sizeof(int), st));
-            BAEMM_CUDA(cudaEventRecord(e0, st));
-            launch_cg_block(st, n, c, b.p, c, m.mass_outer, m.mass_inner, Mv, Lv, x_.p, r_.p, z_.p, q_.p, y.p, c,
-                            flags_.p, -1.0, iterations);
-            BAEMM_CUDA(cudaEventRecord(e1, st));
-        }
-    };
-    if (fp64_values) runb(m.lumped_d.p, m.mass_d.p);
-    else runb(m.lumped_f.p, m.mass_f.p);
+    // tol < 0: no column converges, every iteration does its work; a first launch warms up
+    for (int rep = 0; rep < 2; ++rep)
+    {
+        BAEMM_CUDA(cudaMemsetAsync(flags_.p, 0, 2 * sizeof(int), st));
+        BAEMM_CUDA(cudaEventRecord(e0, st));
+        if (fp64_values)
+            launch_cg_cluster<double>(st, m, c, b.p, c, m.mass_d, m.mass_ell_d, m.lumped_d, y.p, c, flags_.p, -1.0, iterations);
+        else
+            launch_cg_cluster<float>(st, m, c, b.p, c, m.mass_f, m.mass_ell_f, m.lumped_f, y.p, c, flags_.p, -1.0, iterations);
+        BAEMM_CUDA(cudaEventRecord(e1, st));
+    }
     BAEMM_LAUNCH_CHECK();
     BAEMM_CUDA(cudaEventSynchronize(e1));
     BAEMM_CUDA(cudaEventElapsedTime(&ms, e0, e1));

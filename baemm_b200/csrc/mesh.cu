@@ -82,7 +82,8 @@ template <class R>
 __global__ void mass_values_kernel(int64_t nv, const int32_t *__restrict__ tris, const int32_t *__restrict__ avt_outer,
                                    const int32_t *__restrict__ avt_inner, const R *__restrict__ area,
                                    const int32_t *__restrict__ m_outer, const int32_t *__restrict__ m_inner,
-                                   R *__restrict__ m_val, R *__restrict__ lumped)
+                                   R *__restrict__ m_val, R *__restrict__ lumped, uint16_t *__restrict__ ell_idx,
+                                   R *__restrict__ ell_val)
 {
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nv) return;
@@ -106,6 +107,13 @@ __global__ void mass_values_kernel(int64_t nv, const int32_t *__restrict__ tris,
         }
     }
     lumped[v] = R(1) / lump;
+    if (!ell_val) return;   // slot-major copy of the row (MeshDev::mass_ell_*)
+    for (int j = 0; j < kMassEll; ++j)
+    {
+        const bool in = e0 + j < e1;
+        ell_idx[j * nv + v] = (uint16_t)(in ? m_inner[e0 + j] : v);
+        ell_val[j * nv + v] = in ? m_val[e0 + j] : R(0);
+    }
 }
 
 // CurlOp (Initialize.hpp:146-211): per triangle three rows (x, y, z) of
@@ -202,14 +210,15 @@ void launch_mass_values(const MeshDev &m, bool fp64, cudaStream_t st)
 {
     if (m.nv == 0) return;
     const int T = 128;
+    const bool ell = m.nv <= kMassEllMaxRows;
     if (fp64)
         mass_values_kernel<double><<<ceil_div(m.nv, T), T, 0, st>>>(m.nv, m.tris, m.avt_outer, m.avt_inner, m.area_d,
                                                                     m.mass_outer, m.mass_inner, m.mass_d,
-                                                                    m.lumped_d);
+                                                                    m.lumped_d, m.mass_ell_idx, ell ? m.mass_ell_d.p : nullptr);
     else
         mass_values_kernel<float><<<ceil_div(m.nv, T), T, 0, st>>>(m.nv, m.tris, m.avt_outer, m.avt_inner, m.area_f,
                                                                    m.mass_outer, m.mass_inner, m.mass_f,
-                                                                   m.lumped_f);
+                                                                   m.lumped_f, m.mass_ell_idx, ell ? m.mass_ell_f.p : nullptr);
     BAEMM_LAUNCH_CHECK();
 }
 

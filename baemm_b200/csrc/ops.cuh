@@ -14,6 +14,12 @@
 namespace baemm
 {
 
+// The mass matrix in slots, slot-major (8 x nv; a row's first 8 CSR entries, then
+// zeros in its own column), for meshes of up to kMassEllMaxRows vertices
+// (16-bit column indices; the CG of such meshes reads it).
+constexpr int kMassEll = 8;
+constexpr int64_t kMassEllMaxRows = 16384;
+
 struct MeshDev
 {
     int64_t nv = 0, nt = 0, nm = 0;
@@ -22,6 +28,9 @@ struct MeshDev
     DevBuf<int32_t> tri_sorted;  // nt x 3 (AvOp columns, sorted)
     DevBuf<int32_t> avt_outer, avt_inner;
     DevBuf<int32_t> mass_outer, mass_inner;
+    DevBuf<uint16_t> mass_ell_idx;
+    DevBuf<float> mass_ell_f;
+    DevBuf<double> mass_ell_d;
     DevBuf<float> mid_f, nrm_f, area_f, a3_f, diag_f, mass_f, lumped_f, meas_f;
     DevBuf<float> tgeo_f;        // tensor-core form: source geometry per source tile (lazily built)
     DevBuf<double> mid_d, nrm_d, area_d, a3_d, diag_d, mass_d, lumped_d, meas_d;

@@ -126,3 +126,34 @@ def test_fp64_far_and_near(count, wc, wcs):
             getattr(H, name)(0.7, B, 0.3, got, kap, coeff, wc, wcs, *extra)
             getattr(orc, name)(0.7, B, 0.3, ref, kap, coeff, wc, wcs, *extra)
             assert relerr(got, ref) < TOL64, name
+
+
+def _bipyramid(n):
+    """n equatorial vertices and two poles of degree n."""
+    a = 2 * np.pi * np.arange(n) / n
+    coords = np.concatenate([np.stack([np.cos(a), np.sin(a), 0 * a], 1), [[0, 0, 0.5], [0, 0, -0.5]]])
+    i, j = np.arange(n), (np.arange(n) + 1) % n
+    return coords, np.concatenate([np.stack([i, j, 0 * i + n], 1), np.stack([j, i, 0 * i + n + 1], 1)])
+
+
+@pytest.mark.parametrize("ncols", [1, 5, 70])
+@pytest.mark.parametrize("mesh", ["9", "511", "512", "513", "5125", "16384", "poles of degree 3", "poles of degree 60"])
+def test_one_launch_mass_inverse(mesh, ncols):
+    """Rows that do and do not fill the blocks of a cluster, matrix rows in and
+    out of shared memory, and rows of the mass matrix with more than 8 entries."""
+    grids = {"9": (3, 3), "511": (7, 73), "512": (16, 32), "513": (19, 27), "5125": (41, 125), "16384": (128, 128)}
+    coords, tris = meshes.torus(n_minor=grids[mesh][0], n_major=grids[mesh][1]) if mesh in grids else \
+        _bipyramid(int(mesh.split()[-1]))
+    X = np.random.default_rng(ncols).standard_normal((coords.shape[0], ncols))
+    got, ref = np.zeros_like(X), np.zeros_like(X)
+    with Helmholtz_CUDA(coords, tris, np.eye(3)) as H:
+        assert H.ProfileKrylov(1, 1, 1)["cg_iteration"]["one_launch_path"]
+        for mode, tol in ((APPLY_FP64, TOL64), (APPLY_FP32, 1e-6)):   # FP32: mass values rounded to float
+            H.SetApplyMode(mode)
+            H.ApplyMassInverse(X, got, 1e-10)
+            orc = O.Oracle(coords, tris, np.eye(3), precision=64 if mode == APPLY_FP64 else 32)
+            for k in range(ncols):   # the oracle iterates a block until its last column has converged, the library each column
+                one = np.zeros((coords.shape[0], 1))
+                orc.ApplyMassInverse(np.ascontiguousarray(X[:, k:k + 1]), one, 1e-10)
+                ref[:, k] = one[:, 0]
+            assert relerr(got, ref) < tol, mode
