@@ -18,6 +18,8 @@
 // Herglotz kernels whose mask is always 1, FarFieldOperatorKernel.cl:89).
 #include "ops.cuh"
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 namespace baemm
@@ -83,26 +85,24 @@ __device__ __forceinline__ void stage_tile(Tile<R, COLS> &t, const R *__restrict
     }
 }
 
-// In FP64 only chunks of fewer than 8 columns come here (dense64.cu takes the others).
-template <class R, int COLS, bool SL, bool DL, bool ADL>
+// Scalar FP32 form (variant 0; dense64.cu has the FP64 form).
+template <int COLS, bool SL, bool DL, bool ADL>
 __global__ void __launch_bounds__(kTargets)
-boundary_dense_kernel(DenseTargets<R> tg, const R *__restrict__ mid4, const R *__restrict__ nrm4,
-                      const cplx<R> *__restrict__ B, cplx<R> *__restrict__ C,
-                      const typename Prm<R>::type *__restrict__ prm, int n, int wc, int wcs, int per_split)
+boundary_dense_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, const float *__restrict__ nrm4,
+                      const float2 *__restrict__ B, float2 *__restrict__ C,
+                      const ChunkParamsF *__restrict__ prm, int n, int wc, int wcs)
 {
-    __shared__ Tile<R, COLS> tile;
-    const int jb = blockIdx.z * per_split, je = min(n, jb + per_split);   // this split's sources
-    C += (int64_t)blockIdx.z * tg.m * wc;
+    __shared__ Tile<float, COLS> tile;
     const int i = blockIdx.x * kTargets + threadIdx.x;
     const int iself = tg.self ? tg.off + i : -1;   // the source index excluded for this target (none: -1)
     const int col0 = blockIdx.y * COLS;
     const int ch = col0 / wcs;
-    const R kap = prm[ch].kappa;
-    const cplx<R> c1 = prm[ch].c[1], c2 = prm[ch].c[2], c3 = prm[ch].c[3];
-    R x0 = R(0), x1 = R(0), x2 = R(0), n0 = R(0), n1 = R(0), n2 = R(0);
+    const float kap = prm[ch].kappa;
+    const float2 c1 = prm[ch].c[1], c2 = prm[ch].c[2], c3 = prm[ch].c[3];
+    float x0 = 0.f, x1 = 0.f, x2 = 0.f, n0 = 0.f, n1 = 0.f, n2 = 0.f;
     if (i < tg.m)
     {
-        const R *x = tg.pts4;
+        const float *x = tg.pts4;
         x0 = x[4 * (int64_t)i]; x1 = x[4 * (int64_t)i + 1]; x2 = x[4 * (int64_t)i + 2];
         if (ADL)
         {
@@ -110,61 +110,59 @@ boundary_dense_kernel(DenseTargets<R> tg, const R *__restrict__ mid4, const R *_
             n0 = nrm4[4 * gi]; n1 = nrm4[4 * gi + 1]; n2 = nrm4[4 * gi + 2];
         }
     }
-    // FP32: two-level sum -- each 64-source tile into fresh accumulators, then
-    // into the running total (the error of one long FP32 chain over ~1e5
-    // sources would be ~5x larger); FP64: one accumulator.
-    constexpr bool kTwoLevel = std::is_same<R, float>::value;
-    cplx<R> acc[COLS], tacc[COLS];
+    // two-level sum: each 64-source tile into fresh accumulators, then into the
+    // running total (the error of one long FP32 chain over ~1e5 sources would be
+    // ~5x larger)
+    float2 acc[COLS], tacc[COLS];
     #pragma unroll
-    for (int k = 0; k < COLS; ++k) { acc[k].x = R(0); acc[k].y = R(0); }
+    for (int k = 0; k < COLS; ++k) { acc[k].x = 0.f; acc[k].y = 0.f; }
 
-    for (int j0 = jb; j0 < je; j0 += kTile)
+    for (int j0 = 0; j0 < n; j0 += kTile)
     {
         __syncthreads();
-        stage_tile<R, COLS, DL, false>(tile, mid4, nrm4, B, wc, col0, j0, je);
+        stage_tile<float, COLS, DL, false>(tile, mid4, nrm4, B, wc, col0, j0, n);
         __syncthreads();
-        const int smax = min(kTile, je - j0);
+        const int smax = min(kTile, n - j0);
         #pragma unroll
         for (int k = 0; k < COLS; ++k)
         {
-            tacc[k].x = R(0);
-            tacc[k].y = R(0);
+            tacc[k].x = 0.f;
+            tacc[k].y = 0.f;
         }
-        cplx<R>(&sum)[COLS] = kTwoLevel ? tacc : acc;
         #pragma unroll 2
         for (int s = 0; s < smax; ++s)
         {
-            const R zx = tile.y[s][0] - x0, zy = tile.y[s][1] - x1, zz = tile.y[s][2] - x2;
-            const R r2 = zx * zx + zy * zy + zz * zz;
-            const R rinv = (j0 + s == iself) ? R(0) : drsqrt(r2);
-            const R r = r2 * rinv;
-            const R kr = kap * r;
-            R sn, cs;
+            const float zx = tile.y[s][0] - x0, zy = tile.y[s][1] - x1, zz = tile.y[s][2] - x2;
+            const float r2 = zx * zx + zy * zy + zz * zz;
+            const float rinv = (j0 + s == iself) ? 0.f : drsqrt(r2);
+            const float r = r2 * rinv;
+            const float kr = kap * r;
+            float sn, cs;
             dsincos(kr, &sn, &cs);
-            cplx<R> A;
-            A.x = R(0);
-            A.y = R(0);
+            float2 A;
+            A.x = 0.f;
+            A.y = 0.f;
             if (SL)
             {
-                const R er = cs * rinv, ei = sn * rinv;
+                const float er = cs * rinv, ei = sn * rinv;
                 A.x = c1.x * er - c1.y * ei;
                 A.y = c1.x * ei + c1.y * er;
             }
             if (DL || ADL)
             {
-                const R r3 = rinv * rinv * rinv;
-                const R g0 = -(kr * sn + cs) * r3;
-                const R g1 = (kr * cs - sn) * r3;
-                R fx = R(0), fy = R(0);
+                const float r3 = rinv * rinv * rinv;
+                const float g0 = -(kr * sn + cs) * r3;
+                const float g1 = (kr * cs - sn) * r3;
+                float fx = 0.f, fy = 0.f;
                 if (DL)
                 {
-                    const R dm = zx * tile.mu[s][0] + zy * tile.mu[s][1] + zz * tile.mu[s][2];
+                    const float dm = zx * tile.mu[s][0] + zy * tile.mu[s][1] + zz * tile.mu[s][2];
                     fx += c2.x * dm;
                     fy += c2.y * dm;
                 }
                 if (ADL)
                 {
-                    const R dn = zx * n0 + zy * n1 + zz * n2;
+                    const float dn = zx * n0 + zy * n1 + zz * n2;
                     fx -= c3.x * dn;
                     fy -= c3.y * dn;
                 }
@@ -172,21 +170,18 @@ boundary_dense_kernel(DenseTargets<R> tg, const R *__restrict__ mid4, const R *_
                 A.y += fx * g1 + fy * g0;
             }
             #pragma unroll
-            for (int k = 0; k < COLS; ++k) cfma(sum[k], A, tile.B[s][k]);
+            for (int k = 0; k < COLS; ++k) cfma(tacc[k], A, tile.B[s][k]);
         }
-        if (kTwoLevel)
+        #pragma unroll
+        for (int k = 0; k < COLS; ++k)
         {
-            #pragma unroll
-            for (int k = 0; k < COLS; ++k)
-            {
-                acc[k].x += tacc[k].x;
-                acc[k].y += tacc[k].y;
-            }
+            acc[k].x += tacc[k].x;
+            acc[k].y += tacc[k].y;
         }
     }
     if (i < tg.m)
     {
-        cplx<R> *out = &C[(int64_t)i * wc + col0];
+        float2 *out = &C[(int64_t)i * wc + col0];
         #pragma unroll
         for (int k = 0; k < COLS; ++k) out[k] = acc[k];
     }
@@ -214,10 +209,9 @@ template <bool SL, bool DL, bool ADL>
 __global__ void __launch_bounds__(kTargets, 4)
 boundary_packed_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, const float *__restrict__ nrm4,
                        const float2 *__restrict__ B, float2 *__restrict__ C, const ChunkParamsF *__restrict__ prm,
-                       int n, int wc, int wcs, int per_split)
+                       int n, int wc, int wcs)
 {
     __shared__ PackedTile tile;
-    const int jb = blockIdx.z * per_split, je = min(n, jb + per_split);   // this split's sources
     const int col0 = blockIdx.y * kPackedCols;
     const int ch = col0 / wcs;
     const float kap = prm[ch].kappa;
@@ -240,28 +234,28 @@ boundary_packed_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, c
     #pragma unroll
     for (int k = 0; k < kPackedCols; ++k) acc[k] = make_float2(0.f, 0.f);
 
-    for (int j0 = jb; j0 < je; j0 += kTile)
+    for (int j0 = 0; j0 < n; j0 += kTile)
     {
         __syncthreads();
         if (tid < kTile)
         {
             const int j = j0 + tid;
-            tile.y[tid] = (j < je) ? reinterpret_cast<const float4 *>(mid4)[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+            tile.y[tid] = (j < n) ? reinterpret_cast<const float4 *>(mid4)[j] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         else if (DL && tid < 2 * kTile)
         {
             const int sidx = tid - kTile, j = j0 + sidx;
-            tile.mu[sidx] = (j < je) ? reinterpret_cast<const float4 *>(nrm4)[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+            tile.mu[sidx] = (j < n) ? reinterpret_cast<const float4 *>(nrm4)[j] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         for (int idx = tid; idx < kTile * kPackedCols; idx += kTargets)
         {
             const int sidx = idx / kPackedCols, k = idx % kPackedCols, j = j0 + sidx;
-            const float2 b = (j < je) ? B[(int64_t)j * wc + col0 + k] : make_float2(0.f, 0.f);
+            const float2 b = (j < n) ? B[(int64_t)j * wc + col0 + k] : make_float2(0.f, 0.f);
             tile.B[sidx][k] = b;
             tile.Bw[sidx][k] = make_float2(-b.y, b.x);
         }
         __syncthreads();
-        const int smax = min(kTile, je - j0);
+        const int smax = min(kTile, n - j0);
         #pragma unroll
         for (int k = 0; k < kPackedCols; ++k) tacc[k] = make_float2(0.f, 0.f);
         for (int s = 0; s < smax; ++s)
@@ -317,7 +311,7 @@ boundary_packed_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, c
     }
     if (ti < tg.m)
     {
-        float2 *out = &C[((int64_t)blockIdx.z * tg.m + ti) * wc + col0];
+        float2 *out = &C[(int64_t)ti * wc + col0];
         #pragma unroll
         for (int k = 0; k < kPackedCols; ++k) out[k] = acc[k];
     }
@@ -337,9 +331,9 @@ boundary_packed_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, c
 // totals in shared memory (a private float4 per thread and column; two-level
 // summation as in boundary_dense_kernel), which leaves the registers for four
 // CTAs of 128 threads per SM.
-// Measured: 2.91 ms on 20234 triangles x 32 columns (SL + DL', FP32 pipe 72 %
+// Measured: 2.80 ms on 20234 triangles x 32 columns (SL + DL', FP32 pipe 72 %
 // busy), the scalar kernel 4.95 ms; 157 us on 5120 x 16 in chunks of 8 columns,
-// the scalar kernel unsplit 480 us.
+// the scalar kernel 480 us.
 constexpr int kPairTile = 32;
 
 template <int COLS>
@@ -474,17 +468,27 @@ boundary_pair_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, con
             tile.tot[k][tid] = t;
         }
     }
-    float2 *out = C + (int64_t)blockIdx.z * tg.m * wc + col0;
-    #pragma unroll
-    for (int k = 0; k < COLS; ++k)
+    // with a cluster of S parts of the sources, block r adds columns r, r + S, ... of all of them in order
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    if (S > 1) cluster.sync();
+    float2 *out = C + (int64_t)(blockIdx.z / S) * tg.m * wc + col0;
+    for (int k = rank; k < COLS; k += S)
     {
-        const float4 t = tile.tot[k][tid];
+        float4 t = S > 1 ? *cluster.map_shared_rank(&tile.tot[k][tid], 0) : tile.tot[k][tid];
+        for (int q = 1; q < S; ++q)
+        {
+            const float4 v = *cluster.map_shared_rank(&tile.tot[k][tid], q);
+            t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
+        }
         if (t0 < tg.m) out[(int64_t)t0 * wc + k] = make_float2(t.x, t.z);
         if (t1 < tg.m) out[(int64_t)t1 * wc + k] = make_float2(t.y, t.w);
     }
+    if (S > 1) cluster.sync();   // no block leaves while its totals are read
 }
 
-// C = the sum of the splits' partial blocks, in split order (four loads in flight).
+// C = the sum of the partial blocks of a split launch, in order (four loads in flight).
 template <class R>
 __global__ void split_sum_kernel(const cplx<R> *__restrict__ partial, int splits, int64_t elems, cplx<R> *__restrict__ C)
 {
@@ -730,23 +734,27 @@ __global__ void pack_points_kernel(int64_t m, const double *__restrict__ pts3, R
 }
 
 // ---- dispatch helpers -----------------------------------------------------------
-template <class R, int COLS>
-void boundary_cols(int code, dim3 grid, cudaStream_t st, DenseTargets<R> tg, const R *mid, const R *nrm,
-                   const cplx<R> *B, cplx<R> *C, const typename Prm<R>::type *p, int n, int wc, int wcs, int per_split)
+// The kernel template KERNEL<ARGS..., SL, DL, ADL> of an operator code
+#define BAEMM_BY_LAYERS(LAUNCH)                     \
+    switch (code)                                   \
+    {                                               \
+        case 1: LAUNCH(true, false, false); break;  \
+        case 2: LAUNCH(false, true, false); break;  \
+        case 3: LAUNCH(true, true, false); break;   \
+        case 4: LAUNCH(false, false, true); break;  \
+        case 5: LAUNCH(true, false, true); break;   \
+        case 6: LAUNCH(false, true, true); break;   \
+        case 7: LAUNCH(true, true, true); break;    \
+        default: break;                             \
+    }
+
+template <int COLS>
+void scalar_dispatch(int code, dim3 grid, cudaStream_t st, DenseTargets<float> tg, const float *mid, const float *nrm,
+                     const float2 *B, float2 *C, const ChunkParamsF *p, int n, int wc, int wcs)
 {
 #define BAEMM_BK(SL, DL, ADL) \
-    boundary_dense_kernel<R, COLS, SL, DL, ADL><<<grid, kTargets, 0, st>>>(tg, mid, nrm, B, C, p, n, wc, wcs, per_split)
-    switch (code)
-    {
-        case 1: BAEMM_BK(true, false, false); break;
-        case 2: BAEMM_BK(false, true, false); break;
-        case 3: BAEMM_BK(true, true, false); break;
-        case 4: BAEMM_BK(false, false, true); break;
-        case 5: BAEMM_BK(true, false, true); break;
-        case 6: BAEMM_BK(false, true, true); break;
-        case 7: BAEMM_BK(true, true, true); break;
-        default: break;
-    }
+    boundary_dense_kernel<COLS, SL, DL, ADL><<<grid, kTargets, 0, st>>>(tg, mid, nrm, B, C, p, n, wc, wcs)
+    BAEMM_BY_LAYERS(BAEMM_BK)
 #undef BAEMM_BK
 }
 
@@ -789,152 +797,146 @@ template <> const double *geo_meas<double>(const MeshDev &m) { return m.meas_d; 
 inline int cols_for(int wcs) { return wcs < 16 ? wcs : 16; }
 
 void packed_dispatch(int code, dim3 grid, cudaStream_t st, DenseTargets<float> tg, const float *mid, const float *nrm,
-                     const float2 *B, float2 *C, const ChunkParamsF *p, int n, int wc, int wcs, int per_split)
+                     const float2 *B, float2 *C, const ChunkParamsF *p, int n, int wc, int wcs)
 {
 #define BAEMM_PK(SL, DL, ADL) \
-    boundary_packed_kernel<SL, DL, ADL><<<grid, kTargets, 0, st>>>(tg, mid, nrm, B, C, p, n, wc, wcs, per_split)
-    switch (code)
-    {
-        case 1: BAEMM_PK(true, false, false); break;
-        case 2: BAEMM_PK(false, true, false); break;
-        case 3: BAEMM_PK(true, true, false); break;
-        case 4: BAEMM_PK(false, false, true); break;
-        case 5: BAEMM_PK(true, false, true); break;
-        case 6: BAEMM_PK(false, true, true); break;
-        case 7: BAEMM_PK(true, true, true); break;
-        default: break;
-    }
+    boundary_packed_kernel<SL, DL, ADL><<<grid, kTargets, 0, st>>>(tg, mid, nrm, B, C, p, n, wc, wcs)
+    BAEMM_BY_LAYERS(BAEMM_PK)
 #undef BAEMM_PK
 }
 
 template <int COLS, bool RI>
-void pair_dispatch(int code, dim3 grid, cudaStream_t st, DenseTargets<float> tg, const float *mid, const float *nrm,
-                   const float2 *B, float2 *C, const ChunkParamsF *p, int n, int wc, int wcs, int per_split)
+void pair_dispatch(int code, dim3 grid, int cluster, cudaStream_t st, DenseTargets<float> tg, const float *mid,
+                   const float *nrm, const float2 *B, float2 *C, const ChunkParamsF *p, int n, int wc, int wcs,
+                   int per_part)
 {
 #define BAEMM_PR(SL, DL, ADL) \
-    boundary_pair_kernel<COLS, SL, DL, ADL, RI><<<grid, kTargets, 0, st>>>(tg, mid, nrm, B, C, p, n, wc, wcs, per_split)
-    switch (code)
-    {
-        case 1: BAEMM_PR(true, false, false); break;
-        case 2: BAEMM_PR(false, true, false); break;
-        case 3: BAEMM_PR(true, true, false); break;
-        case 4: BAEMM_PR(false, false, true); break;
-        case 5: BAEMM_PR(true, false, true); break;
-        case 6: BAEMM_PR(false, true, true); break;
-        case 7: BAEMM_PR(true, true, true); break;
-        default: break;
-    }
+    launch_clustered(boundary_pair_kernel<COLS, SL, DL, ADL, RI>, grid, kTargets, 0, st, cluster, tg, mid, nrm, B, C, p, \
+                     n, wc, wcs, per_part)
+    BAEMM_BY_LAYERS(BAEMM_PR)
 #undef BAEMM_PR
 }
 
-// Source splits of a launch of `ctas` CTAs over n sources (each split writes a
-// partial block, split_sum_kernel adds them): the s that minimises
-//     (n / s + kSplitCost) * max(ceil(ctas s / SMs), 2),
-// the sources of one CTA times the CTAs of the busiest SM.  An SM needs about
-// two CTAs before its FP32 pipe is shared rather than idle (hence the 2), and
-// a CTA costs about kSplitCost sources to start, drain and sum.  Without it a
-// launch of a few CTAs leaves most SMs idle, and one of 1.1 CTAs per SM runs
-// at half speed: 320 triangles x 16 columns ran 44 us as 3 CTAs of the scalar
-// kernel and 7.3 + 3.1 us (the sum) as 2 x 10 of the pair kernel, 5120 x 16
-// 480 us as 80 CTAs and 157 + 2.9 us split.
-constexpr int kSplitCost = 24, kSplitMin = 16, kSplitMax = 128;
-
-int dense_splits(int64_t ctas, int64_t n, int sms)
+// Room for the partial blocks of a split; with less, fewer of them (one: none).
+template <class R>
+cplx<R> *partial_blocks(SplitSpace<R> ws, int64_t elems, SourceSplit &split)
 {
-    int best = 1;
-    double best_cost = 0.0;
-    for (int s = 1; s <= kSplitMax && (s == 1 || n >= (int64_t)s * kSplitMin); ++s)
+    if (split.blocks == 1) return nullptr;
+    if (!ws.grow)
     {
-        const int64_t per_sm = std::max<int64_t>((ctas * s + sms - 1) / sms, 2);
-        const double cost = ((double)n / s + (s > 1 ? kSplitCost : 0)) * (double)per_sm;
-        if (s == 1 || cost < 0.97 * best_cost) { best = s; best_cost = cost; }
+        split.blocks = (int)std::max<size_t>(1, std::min<size_t>(split.blocks, ws.elems / elems));
+        return ws.fixed;
     }
-    return best;
+    try
+    {
+        return ws.grow->reserve((size_t)split.blocks * elems);
+    }
+    catch (const Error &)
+    {
+        split.blocks = 1;
+        return nullptr;
+    }
 }
 
-// Ctri (tg.m x wc) = K Btri over all nt sources for the targets tg, in as many
-// splits as ws can hold.
+// Ctri (tg.m x wc) = K Btri over all nt sources for the targets tg.
 template <class R>
 void dense_dispatch(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
                     DenseTargets<R> tg, const cplx<R> *Btri, cplx<R> *Ctri, cudaStream_t st, int variant,
                     SplitSpace<R> ws)
 {
     if (!f.any_layer() || m.nt == 0 || tg.m == 0) return;
+    BAEMM_REQUIRE(wcs >= 1 && wcs <= 64 && (wcs & (wcs - 1)) == 0, BAEMM_ERR_SIZE,
+                  "wave_chunk_size must be a power of two <= 64");
     const int n = (int)m.nt;
     const int cols = cols_for(wcs);
     const int code = (f.sl() ? 1 : 0) | (f.dl() ? 2 : 0) | (f.adl() ? 4 : 0);
     const auto *p = static_cast<const typename Prm<R>::type *>(chunk_params);
     const R *mid = geo_mid<R>(m), *nrm = geo_nrm<R>(m);
-    // plain FP32: the pair kernel unless a variant was set (its entry is shared by
-    // too few columns below 4 per chunk)
-    const bool pair = std::is_same<R, float>::value && (variant < 0 || variant == 2) && cols >= 4;
-    const bool packed = std::is_same<R, float>::value && variant == 1 && cols == kPackedCols;
-    const bool d64 = std::is_same<R, double>::value && cols >= 8;
-    dim3 grid(ceil_div(tg.m, pair ? 2 * kTargets : kTargets), wc / cols);
     const int64_t elems = (int64_t)tg.m * wc;
-    int splits = dense_splits(d64 ? d64_ctas(d64_unit(wc, wcs), tg.m, wc) : (int64_t)grid.x * grid.y, n, tc_sm_count());
-    cplx<R> *out = Ctri;
-    if (splits > 1 && ws.grow)
+    SourceSplit split;
+    cplx<R> *out = nullptr;
+    if constexpr (std::is_same<R, double>::value)
     {
-        try
-        {
-            out = ws.grow->reserve((size_t)splits * elems);
-        }
-        catch (const Error &)
-        {
-            splits = 1;   // no memory for the partial blocks: one sweep per target
-        }
+        split = dense_split(d64_ctas(d64_unit(wc, wcs), tg.m, wc), n, tc_sm_count());
+        out = partial_blocks<R>(ws, elems, split);
+        launch_boundary_d64(m, f, p, wc, wcs, tg, Btri, split.blocks > 1 ? out : Ctri, split, st);
     }
-    else if (splits > 1)
+    else
     {
-        splits = (int)std::max<size_t>(1, std::min<size_t>(splits, ws.elems / elems));
-        out = ws.fixed;
-    }
-    const int per_split = ceil_div(ceil_div(n, splits), 8) * 8;
-    grid.z = ceil_div(n, per_split);   // every split has sources
-    if (grid.z == 1) out = Ctri;
-    if constexpr (std::is_same<R, float>::value)
-    {
-        // single layer imaginary, double layers real (the tuples of the solves): RI
-        const bool ri = !f.re_sl && !f.im_dl && !f.im_adl;
+        // the pair kernel unless another variant was set
+        const dim3 grid(ceil_div(tg.m, kTargets), wc / cols);
+        if (variant == 1 && cols == kPackedCols) packed_dispatch(code, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs);
+        else if (variant == 0 || variant == 1)
+        {
+            if (cols == 16) scalar_dispatch<16>(code, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs);
+            else if (cols == 8) scalar_dispatch<8>(code, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs);
+            else if (cols == 4) scalar_dispatch<4>(code, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs);
+            else if (cols == 2) scalar_dispatch<2>(code, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs);
+            else scalar_dispatch<1>(code, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs);
+        }
+        else
+        {
+            dim3 pairs(ceil_div(tg.m, 2 * kTargets), wc / cols);
+            split = dense_split((int64_t)pairs.x * pairs.y, n, tc_sm_count());
+            out = partial_blocks<R>(ws, elems, split);
+            pairs.z = split.parts();
+            const int per_part = ceil_div(n, split.parts());
+            cplx<R> *dst = split.blocks > 1 ? out : Ctri;
+            // single layer imaginary, double layers real (the tuples of the solves): RI
+            const bool ri = !f.re_sl && !f.im_dl && !f.im_adl;
 #define BAEMM_PC(COLS) \
-    ri ? pair_dispatch<COLS, true>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split) \
-       : pair_dispatch<COLS, false>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split)
-        if (pair)
-        {
+    ri ? pair_dispatch<COLS, true>(code, pairs, split.cluster, st, tg, mid, nrm, Btri, dst, p, n, wc, wcs, per_part) \
+       : pair_dispatch<COLS, false>(code, pairs, split.cluster, st, tg, mid, nrm, Btri, dst, p, n, wc, wcs, per_part)
             if (cols == 16) BAEMM_PC(16);
             else if (cols == 8) BAEMM_PC(8);
-            else BAEMM_PC(4);
-        }
-        else if (packed) packed_dispatch(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split);
+            else if (cols == 4) BAEMM_PC(4);
+            else if (cols == 2) BAEMM_PC(2);
+            else BAEMM_PC(1);
 #undef BAEMM_PC
-    }
-    else if (d64) launch_boundary_d64(m, f, p, wc, wcs, tg, Btri, out, per_split, st);
-    if (!pair && !packed && !d64)
-        switch (cols)
-        {
-            case 1: boundary_cols<R, 1>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split); break;
-            case 2: boundary_cols<R, 2>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split); break;
-            case 4: boundary_cols<R, 4>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split); break;
-            case 8:
-                if constexpr (std::is_same<R, float>::value)
-                    boundary_cols<R, 8>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split);
-                break;
-            case 16:
-                if constexpr (std::is_same<R, float>::value)
-                    boundary_cols<R, 16>(code, grid, st, tg, mid, nrm, Btri, out, p, n, wc, wcs, per_split);
-                break;
-            default: throw Error(BAEMM_ERR_SIZE, "wave_chunk_size must be a power of two <= 64");
         }
-    if (!d64) BAEMM_LAUNCH_CHECK();
-    if (grid.z > 1)
+        BAEMM_LAUNCH_CHECK();
+    }
+    if (split.blocks > 1)
     {
-        split_sum_kernel<R><<<ceil_div(elems, 256), 256, 0, st>>>(out, (int)grid.z, elems, Ctri);
+        split_sum_kernel<R><<<ceil_div(elems, 256), 256, 0, st>>>(out, split.blocks, elems, Ctri);
         BAEMM_LAUNCH_CHECK();
     }
 }
 
 } // namespace
+
+// The split with the least estimated time,
+//     (n / parts + kSplitCost) * max(ceil(ctas parts / SMs), 2) [+ kSumCost if blocks > 1]:
+// the sources of one CTA times the CTAs of the busiest SM.  An SM needs about two
+// CTAs of four warps before its pipe is shared rather than idle (hence the 2); a
+// CTA costs about kSplitCost sources to start, drain and sum, and the sum of
+// partial blocks (one more kernel) about kSumCost.  Without a split a launch of a
+// few CTAs leaves most SMs idle, and one of 1.1 CTAs per SM runs at half speed.
+// Two parts share a cluster: larger ones leave SMs unevenly loaded (5120 x 16
+// host apply: 268 us without clusters, 250 with clusters of 2, 327 of 8; far
+// field of 81920 triangles in 256 directions x 32: 288, 285, 441).  Up to
+// kTiny sources one cluster takes all parts: its kernel is slower (320 x 16:
+// 13.2 instead of 7.3 + 3.1 us with its sum) but saves a launch, which is what
+// such a call waits for (27.3 instead of 29.4 us a call).
+SourceSplit dense_split(int64_t ctas, int64_t n, int sms)
+{
+    constexpr int kSplitCost = 24, kSumCost = 70, kMinSources = 16, kTiny = 512;
+    const int cluster = n <= kTiny ? 8 : 2, most = n <= kTiny ? 8 : 128;
+    SourceSplit best;
+    double best_cost = 0.0;
+    for (int parts = 1; parts <= most && (parts == 1 || n >= (int64_t)parts * kMinSources); parts += parts < cluster ? 1 : cluster)
+    {
+        const double per_sm = (double)std::max<int64_t>((ctas * parts + sms - 1) / sms, 2);
+        const double cost = ((double)n / parts + (parts > 1 ? kSplitCost : 0)) * per_sm + (parts > cluster ? kSumCost : 0);
+        if (parts == 1 || cost < 0.97 * best_cost)
+        {
+            best.cluster = std::min(parts, cluster);
+            best.blocks = parts / best.cluster;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
 
 template <class R>
 void launch_boundary_dense(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
@@ -965,21 +967,19 @@ void launch_pack_points(int64_t m, const double *pts3, R *pts4, cudaStream_t st)
     BAEMM_LAUNCH_CHECK();
 }
 
-static int farfield_splits(const MeshDev &m, int wc, int wcs, bool fp64)
+// FP64: the matrix-instruction form's split; FP32: parts of whole tiles, four CTAs per SM
+static SourceSplit farfield_split(const MeshDev &m, int wc, int wcs, bool fp64)
 {
-    const int cols = cols_for(wcs);
-    if (fp64 && cols >= 8) return dense_splits(d64_ctas(d64_unit(wc, wcs), m.nm, wc), m.nt, tc_sm_count());
-    const int ctas = ceil_div(m.nm, kTargets) * (wc / cols);
-    int splits = ceil_div(4 * 148, ctas);
-    const int max_splits = ceil_div(m.nt, kTile);
-    if (splits > max_splits) splits = max_splits;
-    if (splits < 1) splits = 1;
-    return splits;
+    if (fp64) return dense_split(d64_ctas(d64_unit(wc, wcs), m.nm, wc), m.nt, tc_sm_count());
+    const int ctas = ceil_div(m.nm, kTargets) * (wc / cols_for(wcs));
+    SourceSplit s;
+    s.blocks = std::max(1, std::min(ceil_div(4 * 148, ctas), ceil_div(m.nt, kTile)));
+    return s;
 }
 
 size_t farfield_partial_elems(const MeshDev &m, int wc, int wcs, bool fp64)
 {
-    return (size_t)farfield_splits(m, wc, wcs, fp64) * (size_t)m.nm * (size_t)wc;
+    return (size_t)farfield_split(m, wc, wcs, fp64).blocks * (size_t)m.nm * (size_t)wc;
 }
 
 template <class R>
@@ -988,35 +988,33 @@ void launch_farfield(const MeshDev &m, const OpFlags &f, const void *chunk_param
                      double2 *Cout, int64_t ldC, cudaStream_t st)
 {
     if (!(f.sl() || f.dl()) || m.nm == 0) return;
+    BAEMM_REQUIRE(wcs >= 1 && wcs <= 64 && (wcs & (wcs - 1)) == 0, BAEMM_ERR_SIZE,
+                  "wave_chunk_size must be a power of two <= 64");
     constexpr bool fp64 = std::is_same<R, double>::value;
-    int splits = farfield_splits(m, wc, wcs, fp64);
-    BAEMM_REQUIRE((size_t)splits * m.nm * wc <= partial_cap, BAEMM_ERR_SIZE, "far-field partial buffer too small");
-    const int cols = cols_for(wcs);
+    SourceSplit split = farfield_split(m, wc, wcs, fp64);
+    BAEMM_REQUIRE((size_t)split.blocks * m.nm * wc <= partial_cap, BAEMM_ERR_SIZE, "far-field partial buffer too small");
     const auto *p = static_cast<const typename Prm<R>::type *>(chunk_params);
-    const R *mid = geo_mid<R>(m), *nrm = geo_nrm<R>(m), *meas = geo_meas<R>(m);
     const int mm = (int)m.nm, n = (int)m.nt;
-    const int unit = fp64 && cols >= 8 ? 8 : kTile;   // sources a split is rounded up to
-    const int per_split = ceil_div(ceil_div(m.nt, splits), unit) * unit;
-    splits = ceil_div(m.nt, per_split);
-    dim3 grid(ceil_div(m.nm, kTargets), wc / cols, splits);
-    switch (cols)
+    if constexpr (fp64) launch_farfield_d64(m, f, p, wc, wcs, Btri, partial, split, st);
+    else
     {
-        case 1: farfield_cols<R, 1>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial); break;
-        case 2: farfield_cols<R, 2>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial); break;
-        case 4: farfield_cols<R, 4>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial); break;
-        case 8:
-            if constexpr (fp64) launch_farfield_d64(m, f, p, wc, wcs, Btri, partial, per_split, st);
-            else farfield_cols<R, 8>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial);
-            break;
-        case 16:
-            if constexpr (fp64) launch_farfield_d64(m, f, p, wc, wcs, Btri, partial, per_split, st);
-            else farfield_cols<R, 16>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial);
-            break;
-        default: throw Error(BAEMM_ERR_SIZE, "wave_chunk_size must be a power of two <= 64");
+        const int cols = cols_for(wcs);
+        const int per_split = ceil_div(ceil_div(n, split.blocks), kTile) * kTile;
+        split.blocks = ceil_div(n, per_split);
+        const dim3 grid(ceil_div(m.nm, kTargets), wc / cols, split.blocks);
+        const R *mid = geo_mid<R>(m), *nrm = geo_nrm<R>(m), *meas = geo_meas<R>(m);
+        switch (cols)
+        {
+            case 1: farfield_cols<R, 1>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial); break;
+            case 2: farfield_cols<R, 2>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial); break;
+            case 4: farfield_cols<R, 4>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial); break;
+            case 8: farfield_cols<R, 8>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial); break;
+            default: farfield_cols<R, 16>(f, grid, st, meas, mid, nrm, Btri, p, mm, n, wc, wcs, per_split, partial); break;
+        }
+        BAEMM_LAUNCH_CHECK();
     }
-    if (!(fp64 && cols >= 8)) BAEMM_LAUNCH_CHECK();
-    farfield_reduce_kernel<R><<<ceil_div((int64_t)mm * wc, 32), dim3(32, kReduceRows), 0, st>>>(partial, splits, mm, wc,
-                                                                                             alpha, beta, Cout, ldC);
+    farfield_reduce_kernel<R><<<ceil_div((int64_t)mm * wc, 32), dim3(32, kReduceRows), 0, st>>>(partial, split.blocks, mm,
+                                                                                             wc, alpha, beta, Cout, ldC);
     BAEMM_LAUNCH_CHECK();
 }
 

@@ -32,11 +32,13 @@
 // Measured: 22.1 ms on 41666 triangles x 32 columns (two wavenumbers, SL + DL;
 // 3.47e9 entries at 40 FP64 instructions and 48 matrix multiply-adds: 75 % of
 // the pipe), 41.6 ms before; far field of 81920 triangles in 256 directions x
-// 32 columns 281 us, 437 before; 1280 x 32 45 us, 446 before (unsplit).  Three
+// 32 columns 285 us, 437 before; 1280 x 32 46 us, 446 before (unsplit).  Three
 // blocks per SM (168 registers) took 24.0 ms, one wavenumber per unit 26.6 ms
 // at 2 to 4 blocks; staging element by element instead of in register order
 // cost 4 ms in bank conflicts.
 #include "ops.cuh"
+
+#include <cooperative_groups.h>
 
 #include <algorithm>
 #include <mutex>
@@ -121,7 +123,7 @@ struct Args
     const double2 *B;             // n x wc
     double2 *out;                 // splits x m x wc
     const ChunkParamsD *prm;
-    int n, wc, wcs, per_split;
+    int n, wc, wcs, cols, per_split;   // cols: real columns per set
 };
 
 // Entry evaluators.  Target: what a thread keeps per target.  pair(): what the
@@ -235,10 +237,9 @@ __global__ void __launch_bounds__(kThreads, 2) d64_kernel(const Args a)
 {
     extern __shared__ __align__(16) uint8_t raw[];
     Smem<E, NT> &sm = *reinterpret_cast<Smem<E, NT> *>(raw);
-    constexpr int COLS = E * NT * 8;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const int col0 = blockIdx.y * COLS;
+    const int col0 = blockIdx.y * E * a.cols;
     const int jb = blockIdx.z * a.per_split, je = min(a.n, jb + a.per_split);
     const int i0 = (blockIdx.x * 4 + warp) * kWarpTargets + g, i1 = i0 + 8;
     const int self0 = a.self ? a.off + i0 : -1, self1 = a.self ? a.off + i1 : -1;
@@ -286,9 +287,10 @@ __global__ void __launch_bounds__(kThreads, 2) d64_kernel(const Args a)
         for (int e = 0; e < kTurns; ++e)
         {
             const int kq = e * 4 + warp, j = j0 + kq / (E * NT) * 8 + t;
-            const double2 *src = a.B + (int64_t)j * a.wc + col0 + kq % (E * NT) * 8 + g;
-            b0[e] = j < je ? __ldg(src) : make_double2(0.0, 0.0);
-            b1[e] = j + 4 < je ? __ldg(src + 4 * (int64_t)a.wc) : make_double2(0.0, 0.0);
+            const int set = kq % (E * NT) / NT, c = kq % NT * 8 + g;   // column of the set
+            const double2 *src = a.B + (int64_t)j * a.wc + col0 + set * a.cols + c;
+            b0[e] = j < je && c < a.cols ? __ldg(src) : make_double2(0.0, 0.0);
+            b1[e] = j + 4 < je && c < a.cols ? __ldg(src + 4 * (int64_t)a.wc) : make_double2(0.0, 0.0);
         }
         #pragma unroll
         for (int e = 0; e < kTurns; ++e)
@@ -368,21 +370,31 @@ __global__ void __launch_bounds__(kThreads, 2) d64_kernel(const Args a)
         }
     }
     flush();
-    double2 *out = a.out + (int64_t)blockIdx.z * a.m * a.wc + col0;
-    #pragma unroll
-    for (int q = 0; q < E * NT; ++q)
-        #pragma unroll
-        for (int v = 0; v < 4; ++v)   // accumulator v: row g + 8 (v / 2), column 2 t + v % 2
+    // accumulator v of tile q: row g + 8 (v / 2), column 8 q + 2 t + v % 2; with a cluster
+    // of S parts, block r adds accumulators r, r + S, ... of all of them in order
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    if (S > 1) cluster.sync();
+    double2 *out = a.out + (int64_t)(blockIdx.z / S) * a.m * a.wc + col0;
+    for (int e = rank; e < E * NT * 4; e += S)
+    {
+        const int q = e / 4, v = e % 4;
+        double2 o = make_double2(0.0, 0.0);
+        for (int s = 0; s < S; ++s)
         {
-            const int i = v < 2 ? i0 : i1;
-            if (i < a.m)
-                out[(int64_t)i * a.wc + q * 8 + 2 * t + (v & 1)] =
-                    make_double2(sm.tot[q * 8 + 2 * v][tid], sm.tot[q * 8 + 2 * v + 1][tid]);
+            const double *tot = S > 1 ? cluster.map_shared_rank(&sm.tot[2 * e][tid], s) : &sm.tot[2 * e][tid];
+            o.x += tot[0];
+            o.y += tot[kThreads];
         }
+        const int i = v < 2 ? i0 : i1, c = q % NT * 8 + 2 * t + (v & 1);
+        if (i < a.m && c < a.cols) out[(int64_t)i * a.wc + q / NT * a.cols + c] = o;
+    }
+    if (S > 1) cluster.sync();   // no block leaves while its totals are read
 }
 
 template <class Entry, int E, int NT>
-void launch(const Args &a, dim3 grid, cudaStream_t st)
+void launch(const Args &a, dim3 grid, int cluster, cudaStream_t st)
 {
     constexpr size_t bytes = sizeof(Smem<E, NT>);
     // the shared-memory limit is a per-device attribute of the function
@@ -399,46 +411,50 @@ void launch(const Args &a, dim3 grid, cudaStream_t st)
             if (dev >= 0 && dev < 64) done[dev] = true;
         }
     }
-    d64_kernel<Entry, E, NT><<<grid, kThreads, bytes, st>>>(a);
+    launch_clustered(d64_kernel<Entry, E, NT>, grid, kThreads, bytes, st, cluster, a);
 }
 
 template <class Entry>
-void by_unit(const D64Unit &u, const Args &a, dim3 grid, cudaStream_t st)
+void by_unit(const D64Unit &u, const Args &a, dim3 grid, int cluster, cudaStream_t st)
 {
-    if (u.sets == 2 && u.tiles == 2) launch<Entry, 2, 2>(a, grid, st);
-    else if (u.sets == 2) launch<Entry, 2, 1>(a, grid, st);
-    else if (u.tiles == 4) launch<Entry, 1, 4>(a, grid, st);
-    else if (u.tiles == 2) launch<Entry, 1, 2>(a, grid, st);
-    else launch<Entry, 1, 1>(a, grid, st);
+    if (u.sets == 2 && u.tiles == 2) launch<Entry, 2, 2>(a, grid, cluster, st);
+    else if (u.sets == 2) launch<Entry, 2, 1>(a, grid, cluster, st);
+    else if (u.tiles == 4) launch<Entry, 1, 4>(a, grid, cluster, st);
+    else if (u.tiles == 2) launch<Entry, 1, 2>(a, grid, cluster, st);
+    else launch<Entry, 1, 1>(a, grid, cluster, st);
 }
 
 template <bool RI>
-void by_layers(int code, const D64Unit &u, const Args &a, dim3 grid, cudaStream_t st)
+void by_layers(int code, const D64Unit &u, const Args &a, dim3 grid, int cluster, cudaStream_t st)
 {
     switch (code)
     {
-        case 1: by_unit<BoundaryEntry<true, false, false, RI>>(u, a, grid, st); break;
-        case 2: by_unit<BoundaryEntry<false, true, false, RI>>(u, a, grid, st); break;
-        case 3: by_unit<BoundaryEntry<true, true, false, RI>>(u, a, grid, st); break;
-        case 4: by_unit<BoundaryEntry<false, false, true, RI>>(u, a, grid, st); break;
-        case 5: by_unit<BoundaryEntry<true, false, true, RI>>(u, a, grid, st); break;
-        case 6: by_unit<BoundaryEntry<false, true, true, RI>>(u, a, grid, st); break;
-        case 7: by_unit<BoundaryEntry<true, true, true, RI>>(u, a, grid, st); break;
+        case 1: by_unit<BoundaryEntry<true, false, false, RI>>(u, a, grid, cluster, st); break;
+        case 2: by_unit<BoundaryEntry<false, true, false, RI>>(u, a, grid, cluster, st); break;
+        case 3: by_unit<BoundaryEntry<true, true, false, RI>>(u, a, grid, cluster, st); break;
+        case 4: by_unit<BoundaryEntry<false, false, true, RI>>(u, a, grid, cluster, st); break;
+        case 5: by_unit<BoundaryEntry<true, false, true, RI>>(u, a, grid, cluster, st); break;
+        case 6: by_unit<BoundaryEntry<false, true, true, RI>>(u, a, grid, cluster, st); break;
+        case 7: by_unit<BoundaryEntry<true, true, true, RI>>(u, a, grid, cluster, st); break;
         default: break;
     }
 }
 
-dim3 grid_of(const D64Unit &u, int64_t m, int64_t n, int wc, int per_split)
+dim3 grid_of(const D64Unit &u, int64_t m, int wc, SourceSplit split)
 {
-    return dim3(ceil_div(m, 4 * kWarpTargets), wc / u.columns(), ceil_div(n, per_split));
+    return dim3(ceil_div(m, 4 * kWarpTargets), wc / u.columns(), split.parts());
 }
+
+// sources per part, whole steps of 8
+int part_of(int64_t n, SourceSplit split) { return ceil_div(ceil_div(n, split.parts()), 8) * 8; }
 
 } // namespace
 
 D64Unit d64_unit(int wc, int wcs)
 {
     D64Unit u;
-    u.tiles = wcs >= 32 ? 4 : wcs / 8;
+    u.tiles = wcs >= 32 ? 4 : wcs >= 16 ? 2 : 1;
+    u.cols = std::min(wcs, u.tiles * 8);
     u.sets = wcs <= 16 && (wc / wcs) % 2 == 0 ? 2 : 1;
     return u;
 }
@@ -446,28 +462,31 @@ D64Unit d64_unit(int wc, int wcs)
 int64_t d64_ctas(const D64Unit &u, int64_t m, int wc) { return (int64_t)ceil_div(m, 4 * kWarpTargets) * (wc / u.columns()); }
 
 void launch_boundary_d64(const MeshDev &m, const OpFlags &f, const ChunkParamsD *prm, int wc, int wcs,
-                         const DenseTargets<double> &tg, const double2 *Btri, double2 *out, int per_split,
+                         const DenseTargets<double> &tg, const double2 *Btri, double2 *out, SourceSplit split,
                          cudaStream_t st)
 {
     const D64Unit u = d64_unit(wc, wcs);
     const Args a{tg.pts4, m.nrm_d + 4 * (int64_t)tg.off, tg.m, tg.self, tg.off, m.mid_d, m.nrm_d, Btri, out, prm,
-                 (int)m.nt, wc, wcs, per_split};
-    const dim3 grid = grid_of(u, tg.m, m.nt, wc, per_split);
+                 (int)m.nt, wc, wcs, u.cols, part_of(m.nt, split)};
+    const dim3 grid = grid_of(u, tg.m, wc, split);
+    const int cluster = split.cluster;
     const int code = (f.sl() ? 1 : 0) | (f.dl() ? 2 : 0) | (f.adl() ? 4 : 0);
-    if (!f.re_sl && !f.im_dl && !f.im_adl) by_layers<true>(code, u, a, grid, st);
-    else by_layers<false>(code, u, a, grid, st);
+    if (!f.re_sl && !f.im_dl && !f.im_adl) by_layers<true>(code, u, a, grid, cluster, st);
+    else by_layers<false>(code, u, a, grid, cluster, st);
     BAEMM_LAUNCH_CHECK();
 }
 
 void launch_farfield_d64(const MeshDev &m, const OpFlags &f, const ChunkParamsD *prm, int wc, int wcs,
-                         const double2 *Btri, double2 *partial, int per_split, cudaStream_t st)
+                         const double2 *Btri, double2 *partial, SourceSplit split, cudaStream_t st)
 {
     const D64Unit u = d64_unit(wc, wcs);
-    const Args a{m.meas_d, nullptr, (int)m.nm, 0, 0, m.mid_d, m.nrm_d, Btri, partial, prm, (int)m.nt, wc, wcs, per_split};
-    const dim3 grid = grid_of(u, m.nm, m.nt, wc, per_split);
-    if (f.sl() && f.dl()) by_unit<FarEntry<true, true>>(u, a, grid, st);
-    else if (f.sl()) by_unit<FarEntry<true, false>>(u, a, grid, st);
-    else by_unit<FarEntry<false, true>>(u, a, grid, st);
+    const Args a{m.meas_d, nullptr, (int)m.nm, 0, 0, m.mid_d, m.nrm_d, Btri, partial, prm,
+                 (int)m.nt, wc, wcs, u.cols, part_of(m.nt, split)};
+    const dim3 grid = grid_of(u, m.nm, wc, split);
+    const int cluster = split.cluster;
+    if (f.sl() && f.dl()) by_unit<FarEntry<true, true>>(u, a, grid, cluster, st);
+    else if (f.sl()) by_unit<FarEntry<true, false>>(u, a, grid, cluster, st);
+    else by_unit<FarEntry<false, true>>(u, a, grid, cluster, st);
     BAEMM_LAUNCH_CHECK();
 }
 

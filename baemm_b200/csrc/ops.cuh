@@ -118,9 +118,8 @@ void launch_axpby(int64_t rows, int cols, T a, const T *x, int64_t ldx, T b, T *
 // Dense boundary kernel (BoundaryOperatorKernel.cl:5-239): Ctri = K(kappa) Btri
 // chunk by chunk, the self pair excluded.  R = float (plain FP32) or double.
 // variant (FP32): 0 scalar FMA kernel, 1 packed FP32x2 kernel (16-column
-// groups), 2 FP32x2 kernel over pairs of targets (groups of 4 columns and
-// more), -1 the library's choice (2 where it applies); where a variant does not
-// apply, 0.  [row_begin, row_end) restricts the targets to those triangles
+// groups; else 0), 2 FP32x2 kernel over pairs of targets, -1 the library's
+// choice (2).  [row_begin, row_end) restricts the targets to those triangles
 // (rows of Ctri outside are not written; row_end < 0: all).
 constexpr int kDenseVariants = 3;
 // Where a launch that is split over the sources keeps its partial blocks: a
@@ -136,22 +135,51 @@ template <class R>
 void launch_boundary_dense(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
                            const cplx<R> *Btri, cplx<R> *Ctri, cudaStream_t st, SplitSpace<R> ws, int variant = -1,
                            int64_t row_begin = 0, int64_t row_end = -1);
+// How a dense launch splits the sources: cluster * blocks parts.  The parts of a
+// cluster are summed through distributed shared memory; each of the `blocks`
+// clusters of a target block writes a partial block (none when blocks == 1).
+struct SourceSplit
+{
+    int cluster = 1, blocks = 1;
+    int parts() const { return cluster * blocks; }
+};
+SourceSplit dense_split(int64_t ctas, int64_t n, int sms);
+
+// Launch with thread-block clusters of `cluster` blocks along z.
+template <class... P, class... A>
+void launch_clustered(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, int cluster, A... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = cluster;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    BAEMM_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}
+
 // ---- dense64.cu: the FP64 forms on the FP64 matrix instructions --------------------
-// They take chunks of 8 columns and more.  A work unit is `sets` wavenumbers of
-// tiles * 8 columns each; splits of `per_split` sources write partial blocks
-// (ceil(n / per_split) x m x wc), summed by the caller.
+// A work unit is `sets` wavenumbers of tiles * 8 columns each (padded where a
+// chunk has fewer).  Part z of the sources (per_split of them) is summed within
+// its cluster; the clusters write partial blocks (blocks x m x wc), summed by
+// the caller.
 struct D64Unit
 {
-    int sets = 1, tiles = 1;
-    int columns() const { return sets * tiles * 8; }
+    int sets = 1, tiles = 1, cols = 8;   // cols: real columns per set, at most tiles * 8
+    int columns() const { return sets * cols; }
 };
 D64Unit d64_unit(int wc, int wcs);
 int64_t d64_ctas(const D64Unit &u, int64_t m, int wc);
 void launch_boundary_d64(const MeshDev &m, const OpFlags &f, const ChunkParamsD *prm, int wc, int wcs,
-                         const DenseTargets<double> &tg, const double2 *Btri, double2 *out, int per_split,
+                         const DenseTargets<double> &tg, const double2 *Btri, double2 *out, SourceSplit split,
                          cudaStream_t st);
 void launch_farfield_d64(const MeshDev &m, const OpFlags &f, const ChunkParamsD *prm, int wc, int wcs,
-                         const double2 *Btri, double2 *partial, int per_split, cudaStream_t st);
+                         const double2 *Btri, double2 *partial, SourceSplit split, cudaStream_t st);
 // Near-field kernel (NearFieldOperatorKernel.cl:5-194): Cpts (npts x wc) =
 // K(kappa) Btri at the points pts4 (npts x 4 reals), single and double layer
 // (c1, c2) only, no pair excluded.  Same kernels and variants as the boundary form.

@@ -523,7 +523,7 @@ class Helmholtz_CUDA:
                    "GB_s": float(out[5 + q] / (out[q] * 1e-3) / 1e9) if out[q] > 0 else None}
                for q, n in enumerate(names)}
         # one CG iteration on the path this mesh's solves take (baemm_profile_cg): on meshes of up to
-        # 16384 vertices one block per column runs every iteration in one launch, so the three kernels
+        # 16384 vertices a cluster of blocks per column runs every iteration in one launch, so the three kernels
         # above are not what the solver runs there
         cg = np.zeros(3)
         self._ck(self._lib.baemm_profile_cg(self._h, int(columns), int(iterations), _dp(cg)))

@@ -355,7 +355,7 @@ int baemm_selftest_bounded_wait(int device, double *elapsed_ms, int *code);
  * columns (columns complex), `iterations` iterations with no column allowed
  * to converge.  out[0] = ms per iteration, out[1] = algorithmic bytes of one
  * iteration (matvec, update and p update), out[2] = 1 when the mesh (at most
- * 16384 vertices) takes the one-launch path (one block per column, every
+ * 16384 vertices) takes the one-launch path (a cluster of blocks per column, every
  * iteration in one launch), 0 for the three-launches-per-iteration kernels
  * of larger meshes. */
 int baemm_profile_cg(baemm_ctx *ctx, int columns, int iterations, double out[3]);
