@@ -533,16 +533,18 @@ int baemm_get_single_layer_diagonal(baemm_ctx *ctx, float *out)
 int baemm_get_mass_matrix(baemm_ctx *ctx, int64_t *outer, int32_t *inner, float *values, int64_t *nnz)
 {
     return guarded(ctx, [&](Ctx &c) {
-        const int64_t z = (int64_t)c.mass_inner_h.size();
+        const int64_t z = c.mass_nnz;
         if (nnz) *nnz = z;
         if (!outer) return;
-        for (int64_t v = 0; v <= c.mesh.nv; ++v) outer[v] = c.mass_outer_h[v];
-        if (inner) std::memcpy(inner, c.mass_inner_h.data(), z * sizeof(int32_t));
+        std::vector<int32_t> o((size_t)c.mesh.nv + 1);
+        BAEMM_CUDA(cudaMemcpyAsync(o.data(), c.mesh.mass_outer.p, o.size() * sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                   c.stream));
+        if (inner)
+            BAEMM_CUDA(cudaMemcpyAsync(inner, c.mesh.mass_inner.p, z * sizeof(int32_t), cudaMemcpyDeviceToHost, c.stream));
         if (values)
-        {
             BAEMM_CUDA(cudaMemcpyAsync(values, c.mesh.mass_f.p, z * sizeof(float), cudaMemcpyDeviceToHost, c.stream));
-            c.sync();
-        }
+        c.sync();
+        std::copy(o.begin(), o.end(), outer);
     });
 }
 int baemm_get_curl_operator(baemm_ctx *ctx, int64_t *outer, int32_t *inner, float *values, int64_t *nnz)
@@ -730,7 +732,7 @@ int baemm_profile_krylov(baemm_ctx *ctx, int columns, int iterations, int basis,
         baemm::CgSolver cg;
         cg.profile(c.mesh, v64, rc, iterations, c.stream, cg_ms);
         baemm::profile_gram_schmidt(c.mesh.nv, columns, basis, iterations, c.stream, gs_ms);
-        const double n = (double)c.mesh.nv, nnz = (double)c.mass_inner_h.size(), vs = v64 ? 8.0 : 4.0;
+        const double n = (double)c.mesh.nv, nnz = (double)c.mass_nnz, vs = v64 ? 8.0 : 4.0;
         const double vec = n * rc * 8.0, cvec = n * columns * 16.0;
         out[0] = cg_ms[0]; out[1] = cg_ms[1]; out[2] = cg_ms[2]; out[3] = gs_ms[0]; out[4] = gs_ms[1];
         out[5] = (n + 1) * 4 + nnz * (4 + vs) + 2 * vec;   // CSR, p gathered once, q written
@@ -750,7 +752,7 @@ int baemm_profile_cg(baemm_ctx *ctx, int columns, int iterations, double out[3])
         const bool v64 = c.mass_values_fp64();
         const int rc = 2 * columns;   // complex columns as interleaved real columns (ApplyMassInverse.hpp:71-98)
         baemm::CgSolver cg;
-        const double n = (double)c.mesh.nv, nnz = (double)c.mass_inner_h.size(), vs = v64 ? 8.0 : 4.0;
+        const double n = (double)c.mesh.nv, nnz = (double)c.mass_nnz, vs = v64 ? 8.0 : 4.0;
         const double vec = n * rc * 8.0;
         // algorithmic bytes of one iteration: the matvec (CSR, p gathered once, q written), the update
         // (L; x, p, r, q read; x, r, z written) and the p update (z, p read; p written)

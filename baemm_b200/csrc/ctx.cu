@@ -63,13 +63,17 @@ void Ctx::init_mesh(const double *coords, int64_t nv, const int32_t *tris, int64
                                stream));
     BAEMM_CUDA(cudaMemcpyAsync(mesh.tris.reserve(3 * nt), tris, 3 * nt * sizeof(int32_t), cudaMemcpyHostToDevice,
                                stream));
-    build_topology(tris);   // ends with a stream synchronisation: the host arrays are free afterwards
+    if (!topo_host) BAEMM_CUDA(cudaMallocHost(&topo_host, 2 * sizeof(int32_t)));
+    // either ends with a stream synchronisation: the host arrays are free afterwards
+    mass_nnz = launch_topology(mesh, topo_scratch, topo_host, stream);
+    if (mass_nnz < 0) build_topology_host(tris);
+    if (topo_scratch.n > (size_t)1 << 24) topo_scratch.release();   // 64 MB: not kept
 
     mesh.mid_f.reserve(4 * nt); mesh.nrm_f.reserve(4 * nt);
     mesh.area_f.reserve(nt); mesh.a3_f.reserve(nt); mesh.diag_f.reserve(nt);
     mesh.mid_d.reserve(4 * nt); mesh.nrm_d.reserve(4 * nt);
     mesh.area_d.reserve(nt); mesh.a3_d.reserve(nt); mesh.diag_d.reserve(nt);
-    mesh.mass_f.reserve(mass_inner_h.size()); mesh.mass_d.reserve(mass_inner_h.size());
+    mesh.mass_f.reserve(mass_nnz); mesh.mass_d.reserve(mass_nnz);
     mesh.lumped_f.reserve(nv); mesh.lumped_d.reserve(nv);
     if (nv <= kMassEllMaxRows)
     {
@@ -166,6 +170,7 @@ Ctx::~Ctx()
 {
     clear_graphs();
     if (tc_err_host) cudaFreeHost(tc_err_host);
+    if (topo_host) cudaFreeHost(topo_host);
     for (auto &e : prof_ev)
         if (e) cudaEventDestroy(e);
     if (handoff_ev) cudaEventDestroy(handoff_ev);
@@ -208,10 +213,9 @@ void Ctx::check_tc_error()
     }
 }
 
-// Integer topology (host): AvOp columns sorted per triangle (Initialize.hpp:307-313),
-// AvOp^T as a vertex -> triangle CSR in ascending triangle order (Initialize.hpp:315),
-// and the sparsity pattern of the P1 mass matrix (Initialize.hpp:329-334).
-void Ctx::build_topology(const int32_t *tris)
+// launch_topology's arrays by sorting on the host, for meshes with a vertex of
+// more than kTopologyDegree triangles.
+void Ctx::build_topology_host(const int32_t *tris)
 {
     const int64_t nv = mesh.nv, nt = mesh.nt;
     std::vector<int32_t> ts(3 * nt);
@@ -237,8 +241,8 @@ void Ctx::build_topology(const int32_t *tris)
             for (int q = 0; q < 3; ++q) keys.push_back((int64_t)tris[3 * i + p] * nv + tris[3 * i + q]);
     std::sort(keys.begin(), keys.end());
     keys.erase(std::unique(keys.begin(), keys.end()), keys.end());
-    mass_outer_h.assign(nv + 1, 0);
-    mass_inner_h.resize(keys.size());
+    std::vector<int32_t> mass_outer_h(nv + 1, 0), mass_inner_h(keys.size());
+    mass_nnz = (int64_t)keys.size();
     for (size_t e = 0; e < keys.size(); ++e)
     {
         mass_outer_h[keys[e] / nv + 1]++;

@@ -32,7 +32,9 @@ public:
     cudaStream_t stream = nullptr;
     MeshDev mesh;
     std::vector<double> meas_h;                     // nm x 3 (as given)
-    std::vector<int32_t> mass_outer_h, mass_inner_h;
+    int64_t mass_nnz = 0;
+    DevBuf<int32_t> topo_scratch;
+    int32_t *topo_host = nullptr;                   // pinned: what launch_topology reads back
 
     int wave_count = 0, wave_chunk_size = 16, wave_chunk_count = 0;
     std::vector<double> kappa_h;
@@ -210,7 +212,7 @@ public:
 
 private:
     void init_mesh(const double *coords, int64_t nv, const int32_t *tris, int64_t nt);
-    void build_topology(const int32_t *tris);
+    void build_topology_host(const int32_t *tris);
     template <class R>
     void dense_apply(const cplx<R> *Btri, cplx<R> *Ctri, int64_t r0 = 0, int64_t r1 = -1);
 };

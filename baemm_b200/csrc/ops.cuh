@@ -50,6 +50,14 @@ struct DenseTargets
     int off;
 };
 
+// ---- topology.cu ---------------------------------------------------------------
+// tri_sorted, avt_outer, avt_inner, mass_outer, mass_inner of m.tris on the
+// device; returns the entries of the mass matrix, or -1 (the arrays then hold
+// nothing) where a vertex has more than kTopologyDegree triangles.  Waits for
+// the stream; host2: two pinned ints.
+constexpr int kTopologyDegree = 64;
+int64_t launch_topology(MeshDev &m, DevBuf<int32_t> &scratch, int32_t *host2, cudaStream_t st);
+
 // ---- mesh.cu -------------------------------------------------------------------
 // Initialize.hpp:57-302 (geometry and single-layer diagonal) in precision R.
 void launch_geometry(const MeshDev &m, bool fp64, cudaStream_t st);

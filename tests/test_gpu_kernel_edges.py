@@ -157,3 +157,57 @@ def test_one_launch_mass_inverse(mesh, ncols):
                 orc.ApplyMassInverse(np.ascontiguousarray(X[:, k:k + 1]), one, 1e-10)
                 ref[:, k] = one[:, 0]
             assert relerr(got, ref) < tol, mode
+
+
+def _mass_pattern(nv, tris):
+    rows = [set() for _ in range(nv)]
+    for t in np.asarray(tris).tolist():
+        for v in t:
+            rows[v].update(t)
+    outer = np.concatenate([[0], np.cumsum([len(r) for r in rows])])
+    return outer, np.concatenate([sorted(r) for r in rows if r]).astype(np.int32)
+
+
+def _shuffled(mesh, extra=0):
+    """The mesh with its triangles and vertices in random order, `extra` vertices in no triangle."""
+    coords, tris = mesh
+    rng = np.random.default_rng(1)
+    perm = rng.permutation(len(coords) + extra)
+    out = rng.standard_normal((len(coords) + extra, 3))
+    out[perm[:len(coords)]] = coords
+    return out, perm[np.asarray(tris)][rng.permutation(len(tris))]
+
+
+@pytest.mark.parametrize("name,mesh", [
+    ("one triangle", (np.eye(3), np.array([[2, 0, 1]]))), ("torus 3 x 3", meshes.torus(n_minor=3, n_major=3)),
+    ("degree 64", _shuffled(_bipyramid(64), 3)), ("degree 65", _shuffled(_bipyramid(65), 3)),
+    ("2046 vertices", _shuffled(meshes.torus(n_minor=31, n_major=66))),
+    ("2047 vertices", _shuffled(meshes.torus(n_minor=23, n_major=89))),
+    ("2048 vertices", _shuffled(meshes.torus(n_minor=32, n_major=64), 1)),
+    ("icosphere 5", _shuffled(meshes.icosphere(5), 2))], ids=lambda p: p if isinstance(p, str) else "")
+def test_topology(name, mesh):
+    """Rows of the mass matrix (device and host construction, tiles of the scan)
+    and an apply over the vertex -> triangle rows, re-meshing a context that held another mesh."""
+    coords, tris = mesh
+    with Helmholtz_CUDA(*meshes.icosphere(2), np.eye(3)) as H:
+        H.SetMesh(coords, tris)
+        outer, inner, vals = H.MassMatrix()
+        ref_outer, ref_inner = _mass_pattern(len(coords), tris)
+        assert np.array_equal(outer, ref_outer) and np.array_equal(inner, ref_inner)
+        p = coords[tris]
+        area = 0.5 * np.linalg.norm(np.cross(p[:, 1] - p[:, 0], p[:, 2] - p[:, 0]), axis=1)
+        assert abs(vals.sum() - area.sum()) < 1e-5 * area.sum()
+        if name in ("icosphere 5", "degree 65"):
+            X = np.random.default_rng(2).standard_normal((len(coords), 2))
+            got, ref = np.zeros_like(X), np.zeros_like(X)
+            w = area[:, None, None] / 12
+            np.add.at(ref, tris, w * (X[tris] + X[tris].sum(axis=1, keepdims=True)))
+            assert relerr(H.MassDot(1.0, X, 0.0, got), ref) < TOL32
+            kap, coeff = np.array([2.0]), np.array([COEFF["bie"](2.0)], np.complex128)
+            B = crandn(np.random.default_rng(3), len(coords), 4)
+            got, ref = np.zeros_like(B), np.zeros_like(B)
+            H.SetApplyMode(APPLY_FP64)
+            H.ApplyBoundaryOperators_PL(1.0, B, 0.0, got, kap, coeff, 4, 4)
+            O.Oracle(coords, tris, np.eye(3), precision=64).ApplyBoundaryOperators_PL(1.0, B, 0.0, ref, kap, coeff, 4, 4)
+            used = np.unique(tris)
+            assert relerr(got[used], ref[used]) < TOL64
