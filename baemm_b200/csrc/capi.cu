@@ -207,6 +207,8 @@ static void mass_inverse_host(Ctx &c, const double *X, int64_t ldX, double *Y, i
     h2d_block<double>(c, dX, X, nv, cols, ldX);
     c.stats.cg_converged = 1;
     c.stats.cg_iterations = 0;
+    c.cg.reset_stats(c.stream);
+    c.cg_pending = false;
     if (lumped) baemm::launch_lumped_real(c.mesh, c.mass_values_fp64(), dX, cols, dY, cols, cols, c.stream);
     else c.mass_inverse_real(dX, cols, dY, cols, cols, tol);
     d2h_block<double>(c, Y, ldY, dY, nv, cols);

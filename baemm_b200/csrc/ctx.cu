@@ -193,7 +193,14 @@ void Ctx::switch_stream(cudaStream_t s)
 
 void Ctx::sync()
 {
+    if (cg_pending) cg.read_stats(stream);
     BAEMM_CUDA(cudaStreamSynchronize(stream));
+    if (cg_pending)
+    {
+        cg_pending = false;
+        stats.cg_iterations = std::max(stats.cg_iterations, cg.most_iterations());
+        stats.cg_converged = stats.cg_converged && cg.all_converged();
+    }
     if (tc_pending) check_tc_error();
 }
 
@@ -603,32 +610,35 @@ void Ctx::herglotz(zc alpha, const double2 *g, int64_t ldg, zc beta, double2 *C,
     }
 }
 
-bool Ctx::mass_inverse_real(const double *X, int64_t ldX, double *Y, int64_t ldY, int ncols, double tol)
+void Ctx::mass_inverse_real(const double *X, int64_t ldX, double *Y, int64_t ldY, int ncols, double tol)
 {
-    int it = 0;
     // ApplyMassInverse.hpp:48: max_iter = 20
     const bool v64 = mass_values_fp64();
-    bool ok;
+    auto enqueue = [&] { cg.enqueue_mass(mesh, v64, X, ldX, Y, ldY, ncols, tol, 20, stream); };
     if (use_graphs)
     {
         long long tb = 0;
         std::memcpy(&tb, &tol, sizeof(tb));
-        run_graphed(GraphKey{2, X, Y, ldX, ldY, 2LL * ncols + (v64 ? 1 : 0), tb},
-                    [&] { cg.enqueue_mass(mesh, v64, X, ldX, Y, ldY, ncols, tol, 20, stream); });
-        ok = cg.finish(stream, &it);
+        run_graphed(GraphKey{2, X, Y, ldX, ldY, 2LL * ncols + (v64 ? 1 : 0), tb}, enqueue);
     }
     else
-        ok = cg.solve_mass(mesh, v64, X, ldX, Y, ldY, ncols, tol, 20, stream, &it);
-    stats.cg_iterations = std::max(stats.cg_iterations, it);
-    stats.cg_converged = stats.cg_converged && ok;
-    return ok;
+        enqueue();
+    cg_pending = true;
 }
 
-bool Ctx::mass_inverse_complex(const double2 *X, int64_t ldX, double2 *Y, int64_t ldY, int ncols, double tol)
+void Ctx::mass_inverse_complex(const double2 *X, int64_t ldX, double2 *Y, int64_t ldY, int ncols, double tol)
 {
     // complex columns as interleaved real columns (ApplyMassInverse.hpp:71-98)
-    return mass_inverse_real(reinterpret_cast<const double *>(X), 2 * ldX, reinterpret_cast<double *>(Y), 2 * ldY,
-                             2 * ncols, tol);
+    mass_inverse_real(reinterpret_cast<const double *>(X), 2 * ldX, reinterpret_cast<double *>(Y), 2 * ldY, 2 * ncols,
+                      tol);
+}
+
+void Ctx::reset_stats()
+{
+    stats = baemm_solve_stats{};
+    stats.cg_converged = 1;
+    cg.reset_stats(stream);
+    cg_pending = false;
 }
 
 std::string Ctx::device_info() const

@@ -65,6 +65,8 @@ public:
     int ir_max_steps = 0;
     double ir_inner_tol = 1e-4;
     baemm_solve_stats stats{};
+    bool cg_pending = false;          // mass inverses since the last sync()
+    void reset_stats();
     DevBuf<int> tc_err;               // error word of the tensor-core kernel's bounded waits
     DevBuf<double> reduce_scratch;    // per-block partial sums of device_dot / device_colnorms
     int *tc_err_host = nullptr;
@@ -134,9 +136,9 @@ public:
     // when the apply is FP64 or when FP64 iterative refinement is on.
     bool aux_fp64() const { return apply_mode == BAEMM_APPLY_FP64 || ir_max_steps > 0; }
     bool mass_values_fp64() const { return aux_fp64(); }
-    // CG mass inverse on real columns (device); returns convergence
-    bool mass_inverse_real(const double *X, int64_t ldX, double *Y, int64_t ldY, int ncols, double tol);
-    bool mass_inverse_complex(const double2 *X, int64_t ldX, double2 *Y, int64_t ldY, int ncols, double tol);
+    // CG mass inverse on real columns (device); its convergence joins `stats` at the next sync()
+    void mass_inverse_real(const double *X, int64_t ldX, double *Y, int64_t ldY, int ncols, double tol);
+    void mass_inverse_complex(const double2 *X, int64_t ldX, double2 *Y, int64_t ldY, int ncols, double tol);
 
     // ---- solvers (device blocks, nv x wc) -------------------------------------------
     // GMRES on the loaded boundary operators with P = M^-1 (BoundaryPotential_parameters /

@@ -411,8 +411,8 @@ __global__ void cg_pupdate_kernel(int64_t total, int c, const double *__restrict
 // iteration q = M p, alpha = <r,z> / <p,q>, x += alpha p, r -= alpha q, z = L r,
 // beta = <r,z>_new / <r,z>, converged once ||r|| <= tol ||b|| (a column of zeros
 // at once), p = z + beta p.  All sums are in fixed orders, so runs are
-// reproducible.  flags: [0] columns not converged, [1] the largest iteration
-// count (both zeroed before the launch), [2 + k] column k converged.
+// reproducible.  stats (accumulated): [0] columns not converged, [1] the largest
+// iteration count.
 //
 // Bound by latency (barriers, block sums) on small meshes and by the matrix
 // stream from L2 where it does not fit.  One block per column, the CSR rows read
@@ -465,7 +465,7 @@ template <class RV>
 __global__ void __launch_bounds__(kCgThreads, 1)
 cg_cluster_kernel(int64_t n, int rpc, int staged, const double *b, int64_t ldb, const int32_t *__restrict__ mo,
                   const int32_t *__restrict__ mi, const RV *__restrict__ mv, const uint16_t *__restrict__ ell_idx,
-                  const RV *__restrict__ ell_val, const RV *__restrict__ L, double *y, int64_t ldy, int *flags,
+                  const RV *__restrict__ ell_val, const RV *__restrict__ L, double *y, int64_t ldy, int *stats,
                   double tol, int max_iter)
 {
     namespace cg = cooperative_groups;
@@ -594,15 +594,21 @@ cg_cluster_kernel(int64_t n, int rpc, int staged, const double *b, int64_t ldb, 
     for (int row = tid; row < m; row += T) y[(int64_t)(r0 + row) * ldy + k] = x[row];
     if (rank == 0 && tid == 0)
     {
-        flags[2 + k] = conv ? 1 : 0;
-        if (!conv) atomicAdd(&flags[0], 1);
-        atomicMax(&flags[1], it);
+        if (!conv) atomicAdd(&stats[0], 1);
+        atomicMax(&stats[1], it);
     }
+}
+
+// The same statistics of a solve by the multi-block kernels
+__global__ void cg_stats_kernel(const int *__restrict__ flags, int *__restrict__ stats)
+{
+    if (!flags[0]) atomicAdd(&stats[0], 1);
+    atomicMax(&stats[1], flags[1]);
 }
 
 template <class RV>
 void launch_cg_cluster(cudaStream_t st, const MeshDev &mesh, int c, const double *b, int64_t ldb, const RV *mv,
-                       const RV *ell_val, const RV *L, double *y, int64_t ldy, int *flags, double tol, int max_iter)
+                       const RV *ell_val, const RV *L, double *y, int64_t ldy, int *stats, double tol, int max_iter)
 {
     // the limit above 48 KB is a per-device attribute of each instantiation, set once
     int dev = 0;
@@ -632,7 +638,7 @@ void launch_cg_cluster(cudaStream_t st, const MeshDev &mesh, int c, const double
     cfg.numAttrs = 1;
     BAEMM_CUDA(cudaLaunchKernelEx(&cfg, cg_cluster_kernel<RV>, mesh.nv, h.rpc, h.staged, b, ldb,
                                   (const int32_t *)mesh.mass_outer.p, (const int32_t *)mesh.mass_inner.p, mv,
-                                  (const uint16_t *)mesh.mass_ell_idx.p, ell_val, L, y, ldy, flags, tol, max_iter));
+                                  (const uint16_t *)mesh.mass_ell_idx.p, ell_val, L, y, ldy, stats, tol, max_iter));
 }
 
 __global__ void cg_output_kernel(int64_t n, int c, const double *__restrict__ x, double *__restrict__ y, int64_t ldy)
@@ -907,22 +913,18 @@ inline int eg(int64_t n) { return ceil_div(n, 256); }
 // =================================== CG host ======================================
 CgSolver::~CgSolver()
 {
-    if (host_flags_) cudaFreeHost(host_flags_);
+    if (host_stats_) cudaFreeHost(host_stats_);
 }
 
-bool CgSolver::solve_mass(const MeshDev &m, bool fp64_values, const double *b, int64_t ldb, double *y, int64_t ldy,
-                          int c, double tol, int max_iter, cudaStream_t st, int *iterations)
+void CgSolver::reset_stats(cudaStream_t st)
 {
-    enqueue_mass(m, fp64_values, b, ldb, y, ldy, c, tol, max_iter, st);
-    return finish(st, iterations);
+    BAEMM_CUDA(cudaMemsetAsync(stats_.reserve(2), 0, 2 * sizeof(int), st));
 }
 
-bool CgSolver::finish(cudaStream_t st, int *iterations)
+void CgSolver::read_stats(cudaStream_t st)
 {
-    BAEMM_CUDA(cudaStreamSynchronize(st));
-    if (iterations) *iterations = host_flags_[1];
-    // flags[0]: all converged (multi-block kernels) or columns not converged (cg_cluster_kernel)
-    return cluster_path_ ? host_flags_[0] == 0 : host_flags_[0] != 0;
+    if (!host_stats_) BAEMM_CUDA(cudaMallocHost(&host_stats_, 2 * sizeof(int)));
+    BAEMM_CUDA(cudaMemcpyAsync(host_stats_, stats_.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
 }
 
 void CgSolver::reserve_totals(int nblk, int S, cudaStream_t st)
@@ -943,21 +945,18 @@ void CgSolver::enqueue_mass(const MeshDev &m, bool fp64_values, const double *b,
     const int64_t n = m.nv;
     BAEMM_REQUIRE(c >= 1 && c <= kMaxKrylovColumns, BAEMM_ERR_SIZE, "CG column count out of range");
     const int64_t N = n * c;
-    flags_.reserve(2 + (size_t)c);
-    if (!host_flags_) BAEMM_CUDA(cudaMallocHost(&host_flags_, 2 * sizeof(int)));
-    cluster_path_ = n <= kMassEllMaxRows;
-    if (cluster_path_)
+    if (!stats_.p) reset_stats(st);
+    if (n <= kMassEllMaxRows)
     {
         // all iterations in one launch
-        BAEMM_CUDA(cudaMemsetAsync(flags_.p, 0, 2 * sizeof(int), st));
         if (fp64_values)
-            launch_cg_cluster<double>(st, m, c, b, ldb, m.mass_d, m.mass_ell_d, m.lumped_d, y, ldy, flags_.p, tol, max_iter);
+            launch_cg_cluster<double>(st, m, c, b, ldb, m.mass_d, m.mass_ell_d, m.lumped_d, y, ldy, stats_.p, tol, max_iter);
         else
-            launch_cg_cluster<float>(st, m, c, b, ldb, m.mass_f, m.mass_ell_f, m.lumped_f, y, ldy, flags_.p, tol, max_iter);
+            launch_cg_cluster<float>(st, m, c, b, ldb, m.mass_f, m.mass_ell_f, m.lumped_f, y, ldy, stats_.p, tol, max_iter);
         BAEMM_LAUNCH_CHECK();
-        BAEMM_CUDA(cudaMemcpyAsync(host_flags_, flags_.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
         return;
     }
+    flags_.reserve(2 + (size_t)c);
     x_.reserve(N); r_.reserve(N); z_.reserve(N); p_.reserve(N); q_.reserve(N);
     col_.reserve(4 * (size_t)c);
     const Layout L = make_layout(n, c);
@@ -982,7 +981,8 @@ void CgSolver::enqueue_mass(const MeshDev &m, bool fp64_values, const double *b,
     BAEMM_LAUNCH_CHECK();
     cg_output_kernel<<<eg(N), 256, 0, st>>>(n, c, x_.p, y, ldy);
     BAEMM_LAUNCH_CHECK();
-    BAEMM_CUDA(cudaMemcpyAsync(host_flags_, flags_.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    cg_stats_kernel<<<1, 1, 0, st>>>(flags_.p, stats_.p);
+    BAEMM_LAUNCH_CHECK();
 }
 
 double CgSolver::profile_block(const MeshDev &m, bool fp64_values, int c, int iterations, cudaStream_t st)
@@ -997,7 +997,7 @@ double CgSolver::profile_block(const MeshDev &m, bool fp64_values, int c, int it
     y.reserve(N);
     std::vector<double> ones((size_t)N, 1.0);
     BAEMM_CUDA(cudaMemcpyAsync(b.p, ones.data(), N * sizeof(double), cudaMemcpyHostToDevice, st));
-    flags_.reserve(2 + (size_t)c);
+    reset_stats(st);
     cudaEvent_t e0, e1;
     BAEMM_CUDA(cudaEventCreate(&e0));
     BAEMM_CUDA(cudaEventCreate(&e1));
@@ -1005,12 +1005,11 @@ double CgSolver::profile_block(const MeshDev &m, bool fp64_values, int c, int it
     // tol < 0: no column converges, every iteration does its work; a first launch warms up
     for (int rep = 0; rep < 2; ++rep)
     {
-        BAEMM_CUDA(cudaMemsetAsync(flags_.p, 0, 2 * sizeof(int), st));
         BAEMM_CUDA(cudaEventRecord(e0, st));
         if (fp64_values)
-            launch_cg_cluster<double>(st, m, c, b.p, c, m.mass_d, m.mass_ell_d, m.lumped_d, y.p, c, flags_.p, -1.0, iterations);
+            launch_cg_cluster<double>(st, m, c, b.p, c, m.mass_d, m.mass_ell_d, m.lumped_d, y.p, c, stats_.p, -1.0, iterations);
         else
-            launch_cg_cluster<float>(st, m, c, b.p, c, m.mass_f, m.mass_ell_f, m.lumped_f, y.p, c, flags_.p, -1.0, iterations);
+            launch_cg_cluster<float>(st, m, c, b.p, c, m.mass_f, m.mass_ell_f, m.lumped_f, y.p, c, stats_.p, -1.0, iterations);
         BAEMM_CUDA(cudaEventRecord(e1, st));
     }
     BAEMM_LAUNCH_CHECK();

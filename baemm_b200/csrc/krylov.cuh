@@ -28,17 +28,17 @@ class CgSolver
 {
 public:
     ~CgSolver();
-    // y = M^-1 b on c real columns (b: n x c with ld ldb, y with ld ldy).
-    // Returns true when every column converged; *iterations = iterations run.
-    bool solve_mass(const MeshDev &m, bool fp64_values, const double *b, int64_t ldb, double *y, int64_t ldy, int c,
-                    double tol, int max_iter, cudaStream_t st, int *iterations);
-    // The same in two parts: enqueue_mass only enqueues work on `st` (a fixed
-    // launch sequence plus a copy of the convergence flags to pinned host
-    // memory, so it can be captured in a CUDA graph); finish synchronises `st`
-    // and reads the flags.
+    // y = M^-1 b on c real columns (b: n x c with ld ldb, y with ld ldy).  Only
+    // enqueues work on `st`, a fixed launch sequence (it can be captured in a CUDA
+    // graph); convergence goes to the device's statistics.
     void enqueue_mass(const MeshDev &m, bool fp64_values, const double *b, int64_t ldb, double *y, int64_t ldy, int c,
                       double tol, int max_iter, cudaStream_t st);
-    bool finish(cudaStream_t st, int *iterations);
+    // Statistics over the solves since reset_stats.  read_stats enqueues their copy
+    // to the host; after the stream's next synchronisation the others hold.
+    void reset_stats(cudaStream_t st);
+    void read_stats(cudaStream_t st);
+    bool all_converged() const { return !host_stats_ || host_stats_[0] == 0; }
+    int most_iterations() const { return host_stats_ ? host_stats_[1] : 0; }
     // Device time of the CG iteration's kernels on the mesh's mass matrix:
     // `iterations` iterations on c real columns (right-hand side all ones,
     // no column allowed to converge), each launch bracketed by CUDA events.
@@ -55,10 +55,9 @@ private:
     // between kernels; zeroed whenever the buffer grows)
     void reserve_totals(int nblk, int S, cudaStream_t st);
     DevBuf<double> x_, r_, z_, p_, q_, col_, partial_;
-    DevBuf<int> flags_;
+    DevBuf<int> flags_, stats_;   // stats_: columns (multi-block kernels: solves) not converged, most iterations
     DevBuf<unsigned int> counter_;
-    int *host_flags_ = nullptr;
-    bool cluster_path_ = false;   // the last enqueue_mass ran cg_cluster_kernel (meshes of up to 16384 vertices)
+    int *host_stats_ = nullptr;
 };
 
 // Device time of one classical Gram-Schmidt pass of a GMRES iteration on an

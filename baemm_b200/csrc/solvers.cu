@@ -25,8 +25,7 @@ void Ctx::bie_solve(const double *kappa, const zc *coeff4, const double2 *rhs, d
     const int64_t nv = mesh.nv;
     load_parameters(kappa, coeff4, wc, wcs, 1.0);
     operators_loaded = true;
-    stats = baemm_solve_stats{};
-    stats.cg_converged = 1;
+    reset_stats();
     // With a packer the dense stage joins the packer's launches, which cannot
     // be captured in this context's graph: the apply then runs ungraphed.
     PackerSession session(packer);
