@@ -847,6 +847,257 @@ __global__ void givens_kernel(int c, int m, int j, S *__restrict__ H, double *__
     if (threadIdx.x == 0) flags[0] = all;
 }
 
+// One Arnoldi step of the complex GMRES in one launch: two Gram-Schmidt passes
+// of w against V_0 .. V_j, the norm, V_{j+1} = w / |w|, the Hessenberg column and
+// its Givens rotations.  The columns are independent, so a cluster of S blocks
+// owns two of them (their entries of a row are the 32 bytes of a sector) and its
+// blocks split the rows; w stays in shared memory and the sums go to every block
+// through distributed shared memory, in fixed orders.  flags[0] counts the columns
+// not converged (zero before the launch).
+//
+// Bound by the three cluster sums on small meshes, by the reads of V (four passes,
+// a warp's load touching 16 lines) on larger ones.  A step of a solve on 2562
+// vertices x 32 columns (8 vectors on average) takes 28 us; as ten kernels it took
+// 52 us and their launches.  On 10242 x 32 it takes 86 us, as kernels 88 and their
+// launches; above kArnMaxRows the ten kernels, whose loads cover whole lines, are
+// faster (40962 x 32: a solve of 737 ms took 751).
+constexpr int kArnThreads = 512, kArnWarps = kArnThreads / 32, kArnCluster = 8, kArnCols = 2;
+constexpr int kArnGroup = 8;   // vectors whose sums a thread holds in registers
+constexpr int kArnVecs = kMaxRestart + 1;
+constexpr int64_t kArnMaxRows = 16384;
+
+struct ArnSmem
+{
+    double red[kArnWarps][kArnGroup * 2 * kArnCols];        // a group's sums by warp: (vector, part, column)
+    double xch[2][kArnCluster][kArnVecs * 2 * kArnCols];    // every block's sums of a pass
+    double norm[kArnCluster][kArnCols], norm_red[kArnWarps][kArnCols];
+    double2 h[kArnVecs][kArnCols], col[kArnVecs][kArnCols]; // a pass's products; the Hessenberg column
+    double cs[kMaxRestart][kArnCols];
+    double2 sn[kMaxRestart][kArnCols];
+};
+
+__global__ void __launch_bounds__(kArnThreads, 1)
+arnoldi_kernel(int64_t n, int c, int rpc, int m, int j, const double2 *w_in, const double2 *V, double2 *Vnext,
+               double2 *__restrict__ H, double *__restrict__ cs, double2 *__restrict__ sn, double2 *__restrict__ g,
+               double *__restrict__ res, const double *__restrict__ bnorm, int *__restrict__ flags, double tol)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+    extern __shared__ __align__(16) uint8_t raw[];
+    ArnSmem &sm = *reinterpret_cast<ArnSmem *>(raw);
+    double2 *w = reinterpret_cast<double2 *>(raw + sizeof(ArnSmem));   // rows of this block x 2
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int col = tid & 1, k = (blockIdx.z / S) * kArnCols + col;
+    const bool live = k < c;
+    const int64_t r0 = (int64_t)rank * rpc, stride = n * c;
+    const int rows = (int)max((int64_t)0, min((int64_t)rpc, n - r0)), elems = rows * kArnCols;
+    const int nvec = j + 1;
+    const double2 zero = make_double2(0.0, 0.0);
+    // element e = row * 2 + column of this block, in the n x c blocks: at[e / 2 * c]
+    const double2 *vbase = V + r0 * c + k;
+    for (int e = tid; e < elems; e += kArnThreads) w[e] = live ? w_in[(r0 + e / 2) * c + k] : zero;
+    for (int i = tid; i < j * kArnCols; i += kArnThreads)
+    {
+        const int kk = (blockIdx.z / S) * kArnCols + (i & 1);
+        sm.cs[i >> 1][i & 1] = kk < c ? cs[(i >> 1) * c + kk] : 0.0;
+        sm.sn[i >> 1][i & 1] = kk < c ? sn[(i >> 1) * c + kk] : zero;
+    }
+    if (S > 1) cluster.sync();   // every block runs before its shared memory is written
+
+    // sm.h = V^H w over the cluster, through xch[pass]
+    auto products = [&](int pass) {
+        for (int g0 = 0; g0 < nvec; g0 += kArnGroup)
+        {
+            double v[2 * kArnGroup];   // (vector, part)
+            #pragma unroll
+            for (int i = 0; i < 2 * kArnGroup; ++i) v[i] = 0.0;
+            for (int e = tid; e < elems; e += kArnThreads)
+            {
+                const double2 wv = w[e];
+                const double2 *p = vbase + (int64_t)(e / 2) * c + g0 * stride;
+                double2 a[kArnGroup];
+                #pragma unroll
+                for (int i = 0; i < kArnGroup; ++i) a[i] = live && g0 + i < nvec ? __ldg(p + i * stride) : zero;
+                #pragma unroll
+                for (int i = 0; i < kArnGroup; ++i)
+                {
+                    v[2 * i] += a[i].x * wv.x + a[i].y * wv.y;
+                    v[2 * i + 1] += a[i].x * wv.y - a[i].y * wv.x;
+                }
+            }
+            // sums over the 16 lanes of a column: each step hands half of the values to
+            // the partner, so that lane l of them ends with the sum of value l
+            #pragma unroll
+            for (int o = 8; o > 0; o >>= 1)
+            {
+                const bool up = (lane >> 1) & o;
+                #pragma unroll
+                for (int i = 0; i < o; ++i)
+                {
+                    const double give = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * o);
+                }
+            }
+            sm.red[warp][(lane >> 1) * kArnCols + col] = v[0];
+            __syncthreads();
+            if (tid < 2 * kArnGroup * kArnCols)
+            {
+                double t = 0.0;
+                #pragma unroll
+                for (int q = 0; q < kArnWarps; ++q) t += sm.red[q][tid];
+                for (int s = 0; s < S; ++s)
+                    if (g0 * 2 * kArnCols + tid < kArnVecs * 2 * kArnCols)
+                        *cluster.map_shared_rank(&sm.xch[pass][rank][g0 * 2 * kArnCols + tid], s) = t;
+            }
+            __syncthreads();   // red is free again
+        }
+        if (S > 1) cluster.sync();
+        for (int i = tid; i < nvec * kArnCols; i += kArnThreads)
+        {
+            double2 t = zero;
+            for (int s = 0; s < S; ++s)
+            {
+                t.x += sm.xch[pass][s][(i >> 1) * 2 * kArnCols + (i & 1)];
+                t.y += sm.xch[pass][s][(i >> 1) * 2 * kArnCols + kArnCols + (i & 1)];
+            }
+            sm.h[i >> 1][i & 1] = t;
+            sm.col[i >> 1][i & 1] = pass == 0 ? t : Sadd(sm.col[i >> 1][i & 1], t);
+        }
+        __syncthreads();
+    };
+    double norm2 = 0.0;
+    // w -= V h; norm2 = |w|^2 over this thread's elements
+    auto subtract = [&]() {
+        norm2 = 0.0;
+        for (int e = tid; e < elems; e += kArnThreads)
+        {
+            double2 acc = w[e];
+            for (int g0 = 0; g0 < nvec; g0 += kArnGroup)
+            {
+                const double2 *p = vbase + (int64_t)(e / 2) * c + g0 * stride;
+                double2 a[kArnGroup];
+                #pragma unroll
+                for (int i = 0; i < kArnGroup; ++i) a[i] = live && g0 + i < nvec ? __ldg(p + i * stride) : zero;
+                #pragma unroll
+                for (int i = 0; i < kArnGroup; ++i)
+                    if (g0 + i < nvec) acc = Ssub(acc, Smul(sm.h[g0 + i][col], a[i]));
+            }
+            w[e] = acc;
+            norm2 += Sabs2(acc);
+        }
+    };
+    products(0);
+    subtract();
+    products(1);   // its reads of w are the thread's own
+    subtract();
+    #pragma unroll
+    for (int o = 16; o > 1; o >>= 1) norm2 += __shfl_xor_sync(0xffffffffu, norm2, o);
+    if (lane < kArnCols) sm.norm_red[warp][lane] = norm2;
+    __syncthreads();
+    if (tid < kArnCols)
+    {
+        double t = 0.0;
+        for (int q = 0; q < kArnWarps; ++q) t += sm.norm_red[q][tid];
+        for (int s = 0; s < S; ++s) *cluster.map_shared_rank(&sm.norm[rank][tid], s) = t;
+    }
+    if (S > 1) cluster.sync();
+    else __syncthreads();
+    double hn = 0.0;
+    for (int s = 0; s < S; ++s) hn += sm.norm[s][col];
+    hn = sqrt(hn);
+    const double inv = hn > 0.0 ? 1.0 / hn : 0.0;
+    for (int e = tid; e < elems; e += kArnThreads)
+        if (live) Vnext[(r0 + e / 2) * c + k] = Sscale(w[e], inv);
+    if (rank != 0 || tid >= kArnCols || !live) return;
+    // the column of the Hessenberg matrix, its rotations and the new residual (givens_kernel)
+    for (int i = 0; i < j; ++i)
+    {
+        const double cc = sm.cs[i][col];
+        const double2 s = sm.sn[i][col], h0 = sm.col[i][col], h1 = sm.col[i + 1][col];
+        sm.col[i][col] = Sadd(Sscale(h0, cc), Smul(s, h1));
+        sm.col[i + 1][col] = Sadd(Sscale(Smul(Sconj(s), h0), -1.0), Sscale(h1, cc));
+        H[((int64_t)i * m + j) * c + k] = sm.col[i][col];
+    }
+    double2 a = sm.col[j][col];
+    double cc;
+    double2 s;
+    const double aa = sqrt(Sabs2(a)), bb = hn;
+    if (aa == 0.0)
+    {
+        cc = 0.0;
+        s = make_double2(1.0, 0.0);
+        a = make_double2(hn, 0.0);
+    }
+    else
+    {
+        const double t = sqrt(aa * aa + bb * bb);
+        cc = aa / t;
+        const double2 ua = Sscale(a, 1.0 / aa);
+        s = Sscale(Smul(ua, make_double2(hn, 0.0)), 1.0 / t);
+        a = Sscale(ua, t);
+    }
+    H[((int64_t)j * m + j) * c + k] = a;
+    cs[j * c + k] = cc;
+    sn[j * c + k] = s;
+    const double2 gj = g[(int64_t)j * c + k];
+    g[(int64_t)j * c + k] = Sscale(gj, cc);
+    const double2 gn = Sscale(Smul(Sconj(s), gj), -1.0);
+    g[(int64_t)(j + 1) * c + k] = gn;
+    const double rn = sqrt(Sabs2(gn));
+    res[k] = rn;
+    if (!(rn <= tol * bnorm[k])) atomicAdd(&flags[0], 1);
+}
+
+struct ArnShape
+{
+    int S = 0, rpc = 0;   // blocks per cluster, rows per block; S = 0: too large
+    size_t bytes = 0;
+};
+
+// The most blocks per cluster that let all clusters run at once (of clusters of
+// 8, fewer fit the chip); more where w would not fit shared memory otherwise.
+ArnShape arnoldi_shape(int64_t n, int c, int sms)
+{
+    ArnShape h;
+    if (n > kArnMaxRows) return h;
+    const int clusters = ceil_div(c, kArnCols);
+    for (int S = 1; S <= kArnCluster; S *= 2)
+    {
+        const int rpc = ceil_div(n, S);
+        const size_t bytes = sizeof(ArnSmem) + (size_t)rpc * kArnCols * sizeof(double2);
+        if (bytes > 227 * 1024) continue;
+        if (h.S == 0 || (int64_t)clusters * S <= (S < 8 ? sms : sms * 3 / 4))
+        {
+            h.S = S;
+            h.rpc = rpc;
+            h.bytes = bytes;
+        }
+    }
+    return h;
+}
+
+void launch_arnoldi(const ArnShape &h, int64_t n, int c, int m, int j, const double2 *w, const double2 *V, double2 *Vnext,
+                    double2 *H, double *cs, double2 *sn, double2 *g, double *res, const double *bnorm, int *flags,
+                    double tol, cudaStream_t st)
+{
+    int dev = 0;
+    BAEMM_CUDA(cudaGetDevice(&dev));
+    static std::mutex mu;
+    static bool done[64] = {};
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (dev < 0 || dev >= 64 || !done[dev])
+        {
+            BAEMM_CUDA(cudaFuncSetAttribute(arnoldi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+            if (dev >= 0 && dev < 64) done[dev] = true;
+        }
+    }
+    launch_clustered(arnoldi_kernel, dim3(1, 1, ceil_div(c, kArnCols) * h.S), kArnThreads, h.bytes, st, h.S, n, c, h.rpc, m,
+                     j, w, V, Vnext, H, cs, sn, g, res, bnorm, flags, tol);
+    BAEMM_LAUNCH_CHECK();
+}
+
 template <class S>
 __global__ void backsolve_kernel(int c, int m, int jend, const S *__restrict__ H, const S *__restrict__ g,
                                  S *__restrict__ y)
@@ -1162,7 +1413,7 @@ typename GmresSolver<S>::Stats GmresSolver<S>::solve(int64_t n, int c, int resta
     y_.reserve((size_t)m * c);
     w_.reserve(N); tmp_.reserve(N); x_.reserve(N); b_.reserve(N);
     res_.reserve(c); bnorm_.reserve(c); hn_.reserve(c);
-    flags_.reserve(4);
+    flags_.reserve(m + 1);   // [0] converged; [1 + j] columns not converged after Arnoldi step j
     const Layout L = make_layout(n, c);
     constexpr int W = kWords<S>;
     partial_.reserve((size_t)L.nblk * (m + 1) * c * W);
@@ -1177,8 +1428,10 @@ typename GmresSolver<S>::Stats GmresSolver<S>::solve(int64_t n, int c, int resta
     const int fin = std::min(1024, ((c + 31) / 32) * 32);   // givens: one thread per column
     const int fin_w = std::min(1024, 32 * c);                // norm finalize: one warp per column
 
-    auto read_flag = [&]() {
-        BAEMM_CUDA(cudaMemcpyAsync(host_flags_, flags_.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    // complex blocks on small meshes: one launch per Arnoldi step
+    const ArnShape arn = std::is_same<S, double2>::value ? arnoldi_shape(n, c, tc_sm_count()) : ArnShape();
+    auto read_flag = [&](int at = 0) {
+        BAEMM_CUDA(cudaMemcpyAsync(host_flags_, flags_.p + at, sizeof(int), cudaMemcpyDeviceToHost, st));
         BAEMM_CUDA(cudaStreamSynchronize(st));
         return host_flags_[0] != 0;
     };
@@ -1213,11 +1466,22 @@ typename GmresSolver<S>::Stats GmresSolver<S>::solve(int64_t n, int c, int resta
         normalize_kernel<S><<<eg(N), 256, 0, st>>>(n, c, w_.p, hn_.p, V_.p);
         BAEMM_CUDA(cudaMemsetAsync(H_.p, 0, (size_t)(m + 1) * m * c * sizeof(S), st));
         int jend = 0;
+        if (arn.S > 0) BAEMM_CUDA(cudaMemsetAsync(flags_.p, 0, (m + 1) * sizeof(int), st));
         for (int j = 0; j < m; ++j)
         {
             S *Vj = V_.p + (int64_t)j * N;
             A(Vj, tmp_.p);
             P(tmp_.p, w_.p);
+            if constexpr (std::is_same<S, double2>::value)
+                if (arn.S > 0)
+                {
+                    launch_arnoldi(arn, n, c, m, j, w_.p, V_.p, Vj + N, H_.p, cs_.p, sn_.p, g_.p, res_.p, bnorm_.p,
+                                   flags_.p + 1 + j, tol, st);
+                    stats.iterations++;
+                    jend = j + 1;
+                    if (!read_flag(1 + j)) { conv = true; break; }
+                    continue;
+                }
             const int nvec = j + 1;
             const int fg = ceil_div((int64_t)nvec * c * 32, 256);   // one warp per item
             for (int pass = 0; pass < 2; ++pass)

@@ -211,3 +211,23 @@ def test_topology(name, mesh):
             O.Oracle(coords, tris, np.eye(3), precision=64).ApplyBoundaryOperators_PL(1.0, B, 0.0, ref, kap, coeff, 4, 4)
             used = np.unique(tris)
             assert relerr(got[used], ref[used]) < TOL64
+
+
+@pytest.mark.parametrize("grid", [(3, 3), (7, 73), (16, 32), (41, 125)])
+@pytest.mark.parametrize("chunks,directions", [(1, 1), (1, 2), (2, 16), (1, 64)])
+def test_one_launch_arnoldi(grid, chunks, directions):
+    """A solve to 1e-10 and its residual by the FP64 apply: 1 to 64 columns (half a
+    pair, one, many), rows that do and do not fill the blocks of a cluster.
+    The solve ends on |P r| <= 1e-10 |P b|; the residual itself is held to 1e-8
+    (the condition of the mass matrix, below 100 on these grids)."""
+    coords, tris = meshes.torus(n_minor=grid[0], n_major=grid[1])
+    kap = np.array([1.0, 2.0][:chunks])
+    wave = crandn(np.random.default_rng(5), coords.shape[0], chunks * directions)
+    phi, back = np.zeros_like(wave), np.zeros_like(wave)
+    coeff = np.zeros((chunks, 4), np.complex128)
+    with Helmholtz_CUDA(coords, tris, np.eye(3)) as H:
+        H.SetApplyMode(APPLY_FP64)
+        H.BoundaryPotential(kap, coeff, wave, phi, directions, 1e-12, 1e-10)
+        assert H.LastSolveStats()["gmres_converged"]
+        H.ApplyBoundaryOperators_PL(1.0, phi, 0.0, back, kap, coeff, wave.shape[1], directions)
+    assert relerr(back, wave) < 1e-8
