@@ -350,6 +350,7 @@ boundary_pair_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, con
                      const float2 *__restrict__ B, float2 *__restrict__ C, const ChunkParamsF *__restrict__ prm,
                      int n, int wc, int wcs, int per_split)
 {
+    chain_wait();
     __shared__ PairTile<COLS> tile;
     const int tid = threadIdx.x;
     const int col0 = blockIdx.y * COLS;
@@ -468,6 +469,7 @@ boundary_pair_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, con
             tile.tot[k][tid] = t;
         }
     }
+    chain_next();
     // with a cluster of S parts of the sources, block r adds columns r, r + S, ... of all of them in order
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -492,6 +494,7 @@ boundary_pair_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, con
 template <class R>
 __global__ void split_sum_kernel(const cplx<R> *__restrict__ partial, int splits, int64_t elems, cplx<R> *__restrict__ C)
 {
+    chain_begin();
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= elems) return;
     const cplx<R> *p = partial + e;
@@ -579,6 +582,7 @@ __global__ void __launch_bounds__(32 * kReduceRows)
 farfield_reduce_kernel(const cplx<R> *__restrict__ partial, int splits, int m, int wc, double2 alpha, double2 beta,
                        double2 *__restrict__ Cout, int64_t ldC)
 {
+    chain_begin();
     __shared__ double2 row[kReduceRows][32];
     const int64_t elems = (int64_t)m * wc, idx = (int64_t)blockIdx.x * 32 + threadIdx.x;
     double2 t = make_double2(0.0, 0.0);
@@ -725,6 +729,7 @@ __global__ void incident_kernel(int64_t nt, const R *__restrict__ mid4, const R 
 template <class R>
 __global__ void pack_points_kernel(int64_t m, const double *__restrict__ pts3, R *__restrict__ pts4)
 {
+    chain_begin();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
     pts4[4 * i + 0] = (R)pts3[3 * i + 0];
@@ -811,7 +816,7 @@ void pair_dispatch(int code, dim3 grid, int cluster, cudaStream_t st, DenseTarge
                    int per_part)
 {
 #define BAEMM_PR(SL, DL, ADL) \
-    launch_clustered(boundary_pair_kernel<COLS, SL, DL, ADL, RI>, grid, kTargets, 0, st, cluster, tg, mid, nrm, B, C, p, \
+    launch_chained(boundary_pair_kernel<COLS, SL, DL, ADL, RI>, grid, kTargets, 0, st, cluster, tg, mid, nrm, B, C, p, \
                      n, wc, wcs, per_part)
     BAEMM_BY_LAYERS(BAEMM_PR)
 #undef BAEMM_PR
@@ -898,7 +903,7 @@ void dense_dispatch(const MeshDev &m, const OpFlags &f, const void *chunk_params
     }
     if (split.blocks > 1)
     {
-        split_sum_kernel<R><<<ceil_div(elems, 256), 256, 0, st>>>(out, split.blocks, elems, Ctri);
+        launch_chained(split_sum_kernel<R>, ceil_div(elems, 256), 256, 0, st, 1, out, split.blocks, elems, Ctri);
         BAEMM_LAUNCH_CHECK();
     }
 }
@@ -963,7 +968,7 @@ template <class R>
 void launch_pack_points(int64_t m, const double *pts3, R *pts4, cudaStream_t st)
 {
     if (m == 0) return;
-    pack_points_kernel<R><<<ceil_div(m, 256), 256, 0, st>>>(m, pts3, pts4);
+    launch_chained(pack_points_kernel<R>, ceil_div(m, 256), 256, 0, st, 1, m, pts3, pts4);
     BAEMM_LAUNCH_CHECK();
 }
 
@@ -1013,8 +1018,8 @@ void launch_farfield(const MeshDev &m, const OpFlags &f, const void *chunk_param
         }
         BAEMM_LAUNCH_CHECK();
     }
-    farfield_reduce_kernel<R><<<ceil_div((int64_t)mm * wc, 32), dim3(32, kReduceRows), 0, st>>>(partial, split.blocks, mm,
-                                                                                             wc, alpha, beta, Cout, ldC);
+    launch_chained(farfield_reduce_kernel<R>, ceil_div((int64_t)mm * wc, 32), dim3(32, kReduceRows), 0, st, 1, partial,
+                   split.blocks, mm, wc, alpha, beta, Cout, ldC);
     BAEMM_LAUNCH_CHECK();
 }
 

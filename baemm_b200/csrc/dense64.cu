@@ -235,6 +235,7 @@ struct Smem
 template <class Entry, int E, int NT>
 __global__ void __launch_bounds__(kThreads, 2) d64_kernel(const Args a)
 {
+    chain_wait();
     extern __shared__ __align__(16) uint8_t raw[];
     Smem<E, NT> &sm = *reinterpret_cast<Smem<E, NT> *>(raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -370,6 +371,7 @@ __global__ void __launch_bounds__(kThreads, 2) d64_kernel(const Args a)
         }
     }
     flush();
+    chain_next();
     // accumulator v of tile q: row g + 8 (v / 2), column 8 q + 2 t + v % 2; with a cluster
     // of S parts, block r adds accumulators r, r + S, ... of all of them in order
     namespace cg = cooperative_groups;
@@ -411,7 +413,7 @@ void launch(const Args &a, dim3 grid, int cluster, cudaStream_t st)
             if (dev >= 0 && dev < 64) done[dev] = true;
         }
     }
-    launch_clustered(d64_kernel<Entry, E, NT>, grid, kThreads, bytes, st, cluster, a);
+    launch_chained(d64_kernel<Entry, E, NT>, grid, kThreads, bytes, st, cluster, a);
 }
 
 template <class Entry>

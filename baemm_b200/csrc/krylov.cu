@@ -468,6 +468,7 @@ cg_cluster_kernel(int64_t n, int rpc, int staged, const double *b, int64_t ldb, 
                   const RV *__restrict__ ell_val, const RV *__restrict__ L, double *y, int64_t ldy, int *stats,
                   double tol, int max_iter)
 {
+    chain_wait();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
@@ -475,7 +476,7 @@ cg_cluster_kernel(int64_t n, int rpc, int staged, const double *b, int64_t ldb, 
     __shared__ double xch[3][kCgCluster];   // every block's sums: <p, q>, <r, z>, <r, r>
     extern __shared__ __align__(16) uint8_t raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5, T = blockDim.x;
-    const int k = blockIdx.x / S;
+    const int k = blockIdx.z / S;
     const int r0 = rank * rpc, m = max(0, min(rpc, (int)n - r0));   // rows of this block
     double *p = reinterpret_cast<double *>(raw), *x = p + n, *r = x + rpc, *q = r + rpc;
     RV *sl = reinterpret_cast<RV *>(q + rpc);   // lumped inverse of the block's rows
@@ -591,6 +592,7 @@ cg_cluster_kernel(int64_t n, int rpc, int staged, const double *b, int64_t ldb, 
         if (S > 1) cluster.sync();   // p complete before the next iteration's gathers, and no write to a block that has left
         else __syncthreads();
     }
+    chain_next();
     for (int row = tid; row < m; row += T) y[(int64_t)(r0 + row) * ldy + k] = x[row];
     if (rank == 0 && tid == 0)
     {
@@ -625,20 +627,9 @@ void launch_cg_cluster(cudaStream_t st, const MeshDev &mesh, int c, const double
         }
     }
     const CgShape h = cg_cluster_shape<RV>(mesh.nv, c, tc_sm_count());
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(c * h.S);
-    cfg.blockDim = dim3(std::min(kCgThreads, ceil_div(h.rpc, 128) * 128));
-    cfg.dynamicSmemBytes = h.bytes;
-    cfg.stream = st;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = h.S;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    BAEMM_CUDA(cudaLaunchKernelEx(&cfg, cg_cluster_kernel<RV>, mesh.nv, h.rpc, h.staged, b, ldb,
-                                  (const int32_t *)mesh.mass_outer.p, (const int32_t *)mesh.mass_inner.p, mv,
-                                  (const uint16_t *)mesh.mass_ell_idx.p, ell_val, L, y, ldy, stats, tol, max_iter));
+    launch_chained(cg_cluster_kernel<RV>, dim3(1, 1, c * h.S), std::min(kCgThreads, ceil_div(h.rpc, 128) * 128), h.bytes, st,
+                   h.S, mesh.nv, h.rpc, h.staged, b, ldb, mesh.mass_outer.p, mesh.mass_inner.p, mv, mesh.mass_ell_idx.p,
+                   ell_val, L, y, ldy, stats, tol, max_iter);
 }
 
 __global__ void cg_output_kernel(int64_t n, int c, const double *__restrict__ x, double *__restrict__ y, int64_t ldy)
@@ -881,6 +872,7 @@ arnoldi_kernel(int64_t n, int c, int rpc, int m, int j, const double2 *w_in, con
                double2 *__restrict__ H, double *__restrict__ cs, double2 *__restrict__ sn, double2 *__restrict__ g,
                double *__restrict__ res, const double *__restrict__ bnorm, int *__restrict__ flags, double tol)
 {
+    chain_wait();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
@@ -1003,6 +995,7 @@ arnoldi_kernel(int64_t n, int c, int rpc, int m, int j, const double2 *w_in, con
     }
     if (S > 1) cluster.sync();
     else __syncthreads();
+    chain_next();
     double hn = 0.0;
     for (int s = 0; s < S; ++s) hn += sm.norm[s][col];
     hn = sqrt(hn);
@@ -1093,7 +1086,7 @@ void launch_arnoldi(const ArnShape &h, int64_t n, int c, int m, int j, const dou
             if (dev >= 0 && dev < 64) done[dev] = true;
         }
     }
-    launch_clustered(arnoldi_kernel, dim3(1, 1, ceil_div(c, kArnCols) * h.S), kArnThreads, h.bytes, st, h.S, n, c, h.rpc, m,
+    launch_chained(arnoldi_kernel, dim3(1, 1, ceil_div(c, kArnCols) * h.S), kArnThreads, h.bytes, st, h.S, n, c, h.rpc, m,
                      j, w, V, Vnext, H, cs, sn, g, res, bnorm, flags, tol);
     BAEMM_LAUNCH_CHECK();
 }

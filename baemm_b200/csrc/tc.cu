@@ -661,6 +661,7 @@ boundary_tc_kernel(const float *__restrict__ mid4, const float *__restrict__ nrm
     const int S = plan.seg_tiles;   // tiles per TMEM partial sum
     const int k_cta = blockIdx.x;
     volatile int *abort_flag = &sm.abort_flag;
+    chain_wait();
     // An earlier CTA gave up: do nothing.  Read once and shared, so the exit is
     // CTA-uniform and happens before any barrier init or TMEM allocation.
     if (tid == 0) sm.abort_flag = *(volatile int *)err;
@@ -1075,6 +1076,7 @@ boundary_tc_kernel(const float *__restrict__ mid4, const float *__restrict__ nrm
         }
     }
 
+    chain_next();
     tc_fence_before();
     __syncthreads();
     if (warp == 0)
@@ -1100,6 +1102,7 @@ boundary_tc_kernel(const float *__restrict__ mid4, const float *__restrict__ nrm
 __global__ void tc_expand_kernel(const float2 *__restrict__ Btri, int n, int wc, int64_t total, int share,
                                  uint8_t *__restrict__ img)
 {
+    chain_begin();
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= total) return;
     const int groups = wc / 16;
@@ -1156,7 +1159,7 @@ const uint8_t *launch_tc_expand(const float2 *Btri, int64_t n, int wc, DevBuf<ui
     const int64_t total = ntiles * groups * 128 * TC_HALVES;
     if (total > 0)
     {
-        tc_expand_kernel<<<ceil_div(total, 256), 256, 0, st>>>(Btri, (int)n, wc, total, share, out);
+        launch_chained(tc_expand_kernel, ceil_div(total, 256), 256, 0, st, 1, Btri, (int)n, wc, total, share, out);
         BAEMM_LAUNCH_CHECK();
     }
     return out;
@@ -1176,6 +1179,7 @@ constexpr int TC_FIX_THREADS = 256;
 __global__ void __launch_bounds__(TC_FIX_THREADS)
 tc_fixup_kernel(const float2 *__restrict__ ws, float2 *__restrict__ Ctri, const TcPlan plan, int cw)
 {
+    chain_begin();
     const int j = blockIdx.x;   // tail block
     const int b = plan.full_waves * plan.ctas + j;
     const int cg = b / plan.nblk, blk = b - cg * plan.nblk;
@@ -1235,8 +1239,8 @@ void tc_launch(cudaStream_t st, const float *mid, const float *nrm, const TcTile
             if (dev >= 0 && dev < 64) done[dev] = true;
         }
     }
-    boundary_tc_kernel<GW, CH, R, SL, DL, ADL, RI, KI, PACK><<<plan.ctas, tc_threads<GW, CH, R>(), bytes, st>>>(
-        mid, nrm, tg, B, C, ws, p, plan, err);
+    launch_chained(boundary_tc_kernel<GW, CH, R, SL, DL, ADL, RI, KI, PACK>, plan.ctas, tc_threads<GW, CH, R>(), bytes, st, 1,
+                   mid, nrm, tg, B, C, ws, p, plan, err);
 }
 
 template <int GW, int CH, bool RI>
@@ -1431,7 +1435,7 @@ void tc_run(const MeshDev &m, const OpFlags &f, const void *chunk_params, const 
     if (plan.tail_blocks > 0)
     {
         const dim3 grid(plan.tail_blocks, TC_M * CH * 16 / (2 * TC_FIX_THREADS));
-        tc_fixup_kernel<<<grid, TC_FIX_THREADS, 0, st>>>(ws, Ctri, plan, CH * 16);
+        launch_chained(tc_fixup_kernel, grid, TC_FIX_THREADS, 0, st, 1, ws, Ctri, plan, CH * 16);
         BAEMM_LAUNCH_CHECK();
     }
 }
