@@ -7,6 +7,7 @@
 #include <cstring>
 #include <stdexcept>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/baemm.h"
@@ -27,6 +28,24 @@ struct Error : std::runtime_error
             throw ::baemm::Error(BAEMM_ERR_CUDA, std::string(#call) + " failed: " +         \
                                                      cudaGetErrorString(e_));               \
     } while (0)
+
+// Waits for the stream, giving up the processor between tests: a solve waits once
+// per GMRES iteration, and threads that drive solves of their own (the serving
+// slots, packed solves) may share a core or the driver's lock with it.
+// (cudaStreamSynchronize spins: of two threads solving side by side, the second
+// could stand still until the first had finished.)
+inline void wait_stream(cudaStream_t st)
+{
+    for (;;)
+    {
+        const cudaError_t e = cudaStreamQuery(st);
+        if (e == cudaSuccess) return;
+        (void)cudaGetLastError();   // "not ready" is kept as the last error
+        if (e != cudaErrorNotReady)
+            throw Error(BAEMM_ERR_CUDA, std::string("waiting for the stream failed: ") + cudaGetErrorString(e));
+        std::this_thread::yield();
+    }
+}
 
 // Process-wide count of kernel launches (reported by baemm_kernel_launch_count).
 extern std::atomic<long long> g_kernel_launches;

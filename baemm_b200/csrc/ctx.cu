@@ -194,7 +194,7 @@ void Ctx::switch_stream(cudaStream_t s)
 void Ctx::sync()
 {
     if (cg_pending) cg.read_stats(stream);
-    BAEMM_CUDA(cudaStreamSynchronize(stream));
+    wait_stream(stream);
     if (cg_pending)
     {
         cg_pending = false;
@@ -209,7 +209,7 @@ void Ctx::check_tc_error()
 {
     tc_pending = false;
     BAEMM_CUDA(cudaMemcpyAsync(tc_err_host, tc_err.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
-    BAEMM_CUDA(cudaStreamSynchronize(stream));
+    wait_stream(stream);
     if (*tc_err_host != 0)
     {
         const int code = *tc_err_host;

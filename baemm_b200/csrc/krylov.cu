@@ -1425,7 +1425,7 @@ typename GmresSolver<S>::Stats GmresSolver<S>::solve(int64_t n, int c, int resta
     const ArnShape arn = std::is_same<S, double2>::value ? arnoldi_shape(n, c, tc_sm_count()) : ArnShape();
     auto read_flag = [&](int at = 0) {
         BAEMM_CUDA(cudaMemcpyAsync(host_flags_, flags_.p + at, sizeof(int), cudaMemcpyDeviceToHost, st));
-        BAEMM_CUDA(cudaStreamSynchronize(st));
+        wait_stream(st);
         return host_flags_[0] != 0;
     };
     // hn = ||w|| columnwise, with `mode` as in norm_finalize_kernel
@@ -1501,7 +1501,7 @@ typename GmresSolver<S>::Stats GmresSolver<S>::solve(int64_t n, int c, int resta
     BAEMM_LAUNCH_CHECK();
     BAEMM_CUDA(cudaMemcpyAsync(host_res_, res_.p, c * sizeof(double), cudaMemcpyDeviceToHost, st));
     BAEMM_CUDA(cudaMemcpyAsync(host_res_ + c, bnorm_.p, c * sizeof(double), cudaMemcpyDeviceToHost, st));
-    BAEMM_CUDA(cudaStreamSynchronize(st));
+    wait_stream(st);
     stats.converged = conv;
     stats.max_rel_res = 0.0;
     for (int k = 0; k < c; ++k)
@@ -1535,7 +1535,7 @@ double device_dot(const double *a, const double *b, int64_t n, DevBuf<double> &p
     dot_partial_kernel<<<nb, RT, 0, st>>>(a, b, n, partial.reserve(nb));
     BAEMM_LAUNCH_CHECK();
     BAEMM_CUDA(cudaMemcpyAsync(h.data(), partial.p, nb * sizeof(double), cudaMemcpyDeviceToHost, st));
-    BAEMM_CUDA(cudaStreamSynchronize(st));
+    wait_stream(st);
     double s = 0.0;
     for (double v : h) s += v;
     return s;
@@ -1551,7 +1551,7 @@ void device_colnorms(const double2 *w, int64_t n, int c, double *out_host, DevBu
     BAEMM_LAUNCH_CHECK();
     std::vector<double> h((size_t)L.nblk * c);
     BAEMM_CUDA(cudaMemcpyAsync(h.data(), partial.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    BAEMM_CUDA(cudaStreamSynchronize(st));
+    wait_stream(st);
     for (int k = 0; k < c; ++k)
     {
         double s = 0.0;

@@ -205,7 +205,7 @@ int64_t launch_topology(MeshDev &m, DevBuf<int32_t> &scratch, int32_t *host2, cu
     scan(nv + 1, rows, m.mass_outer, total, nullptr, st);
     BAEMM_CUDA(cudaMemcpyAsync(&host2[0], most, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     BAEMM_CUDA(cudaMemcpyAsync(&host2[1], m.mass_outer + nv, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    BAEMM_CUDA(cudaStreamSynchronize(st));
+    wait_stream(st);
     if (host2[0] > kTopologyDegree) return -1;
     m.mass_inner.reserve(std::max(host2[1], 1));
     pack_kernel<<<ceil_div(nv, T), T, 0, st>>>(nv, m.avt_outer, slots, m.mass_outer, m.mass_inner);
