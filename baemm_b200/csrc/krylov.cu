@@ -418,12 +418,16 @@ __global__ void cg_pupdate_kernel(int64_t total, int c, const double *__restrict
 // stream from L2 where it does not fit.  One block per column, the CSR rows read
 // one thread per row (uncoalesced) and the vectors in global memory, took 28.4 us
 // per iteration on 10242 vertices x 64 columns and 9.2 us on 2562 x 64.
-// Now, per iteration of a solve's 20: 3.1 us on 642 x 64, 5.2 on 2562 x 64 (two
-// blocks a column), 14.6 on 10242 x 64 (two blocks a column, matrix from L2).
-// 512 threads: the block sums shuffle every warp's doubles through one shuffle
-// unit (1024 threads took 5.95 instead of 5.1 us per iteration on 2562 x 64);
-// the matrix rows in registers made no difference.
-constexpr int kCgThreads = 512, kCgCluster = 8;
+// Now, per iteration of a solve's 20: 2.8 us on 642 x 64, 4.9 on 2562 x 64 (two
+// blocks a column), 13.7 on 10242 x 64 (two blocks a column, matrix from L2).
+// With the matrix in shared memory a block has at most 512 threads and four rows
+// per thread in flight: the block sums shuffle every warp's doubles through one
+// shuffle unit (1024 threads took 5.95 instead of 5.1 us per iteration on 2562 x
+// 64); the matrix rows in registers made no difference.  With the matrix from L2
+// more warps hide its latency: 736 threads of two rows 13.7 us on 10242 x 64, 512
+// threads of two rows 14.7, of four rows 14.5.  cg_threads() takes as few threads
+// as the passes over the rows need: 1281 rows on 448 threads 5.0 us, on 512 5.1.
+constexpr int kCgThreads = 512, kCgThreadsL2 = 736, kCgCluster = 8;
 constexpr size_t kCgSmemBytes = 226 * 1024;   // of 227 KB, beside the static arrays
 
 struct CgShape
@@ -461,8 +465,15 @@ CgShape cg_cluster_shape(int64_t n, int c, int sms)
     return best;
 }
 
-template <class RV>
-__global__ void __launch_bounds__(kCgThreads, 1)
+int cg_threads(const CgShape &h)
+{
+    const int passes = ceil_div(h.rpc, h.staged == 2 ? kCgThreads : kCgThreadsL2);
+    return std::max(64, ceil_div(ceil_div(h.rpc, passes), 32) * 32);   // a warp for each of two block sums
+}
+
+// STAGED: the matrix rows are in shared memory
+template <class RV, bool STAGED>
+__global__ void __launch_bounds__(STAGED ? kCgThreads : kCgThreadsL2, 1)
 cg_cluster_kernel(int64_t n, int rpc, int staged, const double *b, int64_t ldb, const int32_t *__restrict__ mo,
                   const int32_t *__restrict__ mi, const RV *__restrict__ mv, const uint16_t *__restrict__ ell_idx,
                   const RV *__restrict__ ell_val, const RV *__restrict__ L, double *y, int64_t ldy, int *stats,
@@ -472,7 +483,7 @@ cg_cluster_kernel(int64_t n, int rpc, int staged, const double *b, int64_t ldb, 
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
-    __shared__ double red[2][kCgThreads / 32];
+    __shared__ double red[2][32];
     __shared__ double xch[3][kCgCluster];   // every block's sums: <p, q>, <r, z>, <r, r>
     extern __shared__ __align__(16) uint8_t raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5, T = blockDim.x;
@@ -490,7 +501,7 @@ cg_cluster_kernel(int64_t n, int rpc, int staged, const double *b, int64_t ldb, 
         longer |= mo[r0 + row + 1] - mo[r0 + row] > kMassEll;
     }
     longer = __syncthreads_or(longer);
-    if (staged == 2)
+    if (STAGED)
         for (int e = tid; e < m * kMassEll; e += T)
         {
             const int j = e / m, row = e - j * m;
@@ -556,7 +567,7 @@ cg_cluster_kernel(int64_t n, int rpc, int staged, const double *b, int64_t ldb, 
     {
         v[0] = 0.0;
         auto matvec = [&](const RV *val, const uint16_t *idx, int64_t stride) {
-            #pragma unroll 2
+            #pragma unroll (STAGED ? 4 : 2)
             for (int row = tid; row < m; row += T)
             {
                 double s = 0.0;
@@ -568,7 +579,7 @@ cg_cluster_kernel(int64_t n, int rpc, int staged, const double *b, int64_t ldb, 
                 v[0] += p[r0 + row] * s;
             }
         };
-        if (staged == 2) matvec(sv, si, rpc);
+        if (STAGED) matvec(sv, si, rpc);
         else matvec(ell_val + r0, ell_idx + r0, n);
         totals(one, 0, v);
         const double alpha = v[0] == 0.0 ? 0.0 : rz / v[0];
@@ -608,9 +619,10 @@ __global__ void cg_stats_kernel(const int *__restrict__ flags, int *__restrict__
     atomicMax(&stats[1], flags[1]);
 }
 
-template <class RV>
-void launch_cg_cluster(cudaStream_t st, const MeshDev &mesh, int c, const double *b, int64_t ldb, const RV *mv,
-                       const RV *ell_val, const RV *L, double *y, int64_t ldy, int *stats, double tol, int max_iter)
+template <class RV, bool STAGED>
+void launch_cg_shape(cudaStream_t st, const CgShape &h, const MeshDev &mesh, int c, const double *b, int64_t ldb,
+                     const RV *mv, const RV *ell_val, const RV *L, double *y, int64_t ldy, int *stats, double tol,
+                     int max_iter)
 {
     // the limit above 48 KB is a per-device attribute of each instantiation, set once
     int dev = 0;
@@ -621,15 +633,23 @@ void launch_cg_cluster(cudaStream_t st, const MeshDev &mesh, int c, const double
         std::lock_guard<std::mutex> lock(mu);
         if (dev < 0 || dev >= 64 || !done[dev])
         {
-            BAEMM_CUDA(cudaFuncSetAttribute(cg_cluster_kernel<RV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            BAEMM_CUDA(cudaFuncSetAttribute(cg_cluster_kernel<RV, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)kCgSmemBytes));
             if (dev >= 0 && dev < 64) done[dev] = true;
         }
     }
+    launch_chained(cg_cluster_kernel<RV, STAGED>, dim3(1, 1, c * h.S), cg_threads(h), h.bytes, st, h.S, mesh.nv, h.rpc,
+                   h.staged, b, ldb, mesh.mass_outer.p, mesh.mass_inner.p, mv, mesh.mass_ell_idx.p, ell_val, L, y, ldy,
+                   stats, tol, max_iter);
+}
+
+template <class RV>
+void launch_cg_cluster(cudaStream_t st, const MeshDev &mesh, int c, const double *b, int64_t ldb, const RV *mv,
+                       const RV *ell_val, const RV *L, double *y, int64_t ldy, int *stats, double tol, int max_iter)
+{
     const CgShape h = cg_cluster_shape<RV>(mesh.nv, c, tc_sm_count());
-    launch_chained(cg_cluster_kernel<RV>, dim3(1, 1, c * h.S), std::min(kCgThreads, ceil_div(h.rpc, 128) * 128), h.bytes, st,
-                   h.S, mesh.nv, h.rpc, h.staged, b, ldb, mesh.mass_outer.p, mesh.mass_inner.p, mv, mesh.mass_ell_idx.p,
-                   ell_val, L, y, ldy, stats, tol, max_iter);
+    if (h.staged == 2) launch_cg_shape<RV, true>(st, h, mesh, c, b, ldb, mv, ell_val, L, y, ldy, stats, tol, max_iter);
+    else launch_cg_shape<RV, false>(st, h, mesh, c, b, ldb, mv, ell_val, L, y, ldy, stats, tol, max_iter);
 }
 
 __global__ void cg_output_kernel(int64_t n, int c, const double *__restrict__ x, double *__restrict__ y, int64_t ldy)
