@@ -823,14 +823,18 @@ void pair_dispatch(int code, dim3 grid, int cluster, cudaStream_t st, DenseTarge
 }
 
 // Room for the partial blocks of a split; with less, fewer of them (one: none).
+// A stream under capture grows nothing: an allocation would end its capture.
 template <class R>
-cplx<R> *partial_blocks(SplitSpace<R> ws, int64_t elems, SourceSplit &split)
+cplx<R> *partial_blocks(SplitSpace<R> ws, int64_t elems, SourceSplit &split, cudaStream_t st)
 {
     if (split.blocks == 1) return nullptr;
-    if (!ws.grow)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (ws.grow && ws.grow->n < (size_t)split.blocks * elems) BAEMM_CUDA(cudaStreamIsCapturing(st, &capture));
+    if (!ws.grow || capture != cudaStreamCaptureStatusNone)
     {
-        split.blocks = (int)std::max<size_t>(1, std::min<size_t>(split.blocks, ws.elems / elems));
-        return ws.fixed;
+        const size_t room = ws.grow ? ws.grow->n : ws.elems;
+        split.blocks = (int)std::max<size_t>(1, std::min<size_t>(split.blocks, room / elems));
+        return ws.grow ? ws.grow->p : ws.fixed;
     }
     try
     {
@@ -863,7 +867,7 @@ void dense_dispatch(const MeshDev &m, const OpFlags &f, const void *chunk_params
     if constexpr (std::is_same<R, double>::value)
     {
         split = dense_split(d64_ctas(d64_unit(wc, wcs), tg.m, wc), n, tc_sm_count());
-        out = partial_blocks<R>(ws, elems, split);
+        out = partial_blocks<R>(ws, elems, split, st);
         launch_boundary_d64(m, f, p, wc, wcs, tg, Btri, split.blocks > 1 ? out : Ctri, split, st);
     }
     else
@@ -883,7 +887,7 @@ void dense_dispatch(const MeshDev &m, const OpFlags &f, const void *chunk_params
         {
             dim3 pairs(ceil_div(tg.m, 2 * kTargets), wc / cols);
             split = dense_split((int64_t)pairs.x * pairs.y, n, tc_sm_count());
-            out = partial_blocks<R>(ws, elems, split);
+            out = partial_blocks<R>(ws, elems, split, st);
             pairs.z = split.parts();
             const int per_part = ceil_div(n, split.parts());
             cplx<R> *dst = split.blocks > 1 ? out : Ctri;

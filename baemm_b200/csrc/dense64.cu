@@ -32,7 +32,7 @@
 // Measured: 22.1 ms on 41666 triangles x 32 columns (two wavenumbers, SL + DL;
 // 3.47e9 entries at 40 FP64 instructions and 48 matrix multiply-adds: 75 % of
 // the pipe), 41.6 ms before; far field of 81920 triangles in 256 directions x
-// 32 columns 285 us, 437 before; 1280 x 32 46 us, 446 before (unsplit).  Three
+// 32 columns 285 us, 437 before; 1280 x 32 41 us, 446 before (unsplit).  Three
 // blocks per SM (168 registers) took 24.0 ms, one wavenumber per unit 26.6 ms
 // at 2 to 4 blocks; staging element by element instead of in register order
 // cost 4 ms in bank conflicts.

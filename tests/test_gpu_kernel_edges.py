@@ -231,3 +231,39 @@ def test_one_launch_arnoldi(grid, chunks, directions):
         assert H.LastSolveStats()["gmres_converged"]
         H.ApplyBoundaryOperators_PL(1.0, phi, 0.0, back, kap, coeff, wave.shape[1], directions)
     assert relerr(back, wave) < 1e-8
+
+
+@pytest.mark.parametrize("mode,tol", [(APPLY_FP32, TOL32), (APPLY_FP64, TOL64)])
+def test_split_launch_under_capture(mode, tol):
+    """A caller captures an apply of 16 columns in a context that has only run 256:
+    the narrow launch is split over the sources, the wide one was not, and under
+    capture the partial blocks have to make do with the room there is."""
+    import torch
+    coords, tris = meshes.torus(n_minor=32, n_major=80)
+    s = torch.cuda.Stream()
+    B = torch.as_tensor(crandn(np.random.default_rng(3), coords.shape[0], 256)).cuda()
+    C, narrow = torch.zeros_like(B), B[:, :16].contiguous()
+    Cn, again = torch.zeros_like(narrow), torch.zeros_like(narrow)
+    coeff = lambda ks: np.array([COEFF["bie"](k) for k in ks], np.complex128)
+    with Helmholtz_CUDA(coords, tris, np.eye(3)) as H:
+        H.SetApplyMode(mode)
+        H.SetStream(s.cuda_stream)
+        torch.cuda.synchronize()
+        wide = np.linspace(1.0, 6.0, 16)
+        H.ApplyBoundaryOperators_PL(1.0, B, 0.0, C, wide, coeff(wide), 256, 16)
+        H.LoadBoundaryOperators_PL(np.array([2.0]), coeff([2.0]), 16, 16)
+        H.Synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            H.ApplyBoundaryOperators_PL(1.0, narrow, 0.0, Cn)
+        g.replay()
+        H.ApplyBoundaryOperators_PL(1.0, narrow, 0.0, again)
+        torch.cuda.synchronize()
+        H.UnloadBoundaryOperators_PL()
+        H.SetStream(None)
+        del g
+    ref = np.zeros((coords.shape[0], 16), np.complex128)
+    O.Oracle(coords, tris, np.eye(3), precision=64).ApplyBoundaryOperators_PL(
+        1.0, narrow.cpu().numpy(), 0.0, ref, np.array([2.0]), coeff([2.0]), 16, 16)
+    assert relerr(Cn.cpu().numpy(), ref) < tol
+    assert relerr(again.cpu().numpy(), ref) < tol
