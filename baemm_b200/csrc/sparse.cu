@@ -26,7 +26,6 @@ __device__ __forceinline__ double2 dmul(double2 a, double2 b) { return make_doub
 // 2-D grid: threadIdx.x / blockIdx.y run over the columns (a warp reads 32
 // consecutive columns of a row), threadIdx.y / blockIdx.x over the rows.
 constexpr int kRowsPerBlock = 8;
-constexpr int kAhead = 3;   // row entries whose loads are in flight together (8 took 30 instead of 23 us on 10242 x 64: too few warps)
 
 template <class Text, class R>
 __global__ void __launch_bounds__(32 * kRowsPerBlock)
@@ -57,7 +56,15 @@ template <class R> struct PrmOf;
 template <> struct PrmOf<float> { using type = ChunkParamsF; };
 template <> struct PrmOf<double> { using type = ChunkParamsD; };
 
-template <class Text, class R>
+// AHEAD row entries have their loads in flight together: 3 where the launch does
+// not fill the chip and the chain of dependent loads is what it waits for, 1 (the
+// row one entry at a time, fewer registers and more warps) where it does.
+// Measured (us, 3 and 1 ahead): 160 vertices x 16 columns 7.8 and 8.7, 2560 x 32 8.6
+// and 9.4, 7040 x 32 10.8 and 10.9, 10240 x 64 24.2 and 22.3, 76800 x 64 154 and
+// 128 (8 ahead took 30 on 10242 x 64).
+constexpr int kFewAhead = 3;
+
+template <class Text, class R, int AHEAD>
 __global__ void __launch_bounds__(32 * kRowsPerBlock)
 epilogue_kernel(int64_t nv, int wc, int wcs, bool layers, bool sl_diag, bool mass,
                                 const int32_t *__restrict__ avt_outer, const int32_t *__restrict__ avt_inner,
@@ -84,49 +91,67 @@ epilogue_kernel(int64_t nv, int wc, int wcs, bool layers, bool sl_diag, bool mas
             ik.x = R(0);
             ik.y = prm[ch].kappa;
         }
-        // kAhead triangles at a time: their indices, then all that depends on them, in
-        // flight together (a vertex has about 6); the sum runs in row order
+        // the sum runs in row order (a vertex has about 6 triangles)
         double2 s = make_double2(0.0, 0.0);
-        for (int32_t e0 = avt_outer[v], e1 = avt_outer[v + 1]; e0 < e1; e0 += kAhead)
-        {
-            int64_t t[kAhead];
-            cplx<R> ct[kAhead], bt[kAhead];
-            R a[kAhead], d[kAhead];
-            #pragma unroll
-            for (int j = 0; j < kAhead; ++j)
+        if constexpr (AHEAD == 1)
+            for (int32_t e = avt_outer[v]; e < avt_outer[v + 1]; ++e)
             {
-                t[j] = e0 + j < e1 ? avt_inner[e0 + j] : -1;
-                if (t[j] < t_begin || t[j] >= t_end) t[j] = -1;   // past the row, or in another shard
-            }
-            #pragma unroll
-            for (int j = 0; j < kAhead; ++j)
-            {
-                ct[j].x = ct[j].y = bt[j].x = bt[j].y = a[j] = d[j] = R(0);
-                if (t[j] < 0) continue;
-                ct[j] = Ctri[t[j] * wc + k];
-                a[j] = a3[t[j]];
-                if (sl_diag)
-                {
-                    bt[j] = Btri[t[j] * wc + k];
-                    d[j] = diag[t[j]];
-                }
-            }
-            #pragma unroll
-            for (int j = 0; j < kAhead; ++j)
-            {
-                if (t[j] < 0) continue;
+                const int64_t t = avt_inner[e];
+                if (t < t_begin || t >= t_end) continue;   // in another shard
+                cplx<R> ct = Ctri[t * wc + k];
                 if (sl_diag)
                 {
                     // C[i,k] += c1 (diag_i + i kappa) B[i,k]   (ApplySingleLayerDiagonal.hpp:427-433)
                     cplx<R> f = ik;
-                    f.x += d[j];
+                    f.x += diag[t];
                     f = cmul(c1, f);
-                    cfma(ct[j], f, bt[j]);
+                    cfma(ct, f, Btri[t * wc + k]);
                 }
-                s.x += (double)a[j] * (double)ct[j].x;
-                s.y += (double)a[j] * (double)ct[j].y;
+                const double a = (double)a3[t];
+                s.x += a * (double)ct.x;
+                s.y += a * (double)ct.y;
             }
-        }
+        else
+            for (int32_t e0 = avt_outer[v], e1 = avt_outer[v + 1]; e0 < e1; e0 += AHEAD)
+            {
+                int64_t t[AHEAD];
+                cplx<R> ct[AHEAD], bt[AHEAD];
+                R a[AHEAD], d[AHEAD];
+                #pragma unroll
+                for (int j = 0; j < AHEAD; ++j)
+                {
+                    t[j] = e0 + j < e1 ? avt_inner[e0 + j] : -1;
+                    if (t[j] < t_begin || t[j] >= t_end) t[j] = -1;   // past the row, or in another shard
+                }
+                #pragma unroll
+                for (int j = 0; j < AHEAD; ++j)
+                {
+                    ct[j].x = ct[j].y = bt[j].x = bt[j].y = a[j] = d[j] = R(0);
+                    if (t[j] < 0) continue;
+                    ct[j] = Ctri[t[j] * wc + k];
+                    a[j] = a3[t[j]];
+                    if (sl_diag)
+                    {
+                        bt[j] = Btri[t[j] * wc + k];
+                        d[j] = diag[t[j]];
+                    }
+                }
+                #pragma unroll
+                for (int j = 0; j < AHEAD; ++j)
+                {
+                    if (t[j] < 0) continue;
+                    if (sl_diag)
+                    {
+                        // C[i,k] += c1 (diag_i + i kappa) B[i,k]   (ApplySingleLayerDiagonal.hpp:427-433)
+                        cplx<R> f = ik;
+                        f.x += d[j];
+                        f = cmul(c1, f);
+                        cfma(ct[j], f, bt[j]);
+                    }
+                    s.x += (double)a[j] * (double)ct[j].x;
+                    s.y += (double)a[j] * (double)ct[j].y;
+                }
+            }
         out = dmul(alpha, s);
     }
     if (mass)
@@ -135,28 +160,37 @@ epilogue_kernel(int64_t nv, int wc, int wcs, bool layers, bool sl_diag, bool mas
         const cplx<R> c0 = prm[ch].c[0];
         const double2 f = dmul(alpha, make_double2((double)c0.x, (double)c0.y));
         double2 s = make_double2(0.0, 0.0);
-        for (int32_t e0 = m_outer[v], e1 = m_outer[v + 1]; e0 < e1; e0 += kAhead)
-        {
-            int32_t i[kAhead];
-            R mv[kAhead];
-            double2 x[kAhead];
-            #pragma unroll
-            for (int j = 0; j < kAhead; ++j)
+        if constexpr (AHEAD == 1)
+            for (int32_t e = m_outer[v]; e < m_outer[v + 1]; ++e)
             {
-                i[j] = e0 + j < e1 ? m_inner[e0 + j] : -1;
-                mv[j] = e0 + j < e1 ? m_val[e0 + j] : R(0);
+                const double mv = (double)m_val[e];
+                const double2 b = ld2<Text>(&Bin[(int64_t)m_inner[e] * ldB + k]);
+                s.x += mv * b.x;
+                s.y += mv * b.y;
             }
-            #pragma unroll
-            for (int j = 0; j < kAhead; ++j)
-                x[j] = i[j] >= 0 ? ld2<Text>(&Bin[(int64_t)i[j] * ldB + k]) : make_double2(0.0, 0.0);
-            #pragma unroll
-            for (int j = 0; j < kAhead; ++j)
+        else
+            for (int32_t e0 = m_outer[v], e1 = m_outer[v + 1]; e0 < e1; e0 += AHEAD)
             {
-                if (i[j] < 0) continue;
-                s.x += (double)mv[j] * x[j].x;
-                s.y += (double)mv[j] * x[j].y;
+                int32_t i[AHEAD];
+                R mv[AHEAD];
+                double2 x[AHEAD];
+                #pragma unroll
+                for (int j = 0; j < AHEAD; ++j)
+                {
+                    i[j] = e0 + j < e1 ? m_inner[e0 + j] : -1;
+                    mv[j] = e0 + j < e1 ? m_val[e0 + j] : R(0);
+                }
+                #pragma unroll
+                for (int j = 0; j < AHEAD; ++j)
+                    x[j] = i[j] >= 0 ? ld2<Text>(&Bin[(int64_t)i[j] * ldB + k]) : make_double2(0.0, 0.0);
+                #pragma unroll
+                for (int j = 0; j < AHEAD; ++j)
+                {
+                    if (i[j] < 0) continue;
+                    s.x += (double)mv[j] * x[j].x;
+                    s.y += (double)mv[j] * x[j].y;
+                }
             }
-        }
         const double2 t = dmul(f, s);
         out.x += t.x;
         out.y += t.y;
@@ -370,11 +404,13 @@ void launch_epilogue(const MeshDev &m, const EpilogueArgs &a, const cplx<R> *Ctr
     const double2 al = make_double2((double)alpha.x, (double)alpha.y);
     const double2 be = make_double2((double)beta.x, (double)beta.y);
     const dim3 grid(ceil_div(m.nv, kRowsPerBlock), ceil_div(a.wc, 32)), block(32, kRowsPerBlock);
-    launch_chained(
-        epilogue_kernel<Text, R>, grid, block, 0, st, 1, m.nv, a.wc, a.wcs, a.layers, a.sl_diag, a.mass, m.avt_outer.p,
-        m.avt_inner.p, a3, diag, Ctri, Btri, static_cast<const typename PrmOf<R>::type *>(chunk_params), m.mass_outer.p,
-        m.mass_inner.p, mv, Bin, ldB, al, be,
-        Cout, ldC, a.t_begin, a.t_end);
+    const int64_t warps = (int64_t)grid.x * grid.y * kRowsPerBlock;
+    // three quarters of the warps the chip holds at once
+    const bool few = warps <= (int64_t)48 * tc_sm_count();
+    launch_chained(few ? epilogue_kernel<Text, R, kFewAhead> : epilogue_kernel<Text, R, 1>, grid, block, 0, st, 1, m.nv,
+                   a.wc, a.wcs, a.layers, a.sl_diag, a.mass, m.avt_outer.p, m.avt_inner.p, a3, diag, Ctri, Btri,
+                   static_cast<const typename PrmOf<R>::type *>(chunk_params), m.mass_outer.p, m.mass_inner.p, mv, Bin,
+                   ldB, al, be, Cout, ldC, a.t_begin, a.t_end);
     BAEMM_LAUNCH_CHECK();
 }
 

@@ -233,6 +233,15 @@ def test_one_launch_arnoldi(grid, chunks, directions):
     assert relerr(back, wave) < 1e-8
 
 
+@pytest.mark.parametrize("wc", [16, 416, 448])
+@pytest.mark.parametrize("mode,tol", [(APPLY_FP32, TOL32), (APPLY_FP64, TOL64)])
+def test_averaging_of_few_and_many_rows(mode, tol, wc):
+    """512 vertices in launches of 512, 6656 and 7168 warps: below and above three
+    quarters of what the chip holds, where the row loops of the epilogue change."""
+    got, ref = _apply(mode, (16, 32), wc, 16, "all")
+    assert relerr(got, ref) < tol
+
+
 @pytest.mark.parametrize("mode,tol", [(APPLY_FP32, TOL32), (APPLY_FP64, TOL64)])
 def test_split_launch_under_capture(mode, tol):
     """A caller captures an apply of 16 columns in a context that has only run 256:
