@@ -538,7 +538,15 @@ void Ctx::apply_farfield(zc alpha, const double2 *B, int64_t ldB, zc beta, doubl
     {
         double2 *Bt = Btri_d.reserve(tri_elems);
         launch_avop<double2, double>(mesh, B, ldB, wave_count, Bt, stream);
-        launch_farfield<double>(mesh, flags, prm_d.p, wave_count, wave_chunk_size, Bt, ff_partial_d.reserve(pe), pe,
+        // a stream under capture splits no further than the partial blocks there are: it must not allocate
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        size_t room = pe;
+        if (ff_partial_d.n < pe && ff_partial_d.n >= (size_t)mesh.nm * wave_count)
+        {
+            BAEMM_CUDA(cudaStreamIsCapturing(stream, &capture));
+            if (capture != cudaStreamCaptureStatusNone) room = ff_partial_d.n;
+        }
+        launch_farfield<double>(mesh, flags, prm_d.p, wave_count, wave_chunk_size, Bt, ff_partial_d.reserve(room), room,
                                 make_double2(alpha.real(), alpha.imag()), be, C, ldC, stream);
     }
     else

@@ -1001,7 +1001,9 @@ void launch_farfield(const MeshDev &m, const OpFlags &f, const void *chunk_param
                   "wave_chunk_size must be a power of two <= 64");
     constexpr bool fp64 = std::is_same<R, double>::value;
     SourceSplit split = farfield_split(m, wc, wcs, fp64);
-    BAEMM_REQUIRE((size_t)split.blocks * m.nm * wc <= partial_cap, BAEMM_ERR_SIZE, "far-field partial buffer too small");
+    const size_t room = partial_cap / ((size_t)m.nm * wc);   // blocks of results
+    BAEMM_REQUIRE(room >= 1, BAEMM_ERR_SIZE, "far-field partial buffer too small");
+    split.blocks = (int)std::min<size_t>(split.blocks, room);
     const auto *p = static_cast<const typename Prm<R>::type *>(chunk_params);
     const int mm = (int)m.nm, n = (int)m.nt;
     if constexpr (fp64) launch_farfield_d64(m, f, p, wc, wcs, Btri, partial, split, st);

@@ -246,33 +246,41 @@ def test_averaging_of_few_and_many_rows(mode, tol, wc):
 def test_split_launch_under_capture(mode, tol):
     """A caller captures an apply of 16 columns in a context that has only run 256:
     the narrow launch is split over the sources, the wide one was not, and under
-    capture the partial blocks have to make do with the room there is."""
+    capture the partial blocks have to make do with the room there is.  The same
+    for the far field."""
     import torch
     coords, tris = meshes.torus(n_minor=32, n_major=80)
     s = torch.cuda.Stream()
     B = torch.as_tensor(crandn(np.random.default_rng(3), coords.shape[0], 256)).cuda()
     C, narrow = torch.zeros_like(B), B[:, :16].contiguous()
     Cn, again = torch.zeros_like(narrow), torch.zeros_like(narrow)
+    meas = meshes.fibonacci_sphere(70)
+    B2, n2 = B.to(torch.complex128), narrow.to(torch.complex128)
+    F, Fn = B2.new_zeros(70, 256), B2.new_zeros(70, 16)
     coeff = lambda ks: np.array([COEFF["bie"](k) for k in ks], np.complex128)
-    with Helmholtz_CUDA(coords, tris, np.eye(3)) as H:
+    with Helmholtz_CUDA(coords, tris, meas) as H:
         H.SetApplyMode(mode)
         H.SetStream(s.cuda_stream)
         torch.cuda.synchronize()
         wide = np.linspace(1.0, 6.0, 16)
         H.ApplyBoundaryOperators_PL(1.0, B, 0.0, C, wide, coeff(wide), 256, 16)
+        H.ApplyFarFieldOperators_PL(1.0, B2, 0.0, F, wide, coeff(wide), 256, 16)
         H.LoadBoundaryOperators_PL(np.array([2.0]), coeff([2.0]), 16, 16)
         H.Synchronize()
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g, stream=s):
             H.ApplyBoundaryOperators_PL(1.0, narrow, 0.0, Cn)
+            H.ApplyFarFieldOperators_PL(1.0, n2, 0.0, Fn)
         g.replay()
         H.ApplyBoundaryOperators_PL(1.0, narrow, 0.0, again)
         torch.cuda.synchronize()
         H.UnloadBoundaryOperators_PL()
         H.SetStream(None)
         del g
-    ref = np.zeros((coords.shape[0], 16), np.complex128)
-    O.Oracle(coords, tris, np.eye(3), precision=64).ApplyBoundaryOperators_PL(
-        1.0, narrow.cpu().numpy(), 0.0, ref, np.array([2.0]), coeff([2.0]), 16, 16)
+    ref, fref = np.zeros((coords.shape[0], 16), np.complex128), np.zeros((70, 16), np.complex128)
+    orc, args = O.Oracle(coords, tris, meas, precision=64), (np.array([2.0]), coeff([2.0]), 16, 16)
+    orc.ApplyBoundaryOperators_PL(1.0, narrow.cpu().numpy(), 0.0, ref, *args)
+    orc.ApplyFarFieldOperators_PL(1.0, n2.cpu().numpy(), 0.0, fref, *args)
+    assert relerr(Fn.cpu().numpy(), fref) < tol
     assert relerr(Cn.cpu().numpy(), ref) < tol
     assert relerr(again.cpu().numpy(), ref) < tol
