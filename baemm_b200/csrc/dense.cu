@@ -347,7 +347,7 @@ struct PairTile
 template <int COLS, bool SL, bool DL, bool ADL, bool RI>
 __global__ void __launch_bounds__(kTargets, 4)
 boundary_pair_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, const float *__restrict__ nrm4,
-                     const float2 *__restrict__ B, float2 *__restrict__ C, const ChunkParamsF *__restrict__ prm,
+                     const float2 *B, float2 *__restrict__ C, const ChunkParamsF *__restrict__ prm,
                      int n, int wc, int wcs, int per_split)
 {
     chain_wait();
@@ -492,7 +492,7 @@ boundary_pair_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, con
 
 // C = the sum of the partial blocks of a split launch, in order (four loads in flight).
 template <class R>
-__global__ void split_sum_kernel(const cplx<R> *__restrict__ partial, int splits, int64_t elems, cplx<R> *__restrict__ C)
+__global__ void split_sum_kernel(const cplx<R> *partial, int splits, int64_t elems, cplx<R> *__restrict__ C)
 {
     chain_begin();
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -579,8 +579,8 @@ farfield_partial_kernel(const R *__restrict__ meas4, const R *__restrict__ mid4,
 constexpr int kReduceRows = 8;
 template <class R>
 __global__ void __launch_bounds__(32 * kReduceRows)
-farfield_reduce_kernel(const cplx<R> *__restrict__ partial, int splits, int m, int wc, double2 alpha, double2 beta,
-                       double2 *__restrict__ Cout, int64_t ldC)
+farfield_reduce_kernel(const cplx<R> *partial, int splits, int m, int wc, double2 alpha, double2 beta,
+                       double2 *Cout, int64_t ldC)
 {
     chain_begin();
     __shared__ double2 row[kReduceRows][32];
@@ -727,7 +727,7 @@ __global__ void incident_kernel(int64_t nt, const R *__restrict__ mid4, const R 
 // Evaluation points (m x 3 doubles) as m x 4 reals, w = 0
 // (ApplyNearFieldOperators.hpp:96-107 pads them the same way).
 template <class R>
-__global__ void pack_points_kernel(int64_t m, const double *__restrict__ pts3, R *__restrict__ pts4)
+__global__ void pack_points_kernel(int64_t m, const double *pts3, R *__restrict__ pts4)
 {
     chain_begin();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

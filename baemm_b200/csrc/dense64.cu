@@ -290,8 +290,8 @@ __global__ void __launch_bounds__(kThreads, 2) d64_kernel(const Args a)
             const int kq = e * 4 + warp, j = j0 + kq / (E * NT) * 8 + t;
             const int set = kq % (E * NT) / NT, c = kq % NT * 8 + g;   // column of the set
             const double2 *src = a.B + (int64_t)j * a.wc + col0 + set * a.cols + c;
-            b0[e] = j < je && c < a.cols ? __ldg(src) : make_double2(0.0, 0.0);
-            b1[e] = j + 4 < je && c < a.cols ? __ldg(src + 4 * (int64_t)a.wc) : make_double2(0.0, 0.0);
+            b0[e] = j < je && c < a.cols ? *src : make_double2(0.0, 0.0);
+            b1[e] = j + 4 < je && c < a.cols ? src[4 * (int64_t)a.wc] : make_double2(0.0, 0.0);
         }
         #pragma unroll
         for (int e = 0; e < kTurns; ++e)

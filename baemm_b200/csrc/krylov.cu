@@ -889,8 +889,8 @@ struct ArnSmem
 
 __global__ void __launch_bounds__(kArnThreads, 1)
 arnoldi_kernel(int64_t n, int c, int rpc, int m, int j, const double2 *w_in, const double2 *V, double2 *Vnext,
-               double2 *__restrict__ H, double *__restrict__ cs, double2 *__restrict__ sn, double2 *__restrict__ g,
-               double *__restrict__ res, const double *__restrict__ bnorm, int *__restrict__ flags, double tol)
+               double2 *H, double *cs, double2 *sn, double2 *g, double *res, const double *bnorm, int *flags,
+               double tol)
 {
     chain_wait();
     namespace cg = cooperative_groups;
@@ -930,7 +930,7 @@ arnoldi_kernel(int64_t n, int c, int rpc, int m, int j, const double2 *w_in, con
                 const double2 *p = vbase + (int64_t)(e / 2) * c + g0 * stride;
                 double2 a[kArnGroup];
                 #pragma unroll
-                for (int i = 0; i < kArnGroup; ++i) a[i] = live && g0 + i < nvec ? __ldg(p + i * stride) : zero;
+                for (int i = 0; i < kArnGroup; ++i) a[i] = live && g0 + i < nvec ? p[i * stride] : zero;
                 #pragma unroll
                 for (int i = 0; i < kArnGroup; ++i)
                 {
@@ -990,7 +990,7 @@ arnoldi_kernel(int64_t n, int c, int rpc, int m, int j, const double2 *w_in, con
                 const double2 *p = vbase + (int64_t)(e / 2) * c + g0 * stride;
                 double2 a[kArnGroup];
                 #pragma unroll
-                for (int i = 0; i < kArnGroup; ++i) a[i] = live && g0 + i < nvec ? __ldg(p + i * stride) : zero;
+                for (int i = 0; i < kArnGroup; ++i) a[i] = live && g0 + i < nvec ? p[i * stride] : zero;
                 #pragma unroll
                 for (int i = 0; i < kArnGroup; ++i)
                     if (g0 + i < nvec) acc = Ssub(acc, Smul(sm.h[g0 + i][col], a[i]));

@@ -29,6 +29,12 @@ constexpr int64_t kMassEllMaxRows = 16384;
 // apply of 944 us took 978 with the sums of its split blocks waiting on its SMs).
 // Measured per call: 320 triangles x 16 plain FP32 28.2 -> 25.9 us, 1280 x 32 FP64
 // 45.2 -> 41.0, 5120 x 32 tensor-core 75.6 -> 72.2.
+// Because a chained kernel is on the chip while kernels in front of it still
+// write, what they write is not read-only for its lifetime: it is read through
+// plain pointers.  __ldg, or const __restrict__ (which lets the compiler choose
+// the read-only path, and move the load above chain_wait), would be free to
+// return a line from before the wait.  Only what no kernel of the chain writes
+// (the mesh, the parameters) is __restrict__ there.
 #ifdef __CUDACC__
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -15,8 +15,8 @@ namespace
 {
 
 template <class T> __device__ __forceinline__ double2 ld2(const T *p);
-template <> __device__ __forceinline__ double2 ld2<float2>(const float2 *p) { float2 v = __ldg(p); return make_double2(v.x, v.y); }
-template <> __device__ __forceinline__ double2 ld2<double2>(const double2 *p) { return __ldg(p); }
+template <> __device__ __forceinline__ double2 ld2<float2>(const float2 *p) { const float2 v = *p; return make_double2(v.x, v.y); }
+template <> __device__ __forceinline__ double2 ld2<double2>(const double2 *p) { return *p; }
 template <class T> __device__ __forceinline__ T st2(double2 v);
 template <> __device__ __forceinline__ float2 st2<float2>(double2 v) { return make_float2((float)v.x, (float)v.y); }
 template <> __device__ __forceinline__ double2 st2<double2>(double2 v) { return v; }
@@ -30,7 +30,7 @@ constexpr int kRowsPerBlock = 8;
 template <class Text, class R>
 __global__ void __launch_bounds__(32 * kRowsPerBlock)
 avop_kernel(int64_t nt, int wc, const int32_t *__restrict__ tri_sorted, const R *__restrict__ a3,
-            const Text *__restrict__ Bin, int64_t ldB, cplx<R> *__restrict__ Btri)
+            const Text *Bin, int64_t ldB, cplx<R> *__restrict__ Btri)
 {
     chain_begin();
     const int64_t t = (int64_t)blockIdx.x * kRowsPerBlock + threadIdx.y;
@@ -69,12 +69,12 @@ __global__ void __launch_bounds__(32 * kRowsPerBlock)
 epilogue_kernel(int64_t nv, int wc, int wcs, bool layers, bool sl_diag, bool mass,
                                 const int32_t *__restrict__ avt_outer, const int32_t *__restrict__ avt_inner,
                                 const R *__restrict__ a3, const R *__restrict__ diag,
-                                const cplx<R> *__restrict__ Ctri, const cplx<R> *__restrict__ Btri,
+                                const cplx<R> *Ctri, const cplx<R> *Btri,
                                 const typename PrmOf<R>::type *__restrict__ prm,
                                 const int32_t *__restrict__ m_outer, const int32_t *__restrict__ m_inner,
                                 const R *__restrict__ m_val,
-                                const Text *__restrict__ Bin, int64_t ldB, double2 alpha, double2 beta,
-                                Text *__restrict__ Cout, int64_t ldC, int64_t t_begin, int64_t t_end)
+                                const Text *Bin, int64_t ldB, double2 alpha, double2 beta,
+                                Text *Cout, int64_t ldC, int64_t t_begin, int64_t t_end)
 {
     chain_begin();
     const int64_t v = (int64_t)blockIdx.x * kRowsPerBlock + threadIdx.y;
@@ -353,8 +353,8 @@ __global__ void axpby_kernel(int64_t rows, int cols, T a, const T *__restrict__ 
 // Cout = alpha Cin + beta Cout (keep = false: beta == 0, overwrite, so stale
 // NaNs do not survive), in double, Cin packed with ld wc.
 template <class Text, class R>
-__global__ void combine_kernel(int64_t rows, int wc, double2 alpha, const cplx<R> *__restrict__ Cin, double2 beta,
-                               Text *__restrict__ Cout, int64_t ldC, bool keep)
+__global__ void combine_kernel(int64_t rows, int wc, double2 alpha, const cplx<R> *Cin, double2 beta,
+                               Text *Cout, int64_t ldC, bool keep)
 {
     chain_begin();
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

@@ -643,8 +643,8 @@ __device__ __forceinline__ void tc_entry_ki(const float2 *__restrict__ P, float2
 // Alo Bhi, into the corrections.
 template <int GW, int CH, int R, bool SL, bool DL, bool ADL, bool RI, bool KI, bool PACK>
 __global__ void __launch_bounds__(tc_threads<GW, CH, R>(), 1)
-boundary_tc_kernel(const float *__restrict__ mid4, const float *__restrict__ nrm4, const TcTileGeo *__restrict__ tgeo,
-                   const uint8_t *__restrict__ img, float2 *__restrict__ Ctri, float2 *__restrict__ ws,
+boundary_tc_kernel(const float *mid4, const float *__restrict__ nrm4, const TcTileGeo *__restrict__ tgeo,
+                   const uint8_t *img, float2 *__restrict__ Ctri, float2 *__restrict__ ws,
                    const ChunkParamsF *__restrict__ prm, const TcPlan plan, int *err)
 {
     constexpr int TC_GEN_THREADS = TcShape<GW>::GEN_THREADS;
@@ -1099,7 +1099,7 @@ boundary_tc_kernel(const float *__restrict__ mid4, const float *__restrict__ nrm
 // group sp of row r sits at ((sp ^ (r & 7)) * 16) (img_off16).  hi = tf32(x)
 // rounded to nearest, lo = x - hi (split_tf32).  Sources past n are zero.
 // Thread (t, G, half, q, sp), sp fastest: 8 threads fill one row's 128 bytes.
-__global__ void tc_expand_kernel(const float2 *__restrict__ Btri, int n, int wc, int64_t total, int share,
+__global__ void tc_expand_kernel(const float2 *Btri, int n, int wc, int64_t total, int share,
                                  uint8_t *__restrict__ img)
 {
     chain_begin();
@@ -1177,7 +1177,7 @@ namespace
 // and 86 us.)
 constexpr int TC_FIX_THREADS = 256;
 __global__ void __launch_bounds__(TC_FIX_THREADS)
-tc_fixup_kernel(const float2 *__restrict__ ws, float2 *__restrict__ Ctri, const TcPlan plan, int cw)
+tc_fixup_kernel(const float2 *ws, float2 *__restrict__ Ctri, const TcPlan plan, int cw)
 {
     chain_begin();
     const int j = blockIdx.x;   // tail block
@@ -1194,7 +1194,7 @@ tc_fixup_kernel(const float2 *__restrict__ ws, float2 *__restrict__ Ctri, const 
     // first CTA of a block can have begun in an earlier block.
     constexpr int64_t kSlot = (int64_t)TC_M * (TC_CHMAX * 16);
     const float2 *src = ws + (int64_t)k_first * 2 * kSlot + (int64_t)row * (TC_CHMAX * 16) + col;
-    float4 acc = __ldg(reinterpret_cast<const float4 *>(src + (tc_tail_start(plan, k_first) < lo ? kSlot : 0)));
+    float4 acc = *reinterpret_cast<const float4 *>(src + (tc_tail_start(plan, k_first) < lo ? kSlot : 0));
     auto add = [&](const float4 &v) { acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w; };
     int k = k_first + 1;
     if (plan.tail_units >= plan.ctas)   // every CTA has tail units
@@ -1204,7 +1204,7 @@ tc_fixup_kernel(const float2 *__restrict__ ws, float2 *__restrict__ Ctri, const 
             float4 v[4];
             #pragma unroll
             for (int q = 0; q < 4; ++q)
-                v[q] = __ldg(reinterpret_cast<const float4 *>(src + (int64_t)(k + q - k_first) * 2 * kSlot));
+                v[q] = *reinterpret_cast<const float4 *>(src + (int64_t)(k + q - k_first) * 2 * kSlot);
             #pragma unroll
             for (int q = 0; q < 4; ++q) add(v[q]);
         }
@@ -1212,7 +1212,7 @@ tc_fixup_kernel(const float2 *__restrict__ ws, float2 *__restrict__ Ctri, const 
     for (; k <= k_last; ++k)
     {
         if (tc_tail_start(plan, k + 1) == tc_tail_start(plan, k)) continue;   // no tail units: wrote nothing
-        add(__ldg(reinterpret_cast<const float4 *>(src + (int64_t)(k - k_first) * 2 * kSlot)));
+        add(*reinterpret_cast<const float4 *>(src + (int64_t)(k - k_first) * 2 * kSlot));
     }
     *reinterpret_cast<float4 *>(&Ctri[(int64_t)i * plan.wc + cg * cw + col]) = acc;
 }
