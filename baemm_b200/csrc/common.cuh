@@ -114,6 +114,7 @@ struct DevBuf
         if (count > n)
         {
             release();
+            g_devbuf_epoch.fetch_add(1, std::memory_order_relaxed);   // whether or not the new block can be had
             if (count)
             {
                 cudaError_t e = cudaMalloc(&p, count * sizeof(T));
@@ -126,7 +127,6 @@ struct DevBuf
                 }
             }
             n = count;
-            g_devbuf_epoch.fetch_add(1, std::memory_order_relaxed);
         }
         return p;
     }

@@ -479,7 +479,7 @@ void Ctx::apply_nearfield(Text alpha, const Text *B, int64_t ldB, Text beta, Tex
         launch_pack_points<double>(npts, pts3, p4, stream);
         mark(1);
         launch_nearfield_dense<double>(mesh, nf, prm_d.p, wave_count, wave_chunk_size, p4, npts, Bt, Cp, stream,
-                                       {&split_d});
+                                       {&split_pts_d});
         mark(2);
         launch_combine<Text, double>(npts, wave_count, al, Cp, be, C, ldC, stream);
     }
@@ -504,7 +504,7 @@ void Ctx::apply_nearfield(Text alpha, const Text *B, int64_t ldB, Text beta, Tex
         }
         else
             launch_nearfield_dense<float>(mesh, nf, prm_f.p, wave_count, wave_chunk_size, p4, npts, Bt, Cp, stream,
-                                          {&split_f}, dense_variant);
+                                          {&split_pts_f}, dense_variant);
         mark(2);
         launch_combine<Text, float>(npts, wave_count, al, Cp, be, C, ldC, stream);
     }
@@ -525,6 +525,28 @@ template void Ctx::apply_boundary_rows<float2>(float2, const float2 *, int64_t, 
 template void Ctx::apply_boundary<double2>(double2, const double2 *, int64_t, double2, double2 *, int64_t);
 template void Ctx::apply_boundary<float2>(float2, const float2 *, int64_t, float2, float2 *, int64_t);
 
+// Room for the far field's partial blocks, grown to `elems`; a stream under
+// capture, which must not allocate, makes do with what holds one block, and so
+// does a device without the memory.
+template <class T>
+size_t Ctx::farfield_room(DevBuf<T> &partial, size_t elems)
+{
+    const size_t least = (size_t)mesh.nm * wave_count;
+    if (partial.n >= elems) return partial.n;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    BAEMM_CUDA(cudaStreamIsCapturing(stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone && partial.n >= least) return partial.n;
+    try
+    {
+        partial.reserve(elems);
+    }
+    catch (const Error &)
+    {
+        partial.reserve(least);
+    }
+    return partial.n;
+}
+
 void Ctx::apply_farfield(zc alpha, const double2 *B, int64_t ldB, zc beta, double2 *C, int64_t ldC)
 {
     if (wave_chunk_count < 1) return;
@@ -532,21 +554,13 @@ void Ctx::apply_farfield(zc alpha, const double2 *B, int64_t ldB, zc beta, doubl
     BAEMM_REQUIRE(mesh.nm > 0, BAEMM_ERR_SIZE, "no measurement directions");
     BAEMM_REQUIRE(ldB >= wave_count && ldC >= wave_count, BAEMM_ERR_ARG, "leading dimension smaller than wave_count");
     const int64_t tri_elems = mesh.nt * wave_count;
-    const size_t pe = farfield_partial_elems(mesh, wave_count, wave_chunk_size, aux_fp64());
     const double2 be = make_double2(beta.real(), beta.imag());
     if (aux_fp64())
     {
         double2 *Bt = Btri_d.reserve(tri_elems);
         launch_avop<double2, double>(mesh, B, ldB, wave_count, Bt, stream);
-        // a stream under capture splits no further than the partial blocks there are: it must not allocate
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        size_t room = pe;
-        if (ff_partial_d.n < pe && ff_partial_d.n >= (size_t)mesh.nm * wave_count)
-        {
-            BAEMM_CUDA(cudaStreamIsCapturing(stream, &capture));
-            if (capture != cudaStreamCaptureStatusNone) room = ff_partial_d.n;
-        }
-        launch_farfield<double>(mesh, flags, prm_d.p, wave_count, wave_chunk_size, Bt, ff_partial_d.reserve(room), room,
+        const size_t room = farfield_room(ff_partial_d, farfield_partial_elems(mesh, wave_count, true));
+        launch_farfield<double>(mesh, flags, prm_d.p, wave_count, wave_chunk_size, Bt, ff_partial_d.p, room,
                                 make_double2(alpha.real(), alpha.imag()), be, C, ldC, stream);
     }
     else
@@ -555,8 +569,9 @@ void Ctx::apply_farfield(zc alpha, const double2 *B, int64_t ldB, zc beta, doubl
         launch_avop<double2, float>(mesh, B, ldB, wave_count, Bt, stream);
         // combine_matrices takes alpha as the internal Complex (ApplyFarFieldOperators.hpp:405-409)
         const double2 al = make_double2((double)(float)alpha.real(), (double)(float)alpha.imag());
-        launch_farfield<float>(mesh, flags, prm_f.p, wave_count, wave_chunk_size, Bt, ff_partial_f.reserve(pe), pe,
-                               al, be, C, ldC, stream);
+        const size_t room = farfield_room(ff_partial_f, farfield_partial_elems(mesh, wave_count, false));
+        launch_farfield<float>(mesh, flags, prm_f.p, wave_count, wave_chunk_size, Bt, ff_partial_f.p, room, al, be, C,
+                               ldC, stream);
     }
 }
 

@@ -80,8 +80,10 @@ public:
     // work buffers
     DevBuf<float2> Btri_f, Ctri_f, ff_partial_f;
     DevBuf<double2> Btri_d, Ctri_d, ff_partial_d;
-    DevBuf<float2> split_f;             // partial blocks of dense launches split over the sources
-    DevBuf<double2> split_d;
+    // partial blocks of dense launches split over the sources (split_capacity), of
+    // the triangles and of the near field's points
+    DevBuf<float2> split_f, split_pts_f;
+    DevBuf<double2> split_d, split_pts_d;
     DevBuf<float> dirs_f;
     DevBuf<double> dirs_d;
     DevBuf<float> pts_f;                // near field: evaluation points, npts x 4
@@ -215,6 +217,8 @@ public:
 private:
     void init_mesh(const double *coords, int64_t nv, const int32_t *tris, int64_t nt);
     void build_topology_host(const int32_t *tris);
+    template <class T>
+    size_t farfield_room(DevBuf<T> &partial, size_t elems);
     template <class R>
     void dense_apply(const cplx<R> *Btri, cplx<R> *Ctri, int64_t r0 = 0, int64_t r1 = -1);
 };

@@ -822,36 +822,35 @@ void pair_dispatch(int code, dim3 grid, int cluster, cudaStream_t st, DenseTarge
 #undef BAEMM_PR
 }
 
-// Room for the partial blocks of a split; with less, fewer of them (one: none).
-// A stream under capture grows nothing: an allocation would end its capture.
+// Room (elements) for partial blocks at `at`.  A stream under capture grows
+// nothing: an allocation would end its capture.
 template <class R>
-cplx<R> *partial_blocks(SplitSpace<R> ws, int64_t elems, SourceSplit &split, cudaStream_t st)
+size_t partial_room(SplitSpace<R> ws, size_t capacity, cudaStream_t st, cplx<R> *&at)
 {
-    if (split.blocks == 1) return nullptr;
+    at = ws.fixed;
+    if (!ws.grow) return ws.elems;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (ws.grow && ws.grow->n < (size_t)split.blocks * elems) BAEMM_CUDA(cudaStreamIsCapturing(st, &capture));
-    if (!ws.grow || capture != cudaStreamCaptureStatusNone)
+    if (ws.grow->n < capacity)
     {
-        const size_t room = ws.grow ? ws.grow->n : ws.elems;
-        split.blocks = (int)std::max<size_t>(1, std::min<size_t>(split.blocks, room / elems));
-        return ws.grow ? ws.grow->p : ws.fixed;
+        BAEMM_CUDA(cudaStreamIsCapturing(st, &capture));
+        if (capture == cudaStreamCaptureStatusNone) try
+        {
+            ws.grow->reserve(capacity);
+        }
+        catch (const Error &)   // no memory: not split
+        {
+        }
     }
-    try
-    {
-        return ws.grow->reserve((size_t)split.blocks * elems);
-    }
-    catch (const Error &)
-    {
-        split.blocks = 1;
-        return nullptr;
-    }
+    at = ws.grow->p;
+    return std::min(ws.grow->n, capacity);   // the split does not depend on what else the context has run
 }
 
-// Ctri (tg.m x wc) = K Btri over all nt sources for the targets tg.
+// Ctri (tg.m x wc) = K Btri over all nt sources for the targets tg, of which the
+// context's launches have up to most_targets.
 template <class R>
 void dense_dispatch(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
-                    DenseTargets<R> tg, const cplx<R> *Btri, cplx<R> *Ctri, cudaStream_t st, int variant,
-                    SplitSpace<R> ws)
+                    DenseTargets<R> tg, int64_t most_targets, const cplx<R> *Btri, cplx<R> *Ctri, cudaStream_t st,
+                    int variant, SplitSpace<R> ws)
 {
     if (!f.any_layer() || m.nt == 0 || tg.m == 0) return;
     BAEMM_REQUIRE(wcs >= 1 && wcs <= 64 && (wcs & (wcs - 1)) == 0, BAEMM_ERR_SIZE,
@@ -862,12 +861,13 @@ void dense_dispatch(const MeshDev &m, const OpFlags &f, const void *chunk_params
     const auto *p = static_cast<const typename Prm<R>::type *>(chunk_params);
     const R *mid = geo_mid<R>(m), *nrm = geo_nrm<R>(m);
     const int64_t elems = (int64_t)tg.m * wc;
+    const size_t capacity = split_capacity(n, most_targets * wc, sizeof(cplx<R>));
     SourceSplit split;
     cplx<R> *out = nullptr;
     if constexpr (std::is_same<R, double>::value)
     {
-        split = dense_split(d64_ctas(d64_unit(wc, wcs), tg.m, wc), n, tc_sm_count());
-        out = partial_blocks<R>(ws, elems, split, st);
+        const size_t room = partial_room<R>(ws, capacity, st, out);
+        split = dense_split(d64_ctas(d64_unit(wc, wcs), tg.m, wc), n, tc_sm_count(), room / elems);
         launch_boundary_d64(m, f, p, wc, wcs, tg, Btri, split.blocks > 1 ? out : Ctri, split, st);
     }
     else
@@ -886,8 +886,8 @@ void dense_dispatch(const MeshDev &m, const OpFlags &f, const void *chunk_params
         else
         {
             dim3 pairs(ceil_div(tg.m, 2 * kTargets), wc / cols);
-            split = dense_split((int64_t)pairs.x * pairs.y, n, tc_sm_count());
-            out = partial_blocks<R>(ws, elems, split, st);
+            const size_t room = partial_room<R>(ws, capacity, st, out);
+            split = dense_split((int64_t)pairs.x * pairs.y, n, tc_sm_count(), room / elems);
             pairs.z = split.parts();
             const int per_part = ceil_div(n, split.parts());
             cplx<R> *dst = split.blocks > 1 ? out : Ctri;
@@ -927,10 +927,12 @@ void dense_dispatch(const MeshDev &m, const OpFlags &f, const void *chunk_params
 // kTiny sources one cluster takes all parts: its kernel is slower (320 x 16:
 // 13.2 instead of 7.3 + 3.1 us with its sum) but saves a launch, which is what
 // such a call waits for (27.3 instead of 29.4 us a call).
-SourceSplit dense_split(int64_t ctas, int64_t n, int sms)
+constexpr int kTiny = 512, kMinSources = 16, kCluster = 2, kMostBlocks = 64;
+SourceSplit dense_split(int64_t ctas, int64_t n, int sms, int64_t most_blocks)
 {
-    constexpr int kSplitCost = 24, kSumCost = 70, kMinSources = 16, kTiny = 512;
-    const int cluster = n <= kTiny ? 8 : 2, most = n <= kTiny ? 8 : 128;
+    constexpr int kSplitCost = 24, kSumCost = 70;
+    const int cluster = n <= kTiny ? 8 : kCluster;
+    const int most = n <= kTiny ? 8 : kCluster * (int)std::max<int64_t>(1, std::min<int64_t>(kMostBlocks, most_blocks));
     SourceSplit best;
     double best_cost = 0.0;
     for (int parts = 1; parts <= most && (parts == 1 || n >= (int64_t)parts * kMinSources); parts += parts < cluster ? 1 : cluster)
@@ -947,6 +949,19 @@ SourceSplit dense_split(int64_t ctas, int64_t n, int sms)
     return best;
 }
 
+// At most kMostBlocks blocks of at least kCluster * kMinSources sources; 8 MB of
+// them (which give a launch of few CTAs the whole chip) or kEvenBlocks (which even
+// out the waves of a launch that has more); and at most 64 MB.  The estimate above
+// is within 5 % of the unlimited split's, which takes up to 800 MB.
+size_t split_capacity(int64_t n, int64_t elems, size_t elem_bytes)
+{
+    constexpr size_t kFewBytes = (size_t)8 << 20, kMostBytes = (size_t)64 << 20, kEvenBlocks = 14;
+    if (n <= kTiny) return 0;
+    const size_t blocks = std::min<int64_t>(kMostBlocks, n / (kCluster * kMinSources));
+    return std::min({(size_t)elems * blocks, std::max(kFewBytes / elem_bytes, elems * kEvenBlocks),
+                     kMostBytes / elem_bytes});
+}
+
 template <class R>
 void launch_boundary_dense(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
                            const cplx<R> *Btri, cplx<R> *Ctri, cudaStream_t st, SplitSpace<R> ws, int variant,
@@ -955,7 +970,7 @@ void launch_boundary_dense(const MeshDev &m, const OpFlags &f, const void *chunk
     const int64_t r0 = std::max<int64_t>(0, row_begin), r1 = row_end < 0 ? m.nt : std::min<int64_t>(row_end, m.nt);
     if (r1 <= r0) return;
     dense_dispatch<R>(m, f, chunk_params, wc, wcs, DenseTargets<R>{geo_mid<R>(m) + 4 * r0, (int)(r1 - r0), 1, (int)r0},
-                      Btri, Ctri + r0 * wc, st, variant, ws);
+                      m.nt, Btri, Ctri + r0 * wc, st, variant, ws);
 }
 
 template <class R>
@@ -965,7 +980,8 @@ void launch_nearfield_dense(const MeshDev &m, const OpFlags &f, const void *chun
 {
     BAEMM_REQUIRE(!f.adl() && !f.mass(), BAEMM_ERR_ARG, "near field: single and double layer only");
     BAEMM_REQUIRE(npts <= INT32_MAX, BAEMM_ERR_SIZE, "too many evaluation points");
-    dense_dispatch<R>(m, f, chunk_params, wc, wcs, DenseTargets<R>{pts4, (int)npts, 0, 0}, Btri, Cpts, st, variant, ws);
+    dense_dispatch<R>(m, f, chunk_params, wc, wcs, DenseTargets<R>{pts4, (int)npts, 0, 0}, npts, Btri, Cpts, st, variant,
+                      ws);
 }
 
 template <class R>
@@ -976,19 +992,20 @@ void launch_pack_points(int64_t m, const double *pts3, R *pts4, cudaStream_t st)
     BAEMM_LAUNCH_CHECK();
 }
 
-// FP64: the matrix-instruction form's split; FP32: parts of whole tiles, four CTAs per SM
-static SourceSplit farfield_split(const MeshDev &m, int wc, int wcs, bool fp64)
+// The FP32 far field's parts of whole tiles, four CTAs per SM
+constexpr int kFarCtas = 4 * 148;
+static int farfield_splits(const MeshDev &m, int wc, int wcs)
 {
-    if (fp64) return dense_split(d64_ctas(d64_unit(wc, wcs), m.nm, wc), m.nt, tc_sm_count());
     const int ctas = ceil_div(m.nm, kTargets) * (wc / cols_for(wcs));
-    SourceSplit s;
-    s.blocks = std::max(1, std::min(ceil_div(4 * 148, ctas), ceil_div(m.nt, kTile)));
-    return s;
+    return std::max(1, std::min(ceil_div(kFarCtas, ctas), ceil_div(m.nt, kTile)));
 }
 
-size_t farfield_partial_elems(const MeshDev &m, int wc, int wcs, bool fp64)
+size_t farfield_partial_elems(const MeshDev &m, int wc, bool fp64)
 {
-    return (size_t)farfield_split(m, wc, wcs, fp64).blocks * (size_t)m.nm * (size_t)wc;
+    const size_t elems = (size_t)m.nm * wc;
+    if (fp64) return std::max(elems, split_capacity(m.nt, (int64_t)elems, sizeof(double2)));
+    // at most kFarCtas / CTAs + 1 parts, a CTA's results at most kTargets x 16
+    return std::min(elems * ceil_div(m.nt, kTile), elems + (size_t)kFarCtas * kTargets * 16);
 }
 
 template <class R>
@@ -1000,15 +1017,20 @@ void launch_farfield(const MeshDev &m, const OpFlags &f, const void *chunk_param
     BAEMM_REQUIRE(wcs >= 1 && wcs <= 64 && (wcs & (wcs - 1)) == 0, BAEMM_ERR_SIZE,
                   "wave_chunk_size must be a power of two <= 64");
     constexpr bool fp64 = std::is_same<R, double>::value;
-    SourceSplit split = farfield_split(m, wc, wcs, fp64);
     const size_t room = partial_cap / ((size_t)m.nm * wc);   // blocks of results
     BAEMM_REQUIRE(room >= 1, BAEMM_ERR_SIZE, "far-field partial buffer too small");
-    split.blocks = (int)std::min<size_t>(split.blocks, room);
+    SourceSplit split;
     const auto *p = static_cast<const typename Prm<R>::type *>(chunk_params);
     const int mm = (int)m.nm, n = (int)m.nt;
-    if constexpr (fp64) launch_farfield_d64(m, f, p, wc, wcs, Btri, partial, split, st);
+    if constexpr (fp64)
+    {
+        const size_t most = farfield_partial_elems(m, wc, true) / ((size_t)m.nm * wc);
+        split = dense_split(d64_ctas(d64_unit(wc, wcs), m.nm, wc), m.nt, tc_sm_count(), std::min(room, most));
+        launch_farfield_d64(m, f, p, wc, wcs, Btri, partial, split, st);
+    }
     else
     {
+        split.blocks = (int)std::min<size_t>(farfield_splits(m, wc, wcs), room);
         const int cols = cols_for(wcs);
         const int per_split = ceil_div(ceil_div(n, split.blocks), kTile) * kTile;
         split.blocks = ceil_div(n, per_split);

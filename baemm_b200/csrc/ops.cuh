@@ -175,7 +175,7 @@ void launch_axpby(int64_t rows, int cols, T a, const T *x, int64_t ldx, T b, T *
 // (rows of Ctri outside are not written; row_end < 0: all).
 constexpr int kDenseVariants = 3;
 // Where a launch that is split over the sources keeps its partial blocks: a
-// context's buffer that grows as needed, or a fixed block of `elems` elements.
+// context's buffer that grows to split_capacity, or a fixed block of `elems` elements.
 template <class R>
 struct SplitSpace
 {
@@ -195,7 +195,11 @@ struct SourceSplit
     int cluster = 1, blocks = 1;
     int parts() const { return cluster * blocks; }
 };
-SourceSplit dense_split(int64_t ctas, int64_t n, int sms);
+SourceSplit dense_split(int64_t ctas, int64_t n, int sms, int64_t most_blocks);
+// Elements that the partial blocks of launches over at most n sources with at
+// most `elems` results take: never less for more sources or results, so a context
+// that has run a problem has the room for every smaller one, whatever its split.
+size_t split_capacity(int64_t n, int64_t elems, size_t elem_bytes);
 
 // ---- dense64.cu: the FP64 forms on the FP64 matrix instructions --------------------
 // A work unit is `sets` wavenumbers of tiles * 8 columns each (padded where a
@@ -339,7 +343,9 @@ template <class R>
 void launch_farfield(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
                      const cplx<R> *Btri, cplx<R> *partial, size_t partial_cap, double2 alpha, double2 beta,
                      double2 *Cout, int64_t ldC, cudaStream_t st);
-size_t farfield_partial_elems(const MeshDev &m, int wc, int wcs, bool fp64);
+// Elements of `partial` for at most m.nt triangles, m.nm directions and wc columns
+// (never less for more of them).  Any `partial_cap` of at least m.nm * wc will do.
+size_t farfield_partial_elems(const MeshDev &m, int wc, bool fp64);
 // Herglotz kernel (HerglotzWaveKernel.cl:5-176) applied to conj(g).
 template <class R>
 void launch_herglotz(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
