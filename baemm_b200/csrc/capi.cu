@@ -489,7 +489,7 @@ int baemm_set_tuning(baemm_ctx *ctx, int key, int value)
 int baemm_get_tuning(const baemm_ctx *ctx, int key)
 {
     if (!ctx || !ctx->impl) return -1;
-    if (key == BAEMM_TUNE_DENSE_VARIANT) return std::max(0, ctx->impl->dense_variant);   // not set: 0
+    if (key == BAEMM_TUNE_DENSE_VARIANT) return ctx->impl->dense_variant;
     if (key == BAEMM_TUNE_TC_SEGMENT) return ctx->impl->tc_tune.seg_tiles;
     if (key == BAEMM_TUNE_TC_CTAS) return ctx->impl->tc_tune.ctas;
     if (key == BAEMM_TUNE_TC_STAGGER) return ctx->impl->tc_tune.stagger;

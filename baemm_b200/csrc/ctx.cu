@@ -351,7 +351,7 @@ void Ctx::dense_apply(const cplx<R> *Btri, cplx<R> *Ctri, int64_t r0, int64_t r1
 {
     if constexpr (std::is_same<R, double>::value)
         launch_boundary_dense<double>(mesh, flags, prm_d.p, wave_count, wave_chunk_size, Btri, Ctri, stream,
-                                      {&split_d}, -1, r0, r1);
+                                      {&split_d}, 0, r0, r1);
     else if (apply_mode == BAEMM_APPLY_TC && tc_supported(wave_count, wave_chunk_size))
     {
         if (!tc_geo_ready)

@@ -58,7 +58,7 @@ public:
     int block_size = 64;
     int gmres_max_iter = 30, gmres_max_restarts = 3;
     int apply_mode = BAEMM_APPLY_FP32;
-    int dense_variant = -1;           // plain FP32 dense kernel variant (launch_boundary_dense); -1: not set
+    int dense_variant = 0;            // plain FP32 dense kernel variant (launch_boundary_dense); 0: the library's choice
     TcTuning tc_tune;                 // tensor-core form settings (TcTuning in ops.cuh)
     DevBuf<float2> tc_ws;             // tensor-core form: partial sums of target blocks split between CTAs
     bool tc_geo_ready = false;        // mesh.tgeo_f built

@@ -9,13 +9,14 @@
 //   Herglotz  C_i = sum_j (c1 - i k c2 (nu_i.d_j)) e^{-i k x_i.d_j} conj(g_j) HerglotzWaveKernel.cl:85-160
 //   incident  plane / radial waves at the midpoints                          IncidentWaveKernel_*.hpp
 //
-// Plain form (this file): one thread owns one target and a group of COLS
-// (<= 16) right-hand-side columns of one wave chunk, accumulating COLS complex
-// sums in registers; a CTA of 128 targets streams the sources through shared
-// memory in tiles of 64 (midpoint, normal and the tile's RHS rows), so every
-// generated kernel entry is reused for COLS complex FMAs.  Padded sources are
-// zero (no reading of padded rows, unlike the reference's far-field and
-// Herglotz kernels whose mask is always 1, FarFieldOperatorKernel.cl:89).
+// Plain form (this file; dense64.cu has the FP64 form): a thread owns one or two
+// targets and a group of COLS (<= 16) right-hand-side columns of one wave chunk,
+// accumulating COLS complex sums per target in registers; a CTA of 128 threads
+// streams the sources through shared memory in tiles (midpoint, normal and the
+// tile's RHS rows), so every generated kernel entry is reused for COLS complex
+// FMAs.  Padded sources are zero (no reading of padded rows, unlike the
+// reference's far-field and Herglotz kernels whose mask is always 1,
+// FarFieldOperatorKernel.cl:89).
 #include "ops.cuh"
 
 #include <cooperative_groups.h>
@@ -36,8 +37,6 @@ __device__ __forceinline__ void dsincos(float x, float *s, float *c) { __sincosf
 __device__ __forceinline__ void dsincos(double x, double *s, double *c) { sincos(x, s, c); }
 __device__ __forceinline__ void acc_sincos(float x, float *s, float *c) { sincosf(x, s, c); }
 __device__ __forceinline__ void acc_sincos(double x, double *s, double *c) { sincos(x, s, c); }
-__device__ __forceinline__ float drsqrt(float x) { return rsqrtf(x); }
-__device__ __forceinline__ double drsqrt(double x) { return rsqrt(x); }
 
 constexpr int kTargets = 128;   // threads per CTA (one target per thread per pass)
 constexpr int kTile = 64;       // sources per shared-memory tile
@@ -85,116 +84,13 @@ __device__ __forceinline__ void stage_tile(Tile<R, COLS> &t, const R *__restrict
     }
 }
 
-// Scalar FP32 form (variant 0; dense64.cu has the FP64 form).
-template <int COLS, bool SL, bool DL, bool ADL>
-__global__ void __launch_bounds__(kTargets)
-boundary_dense_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, const float *__restrict__ nrm4,
-                      const float2 *__restrict__ B, float2 *__restrict__ C,
-                      const ChunkParamsF *__restrict__ prm, int n, int wc, int wcs)
-{
-    __shared__ Tile<float, COLS> tile;
-    const int i = blockIdx.x * kTargets + threadIdx.x;
-    const int iself = tg.self ? tg.off + i : -1;   // the source index excluded for this target (none: -1)
-    const int col0 = blockIdx.y * COLS;
-    const int ch = col0 / wcs;
-    const float kap = prm[ch].kappa;
-    const float2 c1 = prm[ch].c[1], c2 = prm[ch].c[2], c3 = prm[ch].c[3];
-    float x0 = 0.f, x1 = 0.f, x2 = 0.f, n0 = 0.f, n1 = 0.f, n2 = 0.f;
-    if (i < tg.m)
-    {
-        const float *x = tg.pts4;
-        x0 = x[4 * (int64_t)i]; x1 = x[4 * (int64_t)i + 1]; x2 = x[4 * (int64_t)i + 2];
-        if (ADL)
-        {
-            const int64_t gi = (int64_t)tg.off + i;   // the target's triangle (ADL: targets are midpoints)
-            n0 = nrm4[4 * gi]; n1 = nrm4[4 * gi + 1]; n2 = nrm4[4 * gi + 2];
-        }
-    }
-    // two-level sum: each 64-source tile into fresh accumulators, then into the
-    // running total (the error of one long FP32 chain over ~1e5 sources would be
-    // ~5x larger)
-    float2 acc[COLS], tacc[COLS];
-    #pragma unroll
-    for (int k = 0; k < COLS; ++k) { acc[k].x = 0.f; acc[k].y = 0.f; }
-
-    for (int j0 = 0; j0 < n; j0 += kTile)
-    {
-        __syncthreads();
-        stage_tile<float, COLS, DL, false>(tile, mid4, nrm4, B, wc, col0, j0, n);
-        __syncthreads();
-        const int smax = min(kTile, n - j0);
-        #pragma unroll
-        for (int k = 0; k < COLS; ++k)
-        {
-            tacc[k].x = 0.f;
-            tacc[k].y = 0.f;
-        }
-        #pragma unroll 2
-        for (int s = 0; s < smax; ++s)
-        {
-            const float zx = tile.y[s][0] - x0, zy = tile.y[s][1] - x1, zz = tile.y[s][2] - x2;
-            const float r2 = zx * zx + zy * zy + zz * zz;
-            const float rinv = (j0 + s == iself) ? 0.f : drsqrt(r2);
-            const float r = r2 * rinv;
-            const float kr = kap * r;
-            float sn, cs;
-            dsincos(kr, &sn, &cs);
-            float2 A;
-            A.x = 0.f;
-            A.y = 0.f;
-            if (SL)
-            {
-                const float er = cs * rinv, ei = sn * rinv;
-                A.x = c1.x * er - c1.y * ei;
-                A.y = c1.x * ei + c1.y * er;
-            }
-            if (DL || ADL)
-            {
-                const float r3 = rinv * rinv * rinv;
-                const float g0 = -(kr * sn + cs) * r3;
-                const float g1 = (kr * cs - sn) * r3;
-                float fx = 0.f, fy = 0.f;
-                if (DL)
-                {
-                    const float dm = zx * tile.mu[s][0] + zy * tile.mu[s][1] + zz * tile.mu[s][2];
-                    fx += c2.x * dm;
-                    fy += c2.y * dm;
-                }
-                if (ADL)
-                {
-                    const float dn = zx * n0 + zy * n1 + zz * n2;
-                    fx -= c3.x * dn;
-                    fy -= c3.y * dn;
-                }
-                A.x += fx * g0 - fy * g1;
-                A.y += fx * g1 + fy * g0;
-            }
-            #pragma unroll
-            for (int k = 0; k < COLS; ++k) cfma(tacc[k], A, tile.B[s][k]);
-        }
-        #pragma unroll
-        for (int k = 0; k < COLS; ++k)
-        {
-            acc[k].x += tacc[k].x;
-            acc[k].y += tacc[k].y;
-        }
-    }
-    if (i < tg.m)
-    {
-        float2 *out = &C[(int64_t)i * wc + col0];
-        #pragma unroll
-        for (int k = 0; k < COLS; ++k) out[k] = acc[k];
-    }
-}
-
 // Packed FP32x2 arithmetic (sm_100 FFMA2), one target per thread and the 16
 // columns of one wave chunk (variant 1).  A complex MAC  c += a b  is two
 // packed FMAs:
 //     c += (a.re, a.re) * (b.re, b.im)
 //     c += (a.im, a.im) * (-b.im, b.re)
 // so the tile stages every RHS row twice, as b and as the swapped, negated
-// (-b.im, b.re).  Half the issue slots of the scalar form for the same FMA-pipe
-// work.
+// (-b.im, b.re).
 constexpr int kPackedCols = 16;
 
 struct PackedTile
@@ -317,9 +213,9 @@ boundary_packed_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, c
     }
 }
 
-// Plain FP32 form over pairs of targets (variant 2): the two halves of every
-// FP32x2 register are two targets (i, i + 128) of the thread, in the entry
-// evaluation as well as in the contraction
+// Plain FP32 form over pairs of targets (the default, and variant 2): the two
+// halves of every FP32x2 register are two targets (i, i + 128) of the thread, in
+// the entry evaluation as well as in the contraction
 //     (c.re, c.im) += (a.re b.re - a.im b.im, a.re b.im + a.im b.re),
 // four packed FMAs per column and pair of targets, with the right-hand side
 // staged as broadcast pairs (b.re, b.re, b.im, b.im): one 16-byte shared load
@@ -328,12 +224,12 @@ boundary_packed_kernel(DenseTargets<float> tg, const float *__restrict__ mid4, c
 // shared by both targets.  Bound by the FP32 pipe: 64 packed FMAs per source
 // and pair of targets at 16 columns, a packed FMA taking two of its cycles.
 // Each 32-source tile is summed into fresh accumulators and added to running
-// totals in shared memory (a private float4 per thread and column; two-level
-// summation as in boundary_dense_kernel), which leaves the registers for four
-// CTAs of 128 threads per SM.
+// totals in shared memory (a private float4 per thread and column; the error of
+// one long FP32 chain over ~1e5 sources would be ~5x larger), which leaves the
+// registers for four CTAs of 128 threads per SM.
 // Measured: 2.80 ms on 20234 triangles x 32 columns (SL + DL', FP32 pipe 72 %
-// busy), the scalar kernel 4.95 ms; 157 us on 5120 x 16 in chunks of 8 columns,
-// the scalar kernel 480 us.
+// busy), one target per thread and unpacked FMAs 4.95 ms; 157 us on 5120 x 16 in
+// chunks of 8 columns, 480 us before.
 constexpr int kPairTile = 32;
 
 template <int COLS>
@@ -753,16 +649,6 @@ __global__ void pack_points_kernel(int64_t m, const double *pts3, R *__restrict_
         default: break;                             \
     }
 
-template <int COLS>
-void scalar_dispatch(int code, dim3 grid, cudaStream_t st, DenseTargets<float> tg, const float *mid, const float *nrm,
-                     const float2 *B, float2 *C, const ChunkParamsF *p, int n, int wc, int wcs)
-{
-#define BAEMM_BK(SL, DL, ADL) \
-    boundary_dense_kernel<COLS, SL, DL, ADL><<<grid, kTargets, 0, st>>>(tg, mid, nrm, B, C, p, n, wc, wcs)
-    BAEMM_BY_LAYERS(BAEMM_BK)
-#undef BAEMM_BK
-}
-
 template <class R, int COLS>
 void farfield_cols(const OpFlags &f, dim3 grid, cudaStream_t st, const R *meas, const R *mid, const R *nrm,
                    const cplx<R> *B, const typename Prm<R>::type *p, int m, int n, int wc, int wcs, int per_split,
@@ -872,16 +758,10 @@ void dense_dispatch(const MeshDev &m, const OpFlags &f, const void *chunk_params
     }
     else
     {
-        // the pair kernel unless another variant was set
-        const dim3 grid(ceil_div(tg.m, kTargets), wc / cols);
-        if (variant == 1 && cols == kPackedCols) packed_dispatch(code, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs);
-        else if (variant == 0 || variant == 1)
+        if (variant == 1 && cols == kPackedCols)
         {
-            if (cols == 16) scalar_dispatch<16>(code, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs);
-            else if (cols == 8) scalar_dispatch<8>(code, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs);
-            else if (cols == 4) scalar_dispatch<4>(code, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs);
-            else if (cols == 2) scalar_dispatch<2>(code, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs);
-            else scalar_dispatch<1>(code, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs);
+            const dim3 grid(ceil_div(tg.m, kTargets), wc / cols);
+            packed_dispatch(code, grid, st, tg, mid, nrm, Btri, Ctri, p, n, wc, wcs);
         }
         else
         {

@@ -169,9 +169,8 @@ void launch_axpby(int64_t rows, int cols, T a, const T *x, int64_t ldx, T b, T *
 // ---- dense.cu ------------------------------------------------------------------
 // Dense boundary kernel (BoundaryOperatorKernel.cl:5-239): Ctri = K(kappa) Btri
 // chunk by chunk, the self pair excluded.  R = float (plain FP32) or double.
-// variant (FP32): 0 scalar FMA kernel, 1 packed FP32x2 kernel (16-column
-// groups; else 0), 2 FP32x2 kernel over pairs of targets, -1 the library's
-// choice (2).  [row_begin, row_end) restricts the targets to those triangles
+// variant (FP32): 0 the library's choice (2), 1 packed FP32x2 kernel (16-column
+// groups; else 2), 2 FP32x2 kernel over pairs of targets.  [row_begin, row_end) restricts the targets to those triangles
 // (rows of Ctri outside are not written; row_end < 0: all).
 constexpr int kDenseVariants = 3;
 // Where a launch that is split over the sources keeps its partial blocks: a
@@ -185,7 +184,7 @@ struct SplitSpace
 };
 template <class R>
 void launch_boundary_dense(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
-                           const cplx<R> *Btri, cplx<R> *Ctri, cudaStream_t st, SplitSpace<R> ws, int variant = -1,
+                           const cplx<R> *Btri, cplx<R> *Ctri, cudaStream_t st, SplitSpace<R> ws, int variant = 0,
                            int64_t row_begin = 0, int64_t row_end = -1);
 // How a dense launch splits the sources: cluster * blocks parts.  The parts of a
 // cluster are summed through distributed shared memory; each of the `blocks`
@@ -224,7 +223,7 @@ void launch_farfield_d64(const MeshDev &m, const OpFlags &f, const ChunkParamsD 
 template <class R>
 void launch_nearfield_dense(const MeshDev &m, const OpFlags &f, const void *chunk_params, int wc, int wcs,
                             const R *pts4, int64_t npts, const cplx<R> *Btri, cplx<R> *Cpts, cudaStream_t st,
-                            SplitSpace<R> ws, int variant = -1);
+                            SplitSpace<R> ws, int variant = 0);
 // Evaluation points (m x 3 doubles, device) -> m x 4 reals, w = 0.
 template <class R>
 void launch_pack_points(int64_t m, const double *pts3, R *pts4, cudaStream_t st);

@@ -1,8 +1,8 @@
 // Autotuner of the dense boundary kernel (baemm_autotune in include/baemm.h).
 //
 // The kernel shapes that matter depend on the mesh size and the wave block:
-// the plain FP32 form has three variants (scalar FMA with 16 columns per
-// thread, packed FP32x2 with one or two targets per thread); the tensor-core
+// the plain FP32 form has its default and the packed FP32x2 kernels with one or
+// two targets per thread; the tensor-core
 // form has its generator-warp count (8 or 16), the 16-column groups per work
 // unit (1, 2 or 4: fewer give small meshes more units to spread over the SMs
 // at the cost of re-evaluating the pair geometry per group) and the length of
@@ -70,7 +70,7 @@ void Ctx::autotune(int mode, int repeats, baemm_tune_result *out)
                      (tc_tune.share << 5);
     const TuneKey key{device, mesh.nt, mesh.nv, wave_count, wave_chunk_size, mode, code, form};
     auto report = [&](const TuneChoice &ch, double before, int cached) {
-        out->dense_variant = std::max(0, dense_variant);
+        out->dense_variant = dense_variant;
         out->tc_segment = tc_tune.seg_tiles;
         out->tc_ctas = tc_tune.ctas;
         out->tc_stagger = tc_tune.stagger;

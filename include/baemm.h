@@ -134,10 +134,9 @@ int baemm_get_gmres_params(const baemm_ctx *ctx, int *max_iter, int *max_restart
 int baemm_set_apply_mode(baemm_ctx *ctx, int mode);        /* BAEMM_APPLY_*; no reference counterpart */
 int baemm_get_apply_mode(const baemm_ctx *ctx);
 /* Kernel tuning knobs (no reference counterpart; results are the same sums):
- *   BAEMM_TUNE_DENSE_VARIANT  plain FP32 dense kernel: 0 scalar FMA, 1 / 2
- *                             packed FP32x2 with 1 / 2 targets per thread; not
- *                             set (the default, read back as 0): the library
- *                             chooses
+ *   BAEMM_TUNE_DENSE_VARIANT  plain FP32 dense kernel: 0 (default) the library's
+ *                             choice, 1 / 2 packed FP32x2 with 1 / 2 targets per
+ *                             thread
  *   BAEMM_TUNE_TC_SEGMENT     tensor-core form: groups of 16 sources accumulated
  *                             in TMEM (rounded up to an even number of groups)
  *                             before each partial sum is added to the FP32
