@@ -14,28 +14,27 @@
 // The FP64 pipe bounds it: matrix and scalar FP64 instructions share it (37
 // TFLOP/s by either, and the mix takes the sum of both times), so what counts
 // is the number of FP64 operations per entry:
-//   * the complex product with 16 columns is three real products instead of
-//     four, P1 = Re A Re B, P2 = Im A Im B, P3 = (Re A + Im A)(Re B + Im B),
-//     C = (P1 - P2) + i (P3 - P1 - P2): 48 fused multiply-adds per entry
-//     instead of 64;
 //   * the geometry of a pair is shared by the E wavenumbers of a work unit, the
 //     entry by all columns of its wavenumber;
 //   * coefficients of the solves (single layer imaginary, double layers real:
 //     RI) need one rotation per entry;
 //   * sine and cosine share one argument reduction; 1/r is the hardware's
 //     approximation and one third-order step.
-// The three products lose a little against four; sums over at most kSegment
-// sources (and the splits of small launches) are added to running totals in
-// shared memory, which gains more: against 64-bit values computed apart, 20833
-// vertices x 32 columns: 3.7e-16, the four-product kernel with one running sum
-// 2.6e-15.
-// Measured: 22.1 ms on 41666 triangles x 32 columns (two wavenumbers, SL + DL;
-// 3.47e9 entries at 40 FP64 instructions and 48 matrix multiply-adds: 75 % of
-// the pipe), 41.6 ms before; far field of 81920 triangles in 256 directions x
-// 32 columns 285 us, 437 before; 1280 x 32 41 us, 446 before (unsplit).  Three
-// blocks per SM (168 registers) took 24.0 ms, one wavenumber per unit 26.6 ms
-// at 2 to 4 blocks; staging element by element instead of in register order
-// cost 4 ms in bank conflicts.
+// The complex product is four real ones, Re C = Re A Re B - Im A Im B and
+// Im C = Re A Im B + Im A Re B, each part accumulated by itself.  (Three products,
+// P1 = Re A Re B, P2 = Im A Im B, P3 = (Re A + Im A)(Re B + Im B), need 48 multiply-
+// adds per entry and 16 columns instead of 64, 22.2 instead of 24.9 ms below, but
+// round the smaller part against the larger: at kappa = 1e-8 the imaginary part of
+// a single-layer apply was off by 4e-9 of itself, now by 1e-15.)
+// Sums over at most kSegment sources (and the splits of small launches) are added
+// to running totals in shared memory.
+// Measured: 24.9 ms on 41666 triangles x 32 columns (two wavenumbers, SL + DL;
+// 3.47e9 entries at 39 FP64 instructions and 64 matrix multiply-adds: 78 % of
+// the pipe), 41.6 ms with scalar FMAs; far field of 81920 triangles in 256
+// directions x 32 columns 319 us, 437 before; 1280 x 32 43 us, 446 before
+// (unsplit).  Three blocks per SM (168 registers) take 24.9 ms, 460 and 57 us;
+// staging element by element instead of in register order cost 4 ms in bank
+// conflicts.
 #include "ops.cuh"
 
 #include <cooperative_groups.h>
@@ -226,7 +225,7 @@ struct FarEntry
 template <int E, int NT>
 struct Smem
 {
-    double2 frag[kStage / 8][E * NT][3][32];   // per step, 8 columns and product: the B registers of each lane
+    double2 frag[kStage / 8][E * NT][2][32];   // per step, 8 columns and part (re, im): the B registers of each lane
     double tot[E * NT * 8][kThreads];          // running totals, private to the thread
     double geo[kStage][6];                     // source position, normal
     double prm[E][8];                          // kappa, c1, -c2, c3
@@ -258,22 +257,20 @@ __global__ void __launch_bounds__(kThreads, 2) d64_kernel(const Args a)
     }
     #pragma unroll
     for (int q = 0; q < E * NT * 8; ++q) sm.tot[q][tid] = 0.0;
-    double acc[E * NT][3][4];
+    double acc[E * NT][2][4];
     #pragma unroll
     for (int q = 0; q < E * NT; ++q)
         #pragma unroll
-        for (int p = 0; p < 3; ++p)
-            #pragma unroll
-            for (int v = 0; v < 4; ++v) acc[q][p][v] = 0.0;
+        for (int v = 0; v < 4; ++v) acc[q][0][v] = acc[q][1][v] = 0.0;
     auto flush = [&]() {
         #pragma unroll
         for (int q = 0; q < E * NT; ++q)
             #pragma unroll
             for (int v = 0; v < 4; ++v)
             {
-                sm.tot[q * 8 + 2 * v][tid] += acc[q][0][v] - acc[q][1][v];
-                sm.tot[q * 8 + 2 * v + 1][tid] += (acc[q][2][v] - acc[q][0][v]) - acc[q][1][v];
-                acc[q][0][v] = acc[q][1][v] = acc[q][2][v] = 0.0;
+                sm.tot[q * 8 + 2 * v][tid] += acc[q][0][v];
+                sm.tot[q * 8 + 2 * v + 1][tid] += acc[q][1][v];
+                acc[q][0][v] = acc[q][1][v] = 0.0;
             }
     };
     int in_segment = 0;
@@ -300,7 +297,6 @@ __global__ void __launch_bounds__(kThreads, 2) d64_kernel(const Args a)
             double2(*f)[32] = sm.frag[kq / (E * NT)][kq % (E * NT)];
             f[0][lane] = make_double2(b0[e].x, b1[e].x);
             f[1][lane] = make_double2(b0[e].y, b1[e].y);
-            f[2][lane] = make_double2(b0[e].x + b0[e].y, b1[e].x + b1[e].y);
         }
         for (int e = tid; e < kStage * 3; e += kThreads)
         {
@@ -328,7 +324,7 @@ __global__ void __launch_bounds__(kThreads, 2) d64_kernel(const Args a)
             #pragma unroll
             for (int e = 0; e < E; ++e)
             {
-                double th[4], sn[4], cs[4], ar[4], ai[4], as[4];
+                double th[4], sn[4], cs[4], ar[4], ai[4], nai[4];
                 bool large = false;
                 #pragma unroll
                 for (int v = 0; v < 4; ++v)
@@ -351,15 +347,17 @@ __global__ void __launch_bounds__(kThreads, 2) d64_kernel(const Args a)
                 for (int v = 0; v < 4; ++v)
                 {
                     Entry::entry(p[v], sm.prm[e], th[v], sn[v], cs[v], ar[v], ai[v]);
-                    as[v] = ar[v] + ai[v];
+                    nai[v] = __hiloint2double(__double2hiint(ai[v]) ^ 0x80000000, __double2loint(ai[v]));
                 }
                 #pragma unroll
                 for (int q = 0; q < NT; ++q)
                 {
                     const double2(*f)[32] = sm.frag[k][e * NT + q];
-                    dmma(acc[e * NT + q][0], ar, f[0][lane]);
-                    dmma(acc[e * NT + q][1], ai, f[1][lane]);
-                    dmma(acc[e * NT + q][2], as, f[2][lane]);
+                    const double2 br = f[0][lane], bi = f[1][lane];
+                    dmma(acc[e * NT + q][0], ar, br);
+                    dmma(acc[e * NT + q][1], ar, bi);
+                    dmma(acc[e * NT + q][0], nai, bi);
+                    dmma(acc[e * NT + q][1], ai, br);
                 }
             }
         }
