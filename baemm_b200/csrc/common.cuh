@@ -175,6 +175,9 @@ struct OpFlags
 {
     bool re_mass = false, im_mass = false, re_sl = false, im_sl = false;
     bool re_dl = false, im_dl = false, re_adl = false, im_adl = false;
+    // in double, where a part below float's range counts: some single-layer
+    // coefficient has a real part, some (adjoint) double-layer one an imaginary part
+    bool re_sl_d = false, im_dl_d = false, im_adl_d = false;
     bool mass() const { return re_mass || im_mass; }
     bool sl() const { return re_sl || im_sl; }
     bool dl() const { return re_dl || im_dl; }

@@ -309,6 +309,9 @@ void Ctx::load_parameters(const double *kappa, const zc *coeff, int wc, int wcs,
             pf.c[q] = make_float2(z.real(), z.imag());
             pd.c[q] = make_double2(zd.real(), zd.imag());
             const bool re = z.real() != 0.f, im = z.imag() != 0.f;
+            flags.re_sl_d |= q == 1 && zd.real() != 0.0;
+            flags.im_dl_d |= q == 2 && zd.imag() != 0.0;
+            flags.im_adl_d |= q == 3 && zd.imag() != 0.0;
             switch (q)
             {
                 case 0: flags.re_mass |= re; flags.im_mass |= im; break;
@@ -454,6 +457,8 @@ void Ctx::apply_nearfield(Text alpha, const Text *B, int64_t ldB, Text beta, Tex
     nf.im_sl = flags.im_sl;
     nf.re_dl = flags.re_dl;
     nf.im_dl = flags.im_dl;
+    nf.re_sl_d = flags.re_sl_d;
+    nf.im_dl_d = flags.im_dl_d;
     if (!nf.any_layer()) return;
     BAEMM_REQUIRE(ldB >= wave_count && ldC >= wave_count, BAEMM_ERR_ARG, "leading dimension smaller than wave_count");
     BAEMM_REQUIRE(npts >= 0, BAEMM_ERR_ARG, "negative evaluation point count");

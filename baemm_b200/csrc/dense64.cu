@@ -471,7 +471,7 @@ void launch_boundary_d64(const MeshDev &m, const OpFlags &f, const ChunkParamsD 
     const dim3 grid = grid_of(u, tg.m, wc, split);
     const int cluster = split.cluster;
     const int code = (f.sl() ? 1 : 0) | (f.dl() ? 2 : 0) | (f.adl() ? 4 : 0);
-    if (!f.re_sl && !f.im_dl && !f.im_adl) by_layers<true>(code, u, a, grid, cluster, st);
+    if (!f.re_sl_d && !f.im_dl_d && !f.im_adl_d) by_layers<true>(code, u, a, grid, cluster, st);
     else by_layers<false>(code, u, a, grid, cluster, st);
     BAEMM_LAUNCH_CHECK();
 }

@@ -53,3 +53,18 @@ def test_block_with_a_small_part(name):
     got, ref = _run([0, 1, 0, 0], B, name, kappa=0.0)
     assert relerr(got.real, ref.real) < TOL
     assert relerr(got.imag, ref.imag) < TOL
+
+
+@pytest.mark.parametrize("name,coeff", [
+    ("ApplyBoundaryOperators_PL", [0, 1e-60 + 1j, 0, 0]), ("ApplyBoundaryOperators_PL", [0, 0, 1 + 1e-60j, 0]),
+    ("ApplyBoundaryOperators_PL", [0, 0, 0, 1 + 1e-60j]), ("ApplyNearFieldOperators_PL", [0, 1e-60 + 1j, 0, 0]),
+    ("ApplyNearFieldOperators_PL", [0, 0, 1 + 1e-60j, 0])])
+def test_coefficient_parts_below_single_precision(name, coeff):
+    """kappa = 0 on a real block: one part of the result is the tiny part of the
+    coefficient times what the other part is the large one times."""
+    B = np.random.default_rng(4).uniform(0.5, 1.5, (255, 16)).astype(complex)
+    got, ref = _run(coeff, B, name, kappa=0.0)
+    small, large = (got.real, got.imag) if coeff[1] else (got.imag, got.real)
+    assert np.abs(large).max() > 0
+    assert relerr(small * 1e60, large) < TOL
+    assert relerr(got, ref) < TOL
