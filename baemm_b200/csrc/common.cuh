@@ -29,13 +29,23 @@ struct Error : std::runtime_error
                                                      cudaGetErrorString(e_));               \
     } while (0)
 
-// Waits for the stream, giving up the processor between tests: a solve waits once
-// per GMRES iteration, and threads that drive solves of their own (the serving
-// slots, packed solves) may share a core or the driver's lock with it.
-// (cudaStreamSynchronize spins: of two threads solving side by side, the second
-// could stand still until the first had finished.)
+// Waits for the stream.  Where the program has chosen how its threads wait
+// (cudaDeviceScheduleBlockingSync, Spin or Yield), the runtime waits so.  Without
+// a choice it would spin, so the processor is given up between tests: a solve
+// waits once per GMRES iteration, and threads that drive solves of their own (the
+// serving slots, packed solves) may share a core or the driver's lock with it (of
+// two threads solving side by side, the second could stand still until the first
+// had finished).
 inline void wait_stream(cudaStream_t st)
 {
+    unsigned flags = 0;
+    BAEMM_CUDA(cudaGetDeviceFlags(&flags));
+    // an error that nobody has read yet is not ours to clear below
+    if ((flags & cudaDeviceScheduleMask) != cudaDeviceScheduleAuto || cudaPeekAtLastError() != cudaSuccess)
+    {
+        BAEMM_CUDA(cudaStreamSynchronize(st));
+        return;
+    }
     for (;;)
     {
         const cudaError_t e = cudaStreamQuery(st);

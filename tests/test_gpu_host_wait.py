@@ -1,0 +1,52 @@
+"""How the host waits for the device."""
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.join(os.path.dirname(__file__), "..")
+
+WAIT = """
+    import ctypes, time
+    cuda = ctypes.CDLL("libcuda.so.1")
+    assert cuda.cuInit(0) == 0
+    dev = ctypes.c_int()
+    assert cuda.cuDeviceGet(ctypes.byref(dev), 0) == 0
+    # before the context exists; the flag lives and dies with this process
+    assert cuda.cuDevicePrimaryCtxSetFlags_v2(dev, 4) == 0   # CU_CTX_SCHED_BLOCKING_SYNC
+    import numpy as np, torch
+    from baemm_b200 import APPLY_FP64, Helmholtz_CUDA, meshes
+    coords, tris = meshes.torus(n_minor=100, n_major=300)
+    kap, coeff = np.array([2.0]), np.array([[0.5, -2j, 1.0, 0.0]])
+    B = torch.ones(coords.shape[0], 32, dtype=torch.complex128, device="cuda")
+    C = torch.zeros_like(B)
+    with Helmholtz_CUDA(coords, tris, np.eye(3)) as H:
+        H.SetApplyMode(APPLY_FP64)
+        H.LoadBoundaryOperators_PL(kap, coeff, 32, 32)
+        H.SetStream(torch.cuda.Stream().cuda_stream)
+        torch.cuda.synchronize()
+        H.ApplyBoundaryOperators_PL(1.0, B, 0.0, C)
+        H.Synchronize()
+        for _ in range(20):
+            H.ApplyBoundaryOperators_PL(1.0, B, 0.0, C)
+        cpu, wall = time.thread_time(), time.perf_counter()
+        H.Synchronize()
+        cpu, wall = time.thread_time() - cpu, time.perf_counter() - wall
+        H.SetStream(None)
+    print("WAIT", wall, cpu)
+"""
+
+
+def test_wait_keeps_the_programs_blocking_choice():
+    """With cudaDeviceScheduleBlockingSync a wait of about a second takes no
+    processor time to speak of (a tenth of it at most)."""
+    r = subprocess.run([sys.executable, "-c", textwrap.dedent(WAIT)], cwd=ROOT, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    wall, cpu = map(float, r.stdout.split("WAIT")[1].split())
+    assert wall > 0.2
+    assert cpu < 0.1 * wall, (cpu, wall)
