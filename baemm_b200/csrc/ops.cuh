@@ -61,7 +61,10 @@ void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cu
     attr[1].val.clusterDim.z = cluster;
     cfg.attrs = attr;
     cfg.numAttrs = cluster > 1 ? 2 : 1;
-    BAEMM_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    if (e == cudaSuccess) return;
+    (void)cudaGetLastError();   // reported here: the next launch's check must not find it
+    throw Error(BAEMM_ERR_CUDA, std::string("kernel launch failed: ") + cudaGetErrorString(e));
 }
 
 struct MeshDev
