@@ -721,6 +721,31 @@ int baemm_selftest_bounded_wait(int device, double *elapsed_ms, int *code)
     }
 }
 
+int baemm_selftest_fp64_math(int device, int64_t n, const double *x, double *out)
+{
+    try
+    {
+        BAEMM_REQUIRE(n >= 1 && n <= baemm::kMaxMeshSize && x && out, BAEMM_ERR_ARG, "invalid arguments");
+        int devices = 0;
+        BAEMM_CUDA(cudaGetDeviceCount(&devices));
+        BAEMM_REQUIRE(device >= 0 && device < devices, BAEMM_ERR_ARG, "no such device");
+        DeviceScope scope(device);
+        baemm::d64_math_probe(n, x, out);
+        g_create_error.clear();
+        return BAEMM_OK;
+    }
+    catch (const Error &e)
+    {
+        g_create_error = e.what();
+        return e.code;
+    }
+    catch (const std::exception &e)
+    {
+        g_create_error = e.what();
+        return BAEMM_ERR_ARG;
+    }
+}
+
 int baemm_profile_krylov(baemm_ctx *ctx, int columns, int iterations, int basis, double out[10])
 {
     return guarded(ctx, [&](Ctx &c) {

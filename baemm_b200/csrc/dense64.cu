@@ -97,7 +97,9 @@ __device__ __forceinline__ void sincos64(double x, double &s, double &c)
 }
 
 // 1 / sqrt(x): the hardware's approximation y (about 20 bits) and one step of
-// third order, y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2.
+// third order of Householder's method (A. S. Householder, The Numerical Treatment
+// of a Single Nonlinear Equation, 1970), which for y^-2 = x is the binomial series
+// of (1 - e)^(-1/2) up to e^2: y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2.
 __device__ __forceinline__ double rsqrt64(double x)
 {
     double y;
@@ -112,6 +114,23 @@ __device__ __forceinline__ void dmma(double (&c)[4], const double (&a)[4], doubl
         "{%0, %1, %2, %3};"
         : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
         : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b.x), "d"(b.y));
+}
+
+// sin, cos and 1 / sqrt(|x|) of each x as the kernels below evaluate them, then CUDA's
+__global__ void math_probe_kernel(int64_t n, const double *__restrict__ x, double *__restrict__ out)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double s, c;
+    sincos64(x[i], s, c);
+    const double2 v = sincos_any(x[i]);
+    const bool large = (__double2hiint(x[i]) & 0x7fffffff) >= kReduceMax;
+    out[i] = large ? v.x : s;
+    out[n + i] = large ? v.y : c;
+    out[2 * n + i] = rsqrt64(fabs(x[i]));
+    out[3 * n + i] = v.x;
+    out[4 * n + i] = v.y;
+    out[5 * n + i] = rsqrt(fabs(x[i]));
 }
 
 struct Args
@@ -460,6 +479,15 @@ D64Unit d64_unit(int wc, int wcs)
 }
 
 int64_t d64_ctas(const D64Unit &u, int64_t m, int wc) { return (int64_t)ceil_div(m, 4 * kWarpTargets) * (wc / u.columns()); }
+
+void d64_math_probe(int64_t n, const double *x, double *out)
+{
+    DevBuf<double> dx, dy;
+    BAEMM_CUDA(cudaMemcpy(dx.reserve(n), x, n * sizeof(double), cudaMemcpyHostToDevice));
+    math_probe_kernel<<<ceil_div(n, 256), 256>>>(n, dx.p, dy.reserve(6 * n));
+    BAEMM_LAUNCH_CHECK();
+    BAEMM_CUDA(cudaMemcpy(out, dy.p, 6 * n * sizeof(double), cudaMemcpyDeviceToHost));
+}
 
 void launch_boundary_d64(const MeshDev &m, const OpFlags &f, const ChunkParamsD *prm, int wc, int wcs,
                          const DenseTargets<double> &tg, const double2 *Btri, double2 *out, SourceSplit split,

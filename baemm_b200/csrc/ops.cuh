@@ -220,6 +220,8 @@ void launch_boundary_d64(const MeshDev &m, const OpFlags &f, const ChunkParamsD 
                          cudaStream_t st);
 void launch_farfield_d64(const MeshDev &m, const OpFlags &f, const ChunkParamsD *prm, int wc, int wcs,
                          const double2 *Btri, double2 *partial, SourceSplit split, cudaStream_t st);
+// baemm_selftest_fp64_math on the current device (host arrays)
+void d64_math_probe(int64_t n, const double *x, double *out);
 // Near-field kernel (NearFieldOperatorKernel.cl:5-194): Cpts (npts x wc) =
 // K(kappa) Btri at the points pts4 (npts x 4 reals), single and double layer
 // (c1, c2) only, no pair excluded.  Same kernels and variants as the boundary form.

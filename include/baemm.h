@@ -349,6 +349,12 @@ int baemm_packer_stats(const baemm_packer *packer, int64_t *launches, int64_t *p
  * in baemm_last_error(NULL). */
 int baemm_selftest_bounded_wait(int device, double *elapsed_ms, int *code);
 
+/* Self-test of the FP64 form's sine, cosine and reciprocal square root (no
+ * reference counterpart): host arrays x (n) and out (6 x n), which receives
+ * sin(x), cos(x) and 1/sqrt(|x|) as that form evaluates them, then the same by
+ * CUDA's own functions.  Errors: message in baemm_last_error(NULL). */
+int baemm_selftest_fp64_math(int device, int64_t n, const double *x, double *out);
+
 /* Device time of one CG iteration of the mass inverse on this context's mesh,
  * on the path its solves take (no reference counterpart): 2 * columns real
  * columns (columns complex), `iterations` iterations with no column allowed
