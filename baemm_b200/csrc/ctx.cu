@@ -85,7 +85,7 @@ void Ctx::init_mesh(const double *coords, int64_t nv, const int32_t *tris, int64
     launch_geometry(mesh, true, stream);
     launch_mass_values(mesh, false, stream);
     launch_mass_values(mesh, true, stream);
-    tc_geo_ready = false;
+    tc_geo_ready = tc_geo16_ready = false;
     operators_loaded = false;
     ++mesh_generation;
     ++graph_state;
@@ -357,11 +357,7 @@ void Ctx::dense_apply(const cplx<R> *Btri, cplx<R> *Ctri, int64_t r0, int64_t r1
                                       {&split_d}, 0, r0, r1);
     else if (apply_mode == BAEMM_APPLY_TC && tc_supported(wave_count, wave_chunk_size))
     {
-        if (!tc_geo_ready)
-        {
-            launch_tc_tile_geometry(mesh, mesh.tgeo_f.reserve(tc_tile_geometry_floats(mesh.nt)), stream);
-            tc_geo_ready = true;
-        }
+        const float *tgeo = tc_geometry();
         // Only problems whose own launch cannot fill the GPU (at most two target blocks per SM) are packed;
         // a large one would hold its packed partners back until its own sweep ends.
         const int64_t blocks = (int64_t)(wave_count / (16 * tc_chunks_per_unit(wave_count, tc_tune.chunks))) *
@@ -370,15 +366,15 @@ void Ctx::dense_apply(const cplx<R> *Btri, cplx<R> *Ctri, int64_t r0, int64_t r1
             tc_packable(flags, tc_form, wave_count, wave_chunk_size))
         {
             // one problem of the packer's next launch (the stream waits for that launch)
-            const uint8_t *img = launch_tc_expand(Btri, mesh.nt, wave_count, tc_img, stream);
-            const TcPackItem item{mesh.mid_f, mesh.nrm_f, mesh.tgeo_f.p, img, Ctri, prm_bc.p, tc_err.p, mesh.nt,
+            const uint8_t *img = launch_tc_expand(Btri, mesh.nt, wave_count, tc_img, stream, tc_tune);
+            const TcPackItem item{mesh.mid_f, mesh.nrm_f, tgeo, img, Ctri, prm_bc.p, tc_err.p, mesh.nt,
                                   wave_count, tc_form.s};
             packer->apply(item, flags, tc_tune, stream);
             tc_pending = true;
             return;
         }
         const size_t ws_elems = tc_workspace_elems(tc_tune.ctas);
-        launch_boundary_tc(mesh, flags, prm16_f.p, tc_form, wave_count, wave_chunk_size, mesh.tgeo_f.p, Btri, Ctri,
+        launch_boundary_tc(mesh, flags, prm16_f.p, tc_form, wave_count, wave_chunk_size, tgeo, Btri, Ctri,
                            tc_ws.reserve(ws_elems), ws_elems, tc_img, tc_err.p, stream, tc_tune, r0,
                            r1);
         tc_pending = true;
@@ -386,6 +382,19 @@ void Ctx::dense_apply(const cplx<R> *Btri, cplx<R> *Ctri, int64_t r0, int64_t r1
     else
         launch_boundary_dense<float>(mesh, flags, prm_f.p, wave_count, wave_chunk_size, Btri, Ctri, stream,
                                      {&split_f}, dense_variant, r0, r1);
+}
+
+const float *Ctx::tc_geometry()
+{
+    const int src = tc_src(tc_tune);
+    DevBuf<float> &geo = src == 16 ? mesh.tgeo16_f : mesh.tgeo_f;
+    bool &ready = src == 16 ? tc_geo16_ready : tc_geo_ready;
+    if (!ready)
+    {
+        launch_tc_tile_geometry(mesh, src, geo.reserve(tc_tile_geometry_floats(mesh.nt, src)), stream);
+        ready = true;
+    }
+    return geo.p;
 }
 
 // ApplyBoundaryOperators.hpp:289-391 on device blocks.
@@ -497,13 +506,9 @@ void Ctx::apply_nearfield(Text alpha, const Text *B, int64_t ldB, Text beta, Tex
         mark(1);
         if (apply_mode == BAEMM_APPLY_TC && tc_supported(wave_count, wave_chunk_size))
         {
-            if (!tc_geo_ready)
-            {
-                launch_tc_tile_geometry(mesh, mesh.tgeo_f.reserve(tc_tile_geometry_floats(mesh.nt)), stream);
-                tc_geo_ready = true;
-            }
+            const float *tgeo = tc_geometry();
             const size_t ws_elems = tc_workspace_elems(tc_tune.ctas);
-            launch_nearfield_tc(mesh, nf, prm16_f.p, tc_form, wave_count, wave_chunk_size, mesh.tgeo_f.p, p4, npts, Bt, Cp,
+            launch_nearfield_tc(mesh, nf, prm16_f.p, tc_form, wave_count, wave_chunk_size, tgeo, p4, npts, Bt, Cp,
                                 tc_ws.reserve(ws_elems), ws_elems, tc_img, tc_err.p, stream, tc_tune);
             tc_pending = true;
         }

@@ -61,7 +61,8 @@ public:
     int dense_variant = 0;            // plain FP32 dense kernel variant (launch_boundary_dense); 0: the library's choice
     TcTuning tc_tune;                 // tensor-core form settings (TcTuning in ops.cuh)
     DevBuf<float2> tc_ws;             // tensor-core form: partial sums of target blocks split between CTAs
-    bool tc_geo_ready = false;        // mesh.tgeo_f built
+    bool tc_geo_ready = false, tc_geo16_ready = false;   // mesh.tgeo_f, tgeo16_f built
+    const float *tc_geometry();       // the one that tc_tune asks for
     int ir_max_steps = 0;
     double ir_inner_tol = 1e-4;
     baemm_solve_stats stats{};

@@ -79,7 +79,7 @@ struct MeshDev
     DevBuf<float> mass_ell_f;
     DevBuf<double> mass_ell_d;
     DevBuf<float> mid_f, nrm_f, area_f, a3_f, diag_f, mass_f, lumped_f, meas_f;
-    DevBuf<float> tgeo_f;        // tensor-core form: source geometry per source tile (lazily built)
+    DevBuf<float> tgeo_f, tgeo16_f;   // tensor-core form: source geometry per tile of 32 and of 16 sources (lazily built)
     DevBuf<double> mid_d, nrm_d, area_d, a3_d, diag_d, mass_d, lumped_d, meas_d;
 };
 
@@ -248,9 +248,8 @@ struct TcCoeffForm
 };
 TcCoeffForm tc_coeff_form(const ChunkParamsF *host_params, int groups);
 // Settings of the tensor-core form (the autotuner's search space):
-//   seg_tiles  groups of 16 sources accumulated in TMEM (rounded up to whole
-//              tiles of 32) before the partial sum is
-//              added to FP32 registers (bounds the tensor-core accumulation chain);
+//   seg_tiles  most groups of 16 sources accumulated in TMEM before the partial sum
+//              is added to FP32 registers (bounds the tensor-core accumulation chain);
 //   ctas       persistent grid size (0: one CTA per SM);
 //   stagger    sweep offset between CTAs (tiles; -1: spread evenly);
 //   gen_warps  generator warps, 8 or 16;
@@ -264,6 +263,8 @@ struct TcTuning
     int chunks = 0;
     int share = 4;   // most groups of 16 columns sharing one evaluation of the kernel entries (1, 2 or 4)
 };
+// Sources per tile of the tensor-core form: 32, or 16 where no more may be accumulated at a time.
+inline int tc_src(const TcTuning &tune) { return tune.seg_tiles <= 1 ? 16 : 32; }
 // The chunk groups per work unit a launch uses for wave_count wc and the setting `chunks`.
 int tc_chunks_per_unit(int wc, int chunks);
 // The groups per entry set a launch uses: groups with one wavenumber share the
@@ -288,7 +289,7 @@ void launch_nearfield_tc(const MeshDev &m, const OpFlags &f, const void *chunk_p
 void tc_bounded_wait_probe(int code, double *elapsed_ms, int *code_out);
 // share: groups per aligned block that share the kernel entries (tc_entry_sharing; 1 for packed launches)
 const uint8_t *launch_tc_expand(const float2 *Btri, int64_t n, int wc, DevBuf<uint8_t> &img, cudaStream_t st,
-                                int share = 1);
+                                const TcTuning &tune, int share = 1);
 // ---- packed tensor-core launches (several problems in one persistent launch) ----
 // One problem as the host describes it: the boundary operator of one mesh
 // (targets = sources = its nt triangles) on its device blocks.
@@ -335,9 +336,9 @@ int tc_pack_class(const OpFlags &f, int wc, const TcTuning &tune);
 // whatever it is packed with.
 void launch_boundary_tc_packed(const TcPackItem *items, int count, const OpFlags &f, const TcTuning &tune,
                                TcPackScratch &scratch, int *err, cudaStream_t st);
-// Source geometry of the tensor-core form, per source tile (built once per mesh).
-size_t tc_tile_geometry_floats(int64_t nt);
-void launch_tc_tile_geometry(const MeshDev &m, float *tgeo, cudaStream_t st);
+// Source geometry of the tensor-core form, per tile of src sources (built once per mesh).
+size_t tc_tile_geometry_floats(int64_t nt, int src);
+void launch_tc_tile_geometry(const MeshDev &m, int src, float *tgeo, cudaStream_t st);
 // float2 elements of the tensor-core workspace for a persistent grid of `ctas`
 // CTAs (0: one per SM of the current device).
 size_t tc_workspace_elems(int ctas = 0);

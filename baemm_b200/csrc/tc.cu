@@ -396,6 +396,7 @@ struct TcProblem
 struct TcPlan
 {
     int n, wc, nblk, ntiles, ncg, seg_tiles;
+    int half;  // ~15: tiles of 16 sources in the first K half (tc_slot; n counts slots then), else 0
     int m;             // targets (rows of C): n for the boundary operators, the point count for the near field
     int self;          // 1: target i is source off + i and the pair is excluded (boundary); 0: no pair excluded
     int off;           // with self: the triangle of target 0 (a row shard of the boundary apply)
@@ -412,6 +413,8 @@ struct TcPlan
     const int2 *pieces;
 };
 
+// The place of source j in the tiles' slots, TC_SRC each: tiles of 16 sources use the first half.
+__host__ __device__ __forceinline__ int tc_slot(int j, int half) { return j + (j & half); }
 __host__ __device__ __forceinline__ int64_t tc_tail_start(const TcPlan &p, int k)
 {
     return (int64_t)k * p.tail_units / p.ctas;
@@ -773,7 +776,7 @@ boundary_tc_kernel(const float *mid4, const float *__restrict__ nrm4, const TcTi
         {
             const int n = V.n, mt = V.m, wc = V.wc, ntiles = V.ntiles;
             const int i = blk * TC_M + row;
-            const int iself = V.self ? V.off + i : -1;   // the source excluded for this target (none: -1)
+            const int iself = V.self ? tc_slot(V.off + i, plan.half) : -1;   // the slot excluded for this target (none: -1)
             // -x_i and nu_i as broadcast pairs
             float2 nx0 = make_float2(0.f, 0.f), nx1 = nx0, nx2 = nx0, tn0 = nx0, tn1 = nx0, tn2 = nx0;
             if (i < mt)
@@ -788,8 +791,8 @@ boundary_tc_kernel(const float *mid4, const float *__restrict__ nrm4, const TcTi
             }
             const float2 *Pg = V.prm + cg * CH * 8;
             // the source tiles that hold the target block's own triangles (masked)
-            const int self_lo = V.self ? (V.off + blk * TC_M) / TC_SRC : ntiles;
-            const int self_hi = V.self ? (V.off + blk * TC_M + TC_M - 1) / TC_SRC : -1;
+            const int self_lo = V.self ? tc_slot(V.off + blk * TC_M, plan.half) / TC_SRC : ntiles;
+            const int self_hi = V.self ? tc_slot(V.off + blk * TC_M + TC_M - 1, plan.half) / TC_SRC : -1;
             bool first_drain = true;
             // A finished segment is drained right after the next segment's first
             // chunk is stored, so the tensor core has work waiting when it resumes.
@@ -1097,9 +1100,10 @@ boundary_tc_kernel(const float *mid4, const float *__restrict__ nrm4, const TcTi
 // sp = (s0, s1) = (2 sp, 2 sp + 1) the 16-byte group (Re b_s0, Re b_s1,
 // -Im b_s0, -Im b_s1); row 16 + q holds (Im b_s0, Im b_s1, Re b_s0, Re b_s1);
 // group sp of row r sits at ((sp ^ (r & 7)) * 16) (img_off16).  hi = tf32(x)
-// rounded to nearest, lo = x - hi (split_tf32).  Sources past n are zero.
+// rounded to nearest, lo = x - hi (split_tf32).  Sources past n, and the second
+// half of tiles of 16 sources, are zero.
 // Thread (t, G, half, q, sp), sp fastest: 8 threads fill one row's 128 bytes.
-__global__ void tc_expand_kernel(const float2 *Btri, int n, int wc, int64_t total, int share,
+__global__ void tc_expand_kernel(const float2 *Btri, int n, int wc, int64_t total, int share, int src,
                                  uint8_t *__restrict__ img)
 {
     chain_begin();
@@ -1110,10 +1114,10 @@ __global__ void tc_expand_kernel(const float2 *Btri, int n, int wc, int64_t tota
     const int64_t tg = e / (128 * TC_HALVES);        // t * groups + G
     const int64_t t = tg / groups;
     const int G = (int)(tg - t * groups);
-    const int64_t j0 = t * TC_SRC + half * 16 + 2 * sp;
-    const int col = G * 16 + q;
-    const float2 v0 = j0 < n ? Btri[j0 * wc + col] : make_float2(0.f, 0.f);
-    const float2 v1 = j0 + 1 < n ? Btri[(j0 + 1) * wc + col] : make_float2(0.f, 0.f);
+    const int64_t j0 = t * src + half * 16 + 2 * sp;
+    const int col = G * 16 + q, end = half * 16 < src ? n : 0;
+    const float2 v0 = j0 < end ? Btri[j0 * wc + col] : make_float2(0.f, 0.f);
+    const float2 v1 = j0 + 1 < end ? Btri[(j0 + 1) * wc + col] : make_float2(0.f, 0.f);
     uint32_t hr0, lr0, hi0, li0, hr1, lr1, hi1, li1;
     split_tf32(v0.x, hr0, lr0);
     split_tf32(v0.y, hi0, li0);
@@ -1129,19 +1133,21 @@ __global__ void tc_expand_kernel(const float2 *Btri, int n, int wc, int64_t tota
     *reinterpret_cast<uint4 *>(lo_img + img_off16(q + 16, sp)) = make_uint4(li0, li1, lr0, lr1);
 }
 
-// Midpoints and normals of each tile as structure of arrays (zeros
-// past the last triangle).
+// Midpoints and normals of each tile of src sources as structure of arrays (zeros
+// past the last triangle).  The second half of tiles of 16 sources meets zero
+// right-hand sides: it holds points far from any target, with finite entries.
 __global__ void tc_tile_geometry_kernel(const float *__restrict__ mid4, const float *__restrict__ nrm4,
-                                        TcTileGeo *__restrict__ out, int n, int ntiles)
+                                        TcTileGeo *__restrict__ out, int n, int ntiles, int src)
 {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= ntiles * TC_SRC) return;
-    const int t = e / TC_SRC, s = e - t * TC_SRC;
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (int64_t)ntiles * TC_SRC) return;
+    const int64_t t = e / TC_SRC, s = e - t * TC_SRC, j = t * src + s;
     float4 m = make_float4(0.f, 0.f, 0.f, 0.f), v = m;
-    if (e < n)
+    if (s >= src) m.x = m.y = m.z = 1e18f;
+    else if (j < n)
     {
-        m = reinterpret_cast<const float4 *>(mid4)[e];
-        v = reinterpret_cast<const float4 *>(nrm4)[e];
+        m = reinterpret_cast<const float4 *>(mid4)[j];
+        v = reinterpret_cast<const float4 *>(nrm4)[j];
     }
     TcTileGeo &G = out[t];
     G.x[s] = m.x; G.y[s] = m.y; G.z[s] = m.z;
@@ -1151,15 +1157,17 @@ __global__ void tc_tile_geometry_kernel(const float *__restrict__ mid4, const fl
 } // namespace
 
 const uint8_t *launch_tc_expand(const float2 *Btri, int64_t n, int wc, DevBuf<uint8_t> &img, cudaStream_t st,
-                                int share)
+                                const TcTuning &tune, int share)
 {
-    const int64_t ntiles = ceil_div(n, TC_SRC), groups = wc / 16;
+    const int src = tc_src(tune);
+    const int64_t ntiles = ceil_div(n, src), groups = wc / 16;
     const size_t bytes = (size_t)(ntiles * groups) * TC_GROUP_BYTES;
     uint8_t *out = img.reserve(bytes);
     const int64_t total = ntiles * groups * 128 * TC_HALVES;
     if (total > 0)
     {
-        launch_chained(tc_expand_kernel, ceil_div(total, 256), 256, 0, st, 1, Btri, (int)n, wc, total, share, out);
+        launch_chained(tc_expand_kernel, ceil_div(total, 256), 256, 0, st, 1, Btri, (int)n, wc, total, share, src,
+                       out);
         BAEMM_LAUNCH_CHECK();
     }
     return out;
@@ -1341,17 +1349,24 @@ size_t tc_workspace_elems(int ctas)
     return (size_t)ctas * 2 * TC_M * TC_CHMAX * 16;
 }
 
-// Settings count 16-source tiles; the kernel's tiles hold TC_SRC sources.
-static int tc_tiles(int tiles16) { return ceil_div((int64_t)tiles16 * 16, TC_SRC); }
+// Settings count groups of 16 sources.  A segment is the largest number of whole
+// tiles within the setting, so the accumulation chain is never longer than asked
+// for; for a single group the tiles hold 16 sources.
+static int tc_half(const TcTuning &tune) { return tc_src(tune) == 16 ? ~15 : 0; }
+static int tc_segment(const TcTuning &tune) { return (int)std::max<int64_t>(1, (int64_t)tune.seg_tiles * 16 / tc_src(tune)); }
+static int tc_stagger(const TcTuning &tune)
+{
+    return tune.stagger < 0 ? -1 : ceil_div((int64_t)tune.stagger * 16, tc_src(tune));
+}
 
-size_t tc_tile_geometry_floats(int64_t nt) { return (size_t)ceil_div(nt, TC_SRC) * (sizeof(TcTileGeo) / sizeof(float)); }
+size_t tc_tile_geometry_floats(int64_t nt, int src) { return (size_t)ceil_div(nt, src) * (sizeof(TcTileGeo) / sizeof(float)); }
 
-void launch_tc_tile_geometry(const MeshDev &m, float *tgeo, cudaStream_t st)
+void launch_tc_tile_geometry(const MeshDev &m, int src, float *tgeo, cudaStream_t st)
 {
     if (m.nt == 0) return;
-    const int n = (int)m.nt, ntiles = ceil_div(n, TC_SRC);
+    const int n = (int)m.nt, ntiles = ceil_div(n, src);
     tc_tile_geometry_kernel<<<ceil_div((int64_t)ntiles * TC_SRC, 256), 256, 0, st>>>(
-        m.mid_f, m.nrm_f, reinterpret_cast<TcTileGeo *>(tgeo), n, ntiles);
+        m.mid_f, m.nrm_f, reinterpret_cast<TcTileGeo *>(tgeo), n, ntiles, src);
     BAEMM_LAUNCH_CHECK();
 }
 
@@ -1401,7 +1416,6 @@ void tc_run(const MeshDev &m, const OpFlags &f, const void *chunk_params, const 
     BAEMM_REQUIRE(tune.gen_warps == 8 || tune.gen_warps == 16, BAEMM_ERR_ARG, "generator warps: 8 or 16");
     if (!f.any_layer() || m.nt == 0 || m_targets == 0) return;
     TcPlan plan;
-    plan.n = (int)m.nt;
     plan.m = (int)m_targets;
     plan.self = self;
     plan.off = (int)off;
@@ -1409,15 +1423,17 @@ void tc_run(const MeshDev &m, const OpFlags &f, const void *chunk_params, const 
     const int CH = tc_chunks_per_unit(wc, tune.chunks);
     plan.ncg = wc / (16 * CH);
     plan.nblk = ceil_div(plan.m, TC_M);
-    plan.ntiles = ceil_div(plan.n, TC_SRC);
-    plan.seg_tiles = std::max(1, tc_tiles(tune.seg_tiles));
+    plan.half = tc_half(tune);
+    plan.ntiles = ceil_div(m.nt, tc_src(tune));
+    plan.n = tc_slot((int)m.nt, plan.half);
+    plan.seg_tiles = tc_segment(tune);
     const int blocks = plan.ncg * plan.nblk;
     const int ctas = tune.ctas > 0 ? tune.ctas : device_sm_count();
     plan.ctas = (int)std::min<int64_t>(ctas, (int64_t)blocks * plan.ntiles);
     plan.full_waves = blocks / plan.ctas;
     plan.tail_blocks = blocks - plan.full_waves * plan.ctas;
     plan.tail_units = (int64_t)plan.tail_blocks * plan.ntiles;
-    plan.stagger = tune.stagger < 0 ? -1 : tc_tiles(tune.stagger);
+    plan.stagger = tc_stagger(tune);
     plan.ki_s = form.s;
     BAEMM_REQUIRE(ws && ws_elems >= tc_workspace_elems(plan.ctas), BAEMM_ERR_ARG, "tensor-core workspace too small");
     const int code = (f.sl() ? 1 : 0) | (f.dl() ? 2 : 0) | (f.adl() ? 4 : 0);
@@ -1428,7 +1444,7 @@ void tc_run(const MeshDev &m, const OpFlags &f, const void *chunk_params, const 
     // the real / imaginary coefficient structure of the BIE solves (see boundary_tc_kernel)
     const bool ri = !f.re_sl && !f.im_dl && !f.im_adl && (f.dl() || f.adl());
     const int R = tc_entry_sharing(f, form, wc, tune);
-    const uint8_t *im = launch_tc_expand(Btri, m.nt, wc, img, st, R);
+    const uint8_t *im = launch_tc_expand(Btri, m.nt, wc, img, st, tune, R);
     if (tune.gen_warps == 8) tc_dispatch<8>(CH, R, ri, form.ki, code, st, pts4, nrm, tg, im, Ctri, ws, p, plan, err);
     else tc_dispatch<16>(CH, R, ri, form.ki, code, st, pts4, nrm, tg, im, Ctri, ws, p, plan, err);
     BAEMM_LAUNCH_CHECK();
@@ -1590,11 +1606,11 @@ void launch_boundary_tc_packed(const TcPackItem *items, int count, const OpFlags
         P.Ctri = it.Ctri;
         P.prm = it.prm_bcast;
         P.err = it.err;
-        P.n = (int)it.nt;
+        P.n = tc_slot((int)it.nt, tc_half(tune));
         P.m = (int)it.nt;
         P.wc = it.wc;
         P.nblk = ceil_div(it.nt, TC_M);
-        P.ntiles = ceil_div(it.nt, TC_SRC);
+        P.ntiles = ceil_div(it.nt, tc_src(tune));   // the packing class holds the segment
         P.self = 1;
         P.off = 0;
         P.ki_s = it.ki_s;
@@ -1634,7 +1650,8 @@ void launch_boundary_tc_packed(const TcPackItem *items, int count, const OpFlags
     uint8_t *dev = scr.stage(host.data(), total, st);
     TcPlan plan{};
     plan.ctas = ctas;
-    plan.seg_tiles = std::max(1, tc_tiles(tune.seg_tiles));
+    plan.half = tc_half(tune);
+    plan.seg_tiles = tc_segment(tune);
     plan.probs = reinterpret_cast<const TcProblem *>(dev);
     plan.cta_begin = reinterpret_cast<const int *>(dev + off_beg);
     plan.pieces = reinterpret_cast<const int2 *>(dev + off_piece);

@@ -137,11 +137,12 @@ int baemm_get_apply_mode(const baemm_ctx *ctx);
  *   BAEMM_TUNE_DENSE_VARIANT  plain FP32 dense kernel: 0 (default) the library's
  *                             choice, 1 / 2 packed FP32x2 with 1 / 2 targets per
  *                             thread
- *   BAEMM_TUNE_TC_SEGMENT     tensor-core form: groups of 16 sources accumulated
- *                             in TMEM (rounded up to an even number of groups)
- *                             before each partial sum is added to the FP32
- *                             sums in shared memory (default 16; bounds the
- *                             tensor-core accumulation chain)
+ *   BAEMM_TUNE_TC_SEGMENT     tensor-core form: most groups of 16 sources
+ *                             accumulated in TMEM before each partial sum is
+ *                             added to the FP32 sums in shared memory (default
+ *                             16; bounds the tensor-core accumulation chain; odd
+ *                             settings above 1 accumulate one group less, 1 takes
+ *                             half-filled tiles, at up to twice the time)
  *   BAEMM_TUNE_TC_CTAS        tensor-core form: persistent grid size (default 0 =
  *                             one CTA per SM)
  *   BAEMM_TUNE_TC_STAGGER     tensor-core form: CTA k starts its sweep of the
