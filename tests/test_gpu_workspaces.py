@@ -132,3 +132,51 @@ def test_capture_without_room_for_a_split():
         del g
         H.UnloadBoundaryOperators_PL()
         H.SetStream(None)
+
+
+@pytest.mark.parametrize("mode,tol", [(APPLY_FP32, 1e-5), (APPLY_FP64, 1e-11)])
+def test_capture_in_the_room_of_another_shape(mode, tol):
+    """512 triangles x 256 columns leave work blocks as large as 8192 x 16 needs, no
+    partial blocks and fewer of the far field's than that would take: captured, the
+    larger mesh makes do with the room there is and allocates nothing."""
+    import torch
+    coords, tris = _mesh((64, 64))
+    s = torch.cuda.Stream()
+    kap, coeff = np.array([2.0]), np.array([[0.5, -2j, 1.0, 0.0]])
+    B = torch.as_tensor(crandn(np.random.default_rng(3), coords.shape[0], 16)).cuda()
+    C, F, free_c, free_f = (torch.zeros_like(B), B.new_zeros(70, 16), torch.zeros_like(B), B.new_zeros(70, 16))
+    with Helmholtz_CUDA(coords, tris, MEAS) as H:   # with all the room it takes
+        H.SetApplyMode(mode)
+        H.LoadBoundaryOperators_PL(kap, coeff, 16, 16)
+        H.ApplyBoundaryOperators_PL(1.0, B, 0.0, free_c)
+        H.ApplyFarFieldOperators_PL(1.0, B, 0.0, free_f)
+        torch.cuda.synchronize()
+    small = _mesh((16, 16))
+    with Helmholtz_CUDA(*small, MEAS) as H:
+        H.SetApplyMode(mode)
+        wide = np.linspace(1.0, 5.0, 16)
+        wide_coeff = np.array([[0.5, -1j * k, 1.0, 0.0] for k in wide])
+        W = np.ones((256, 256), complex)
+        H.ApplyBoundaryOperators_PL(1.0, W, 0.0, np.zeros_like(W), wide, wide_coeff, 256, 16)
+        H.ApplyFarFieldOperators_PL(1.0, W, 0.0, np.zeros((70, 256), complex), wide, wide_coeff, 256, 16)
+        H.SetMesh(coords, tris)
+        H.SetStream(s.cuda_stream)
+        H.LoadBoundaryOperators_PL(kap, coeff, 16, 16)
+        H.Synchronize()
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            before = torch.cuda.mem_get_info()[0]
+            H.ApplyBoundaryOperators_PL(1.0, B, 0.0, C)
+            H.ApplyFarFieldOperators_PL(1.0, B, 0.0, F)
+            assert torch.cuda.mem_get_info()[0] == before
+        g.replay()
+        torch.cuda.synchronize()
+        for a, b in ((C, free_c), (F, free_f)):
+            assert relerr(a.cpu().numpy(), b.cpu().numpy()) < tol
+        assert not torch.equal(C, free_c)   # split less: in another order
+        if mode == APPLY_FP64:   # in FP32 both far fields have the parts they would choose
+            assert not torch.equal(F, free_f)
+        del g
+        H.UnloadBoundaryOperators_PL()
+        H.SetStream(None)
