@@ -829,17 +829,19 @@ SourceSplit dense_split(int64_t ctas, int64_t n, int sms, int64_t most_blocks)
     return best;
 }
 
-// At most kMostBlocks blocks of at least kCluster * kMinSources sources; 8 MB of
+// At most kMostBlocks blocks of at least kCluster * kMinSources sources; 16 MB of
 // them (which give a launch of few CTAs the whole chip) or kEvenBlocks (which even
-// out the waves of a launch that has more); and at most 64 MB.  The estimate above
-// is within 5 % of the unlimited split's, which takes up to 800 MB.
+// out the waves of a launch that has more); and beyond 64 MB no more than four, up
+// to 1 GB.  Without these limits the split takes up to 14 blocks of a large result;
+// of 17000 random shapes 100 would want more than they leave, for a gain of 3.0 to
+// 3.6 % by the estimate above.
 size_t split_capacity(int64_t n, int64_t elems, size_t elem_bytes)
 {
-    constexpr size_t kFewBytes = (size_t)8 << 20, kMostBytes = (size_t)64 << 20, kEvenBlocks = 14;
+    constexpr size_t MB = (size_t)1 << 20, kEvenBlocks = 20, kLargeBlocks = 4;
     if (n <= kTiny) return 0;
-    const size_t blocks = std::min<int64_t>(kMostBlocks, n / (kCluster * kMinSources));
-    return std::min({(size_t)elems * blocks, std::max(kFewBytes / elem_bytes, elems * kEvenBlocks),
-                     kMostBytes / elem_bytes});
+    const size_t blocks = std::min<int64_t>(kMostBlocks, n / (kCluster * kMinSources)), e = (size_t)elems;
+    const size_t most = std::min(std::max(64 * MB / elem_bytes, kLargeBlocks * e), 1024 * MB / elem_bytes);
+    return std::min({blocks * e, std::max(16 * MB / elem_bytes, kEvenBlocks * e), most});
 }
 
 template <class R>

@@ -43,13 +43,13 @@ def solve_footprint_bytes(nv: int, nt: int, wc: int, restart: int = 30) -> int:
     """Device memory a FarField solve of this size holds in a context: the
     GMRES basis ((restart + 1) vectors of nv x wc complex128), the solver's
     vertex blocks, the CG vectors (2 wc real columns), the triangle blocks in
-    FP32 and FP64, the partial blocks of launches split over the sources (at most
-    14 of each, or 8 MB, and at most 64 MB), and the mesh arrays."""
+    FP32 and FP64, the room for partial blocks of launches split over the sources
+    (split_capacity in csrc/dense.cu), and the mesh arrays."""
     krylov = (restart + 1) * nv * wc * 16 + (restart + 1) ** 2 * wc * 16
     vertex_blocks = 10 * nv * wc * 16
     cg = 5 * nv * 2 * wc * 8
     tri_blocks = 2 * nt * wc * 8 + 2 * nt * wc * 16
-    partial = sum(min(64 << 20, max(8 << 20, 14 * nt * wc * b)) for b in (8, 16))
+    partial = sum(min(max(16 << 20, 20 * nt * wc * b), max(64 << 20, 4 * nt * wc * b), 1 << 30) for b in (8, 16))
     mesh = nt * 200 + nv * 120
     return int(krylov + vertex_blocks + cg + tri_blocks + partial + mesh)
 
