@@ -38,7 +38,7 @@
 //               tc_expand_kernel, into shared memory;
 //   warps GW+1, GW+2  MMA issuers, every other entry set each (a chunk, or
 //               R chunks of one wavenumber sharing their entries; one issuer
-//               when a tile has a single set): 8 tcgen05.mma (kind::tf32, A
+//               when a tile has a single set): 16 tcgen05.mma (kind::tf32, A
 //               from TMEM, B from shared memory, M 128, K 8) per set and tile.
 // Pipelines use mbarriers (A stages in TMEM, B and geometry stages in shared
 // memory).  All roles wait with mbarrier.try_wait, which suspends the warp in
@@ -49,8 +49,8 @@
 // gives a thread eight entries per wait for a stage, publication and barrier
 // round, instead of four with tiles of 16: 19.0 instead of 27.0 instructions
 // per entry; 153600 triangles x 64 columns 95.0 -> 89.3 ms, 20480 x 64 (two
-// wavenumbers) 1343 -> 1105 us, the near field of 30246 triangles at 20011
-// points 1709 -> 1390 us, 5120 x 32 86 -> 76 us.
+// wavenumbers) 1343 -> 1195 us, the near field of 30246 triangles at 20011
+// points 1709 -> 1382 us, 5120 x 32 86 -> 76 us.
 // Every wait is bounded: on time-out the CTA raises a shared abort flag, writes
 // an error code for the host, waits (bounded) for its issued MMAs and frees
 // its TMEM before returning.
@@ -74,8 +74,8 @@ constexpr int TC_SRC = 32;         // sources per K tile (two K halves of 16: a 
 constexpr int TC_N = 32;           // MMA N: 16 columns as (re | im)
 constexpr int TC_CHMAX = 4;        // chunks per work unit
 constexpr int TC_MAXCHUNKS = 32;   // wave_count <= 512 with wave_chunk_size 16
-// Generator warps GW = 16 (4 per SM sub-partition, 4 sources per thread and
-// tile) or 8 (8 sources per thread); the autotuner picks one per problem
+// Generator warps GW = 16 (4 per SM sub-partition, 8 sources per thread and
+// tile) or 8 (16 sources per thread); the autotuner picks one per problem
 // shape.  16 hide the latency of the entry evaluation better on large blocks.
 template <int GW>
 struct TcShape

@@ -4,8 +4,8 @@
 // matrix (Initialize.hpp:329-334).  Rows are filled through atomic counters and
 // sorted afterwards, so the result does not depend on timing.
 //
-// Bound by launches and latency: nine small kernels and one host round trip,
-// whatever the mesh.  Setting a mesh (its copies and geometry included) takes 0.22 ms
+// Bound by launches and latency: six small kernels (ten where the vertices take
+// more than one tile of the scan) and one host round trip.  Setting a mesh (its copies and geometry included) takes 0.22 ms
 // with 5120 triangles, 0.28 with 41666, 0.65 with 153600; with the topology built
 // on the host (a sort of 9 nt 64-bit keys) 1.9, 25.8 and 111 ms.
 #include "ops.cuh"
