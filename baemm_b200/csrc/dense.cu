@@ -714,7 +714,7 @@ template <class R>
 size_t partial_room(SplitSpace<R> ws, size_t capacity, cudaStream_t st, cplx<R> *&at)
 {
     at = ws.fixed;
-    if (!ws.grow) return ws.elems;
+    if (!ws.grow) return std::min(ws.elems, capacity);
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (ws.grow->n < capacity)
     {
