@@ -174,9 +174,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
 }
 // try_wait without a suspend-time hint: the thread is suspended in hardware
 // until the phase completes or a system-dependent time limit passes.  (With
-// an explicit hint the wait measured 3.5 % slower on the torus apply: it
-// became a polling loop with sleeps, whose instructions took issue slots from
-// the generator warps.)
+// an explicit hint the torus apply measured 3.5 % slower.)
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
 {
     uint32_t ok;
